@@ -40,6 +40,9 @@ constexpr int kMaxScope2p = WFG_MAX_SCOPE_2P;  // the cap of the large-scope and
 #ifndef WFG_G1_WARPS5
 #define WFG_G1_WARPS5 28
 #endif
+#ifndef WFG_G1_WARPS_TILES
+#define WFG_G1_WARPS_TILES 20
+#endif
 #ifndef WFG_STEP_UNROLL
 #define WFG_STEP_UNROLL 2
 #endif
@@ -52,9 +55,16 @@ constexpr int kMaxScope2p = WFG_MAX_SCOPE_2P;  // the cap of the large-scope and
 // per block (measured equal to four: 2,457 vs 2,459 ms) lets each warp retire on its own when
 // its queue drains, so a launch that follows on another stream takes over warp slots at once
 // instead of waiting for whole blocks.
+// With rows in tiles a lane holds up to 40 offsets in registers: 20 warps per SM (96 registers).
+// Measured end to end against 24 and 28 warps (same GB300): 20,000 uneven pairs 103.7 ms (109, 119),
+// 150,000 mixture pairs 192.5 ms (205, 217), 10,000 1 kbp pairs 3.78 ms (3.71, 3.76), 200,000 150 bp
+// pairs 13.5 ms (12.7, 12.2); 16 warps (128 registers) within 1 % of 20. The 8-warp shape keeps two
+// blocks per SM (128 registers): 48 pairs of 10-20 kbp 117 ms, three blocks 130 ms, four 148 ms.
 constexpr int kG1Groups = WFG_G1_GROUPS;
-template <bool TWO>
-constexpr int g1_min_blocks() { return (TWO ? WFG_G1_WARPS5 : WFG_G1_WARPS3) / kG1Groups; }
+template <bool TWO, bool TILES>
+constexpr int g1_min_blocks() {
+  return (TILES ? WFG_G1_WARPS_TILES : TWO ? WFG_G1_WARPS5 : WFG_G1_WARPS3) / kG1Groups;
+}
 #ifndef WFG_LEAF_UNROLL
 #define WFG_LEAF_UNROLL 1
 #endif
@@ -105,7 +115,9 @@ __device__ __forceinline__ WfRef absent_ref() {
 // DirCfg so that the other distances' functions keep their register budget); go: the
 // gap-opening adjust of the overlap and its stop conditions (o for gap-affine, max(o, o2) for
 // two-piece gap-affine, 0 otherwise, wavefront/wavefront_bialign.c:396-410).
-struct Pen { int x, o, e, scope, metric, go; };
+// tg: spacing of the scores that hold a row when the rows are computed in tiles (biwfa_tiles.cuh;
+// 0: one score at a time); tm: its magic divisor.
+struct Pen { int x, o, e, scope, metric, go, tg; uint32_t tm; };
 constexpr int kMetricAffine = 0, kMetricEdit = 1, kMetricIndel = 2, kMetricLinear = 3, kMetricAffine2p = 4;
 
 // Oriented window over packed words (forward arrays for the forward aligner and the
@@ -156,6 +168,9 @@ __device__ __forceinline__ uint32_t win32(const uint32_t* w, int pos, int bshift
 // with two (127 registers, no spills).
 #ifndef WFG_G8_MIN_BLOCKS
 #define WFG_G8_MIN_BLOCKS 4
+#endif
+#ifndef WFG_G8_TILES_MIN_BLOCKS
+#define WFG_G8_TILES_MIN_BLOCKS 2
 #endif
 
 #if WFG_LCP64 >= 1
@@ -271,6 +286,7 @@ struct DirCfg {
   int scope;
   uint32_t magic;    // floor(2^32 / scope) + 1: slot = s - scope * umulhi(s, magic), s < 2^27
   int W;             // ring width (power of two)
+  int pitch;         // ints from one ring row to the next (>= W)
   int nphys;         // physical ring buffers (round-robin over non-null steps)
   int lmax;          // leaf descriptor capacity (scores)
   int nc;            // stored components: 3 (M, I1, D1) or 5 (+ I2, D2)
@@ -286,8 +302,19 @@ struct DirCfg {
 // One direction of WFA over one window (a wavefront_aligner_t in WFA2). Lives in shared
 // memory; every thread of the group updates its fields with identical values. A field that
 // a call reads is written by that call only after a group barrier (G > 1).
+constexpr int kTileBufs = WFG_TILE_BUFS;
+// Rows of a direction computed in tiles (biwfa_tiles.cuh).
+struct TileState {
+  int on;            // rows come from tiles (0: from dir_step)
+  int t;             // last row computed
+  int valid;         // last row whose values hold (the first touched row, or t)
+  int touched;       // row `valid` touched an end: dir_step continues after it
+  int lo, hi;        // diagonals [lo, hi) that the last block wrote, in each of its rows
+  int akr[kTileBufs];  // largest antidiagonal of each stored row's M
+};
 struct Dir {
   DirCfg cfg;
+  TileState ts;
   int lcap, lused;
   int next_phys;
   SeqView sv;
@@ -313,7 +340,7 @@ __device__ __forceinline__ WfRef ref_raw(const DirCfg& c, int score, int ci) {
     const int2 ds = ci < 3 ? c.rdesc[slot * 3 + ci] : c.rdesc2[slot * 2 + (ci - 3)];
     r.lo = ds.x; r.hi = ds.y;
     const int buf = ci < 3 ? c.rphys[slot] * 3 + ci : c.nphys * 3 + c.rphys[slot] * 2 + (ci - 3);
-    r.base = c.rdata + (size_t)buf * (size_t)c.W;
+    r.base = c.rdata + (size_t)buf * (size_t)c.pitch;
   } else {
     if (score < 0 || score > c.lmax) return absent_ref();
     const int4 ds = ci < 3 ? c.ldesc[score * 3 + ci] : c.ldesc[(c.lmax + 1) * 3 + score * 2 + (ci - 3)];
@@ -351,7 +378,7 @@ __device__ __noinline__ void dir_init_5(const DirCfg& c, int cbi) {
     for (int i = 0; i < c.scope; ++i) c.rphys[i] = 0;
     set_desc<0>(c, 0, cbi, 0, 0, 0, 0);
     // diagonal 0 of score 0 (physical buffer 0)
-    c.rdata[(size_t)(cbi < 3 ? cbi : c.nphys * 3 + (cbi - 3)) * c.W] = 0;
+    c.rdata[(size_t)(cbi < 3 ? cbi : c.nphys * 3 + (cbi - 3)) * c.pitch] = 0;
   } else {
     for (int ci = 0; ci < c.nc; ++ci) set_desc<1>(c, 0, ci, kAbsent, INT_MIN, 0, 0);
     set_desc<1>(c, 0, cbi, 0, 0, 0, 0);
@@ -379,7 +406,7 @@ __device__ void dir_init(Dir& d, const SeqView& sv, int cb, int ce) {
     for (int i = 0; i < c.scope * 3; ++i) c.rdesc[i] = make_int2(kAbsent, INT_MIN);
     for (int i = 0; i < c.scope; ++i) c.rphys[i] = 0;
     c.rdesc[cbi] = make_int2(0, 0);
-    c.rdata[(size_t)cbi * c.W] = 0;  // diagonal 0 of score 0 (physical buffer 0)
+    c.rdata[(size_t)cbi * c.pitch] = 0;  // diagonal 0 of score 0 (physical buffer 0)
     d.next_phys = 1 % c.nphys;
   } else {
     d.lused = 1;
@@ -450,8 +477,8 @@ __device__ __noinline__ int dir_step_linear(Dir& d, const Pen p, int s, const Gr
   int offm = 0, need = 0;
   if (!kLeaf) {
     if (width > c.W) return -1;
-    om.base = c.rdata + (size_t)(nphys * 3 + 0) * c.W;
-    os.base = om.base + c.W;
+    om.base = c.rdata + (size_t)(nphys * 3 + 0) * c.pitch;
+    os.base = om.base + c.pitch;
     om.kbase = os.kbase = 0;
     om.mask = os.mask = (uint32_t)c.W - 1u;
   } else {
@@ -573,11 +600,11 @@ __device__ __noinline__ int dir_step_2p(Dir& d, const Pen p, int s, const Grp<G>
   int offm = 0, offi1 = 0, offd1 = 0, offi2 = 0, offd2 = 0, need = 0;
   if (!kLeaf) {
     if (width > c.W) return -1;
-    om.base = c.rdata + (size_t)(nphys * 3 + 0) * c.W;
-    oi1.base = om.base + c.W;
-    od1.base = oi1.base + c.W;
-    oi2.base = c.rdata + (size_t)(c.nphys * 3 + nphys * 2) * c.W;
-    od2.base = oi2.base + c.W;
+    om.base = c.rdata + (size_t)(nphys * 3 + 0) * c.pitch;
+    oi1.base = om.base + c.pitch;
+    od1.base = oi1.base + c.pitch;
+    oi2.base = c.rdata + (size_t)(c.nphys * 3 + nphys * 2) * c.pitch;
+    od2.base = oi2.base + c.pitch;
     om.kbase = oi1.kbase = od1.kbase = oi2.kbase = od2.kbase = 0;
     om.mask = oi1.mask = od1.mask = oi2.mask = od2.mask = (uint32_t)c.W - 1u;
   } else {
@@ -701,9 +728,9 @@ __device__ __noinline__ int dir_step(Dir& d, const Pen p, int s, const Grp<G> g,
   int offm = 0, offi = 0, offd = 0, need = 0;
   if (!kLeaf) {
     if (width > c.W) return -1;
-    om.base = c.rdata + (size_t)(nphys * 3 + 0) * c.W;
-    oi.base = om.base + c.W;
-    od.base = oi.base + c.W;
+    om.base = c.rdata + (size_t)(nphys * 3 + 0) * c.pitch;
+    oi.base = om.base + c.pitch;
+    od.base = oi.base + c.pitch;
     om.kbase = oi.kbase = od.kbase = 0;
     om.mask = oi.mask = od.mask = (uint32_t)c.W - 1u;
   } else {
@@ -792,6 +819,8 @@ __device__ __noinline__ int dir_step(Dir& d, const Pen p, int s, const Grp<G> g,
   *max_ak_out = r[6];
   return 0;
 }
+
+#include "biwfa_tiles.cuh"
 
 struct BP { int score, sf, sr, kf, kr, of, orv, comp; };
 
@@ -921,33 +950,29 @@ __device__ __forceinline__ int score_guard(const Pen& p, int plen, int tlen) {
   return (int)min(b, (long long)INT_MAX / 4);
 }
 
-// wavefront_bialign_find_breakpoint
-template <int G, bool TWO>
-__device__ __noinline__ int find_breakpoint(Dir& F, Dir& R, const PairSeqs& q, int pb, int pe, int tb, int te,
-                                            int cb, int ce, const Pen p, int max_steps, BP& bp, const Grp<G> g) {
-  g.sync();
-  dir_init<TWO>(F, fwd_view(q, pb, pe, tb, te), cb, ce);
-  dir_init<TWO>(R, rev_view(q, pb, pe, tb, te), ce, cb);
-  g.sync();
-  const int plen = pe - pb, tlen = te - tb;
-  const int max_antidiag = plen + tlen - 1;
-  const int guard = score_guard(p, plen, tlen);
-  int sf = 0, sr = 0, fmax = 0, rmax = 0, ak = 0;
-  bp.score = INT_MAX;
-  if (dir_extend<G>(F, sf, g, &fmax)) return F.status;
-  if (dir_extend<G>(R, sr, g, &rmax)) return R.status;
-  bool last_fwd = false;
-  for (;;) {
+// The breakpoint search score by score from (sf, sr): resume 0 starts it, 1 and 2 enter the second
+// loop before the step of R or of F.
+template <int G, bool TWO, bool TILES>
+__device__ __noinline__ int breakpoint_steps(Dir& F, Dir& R, int sf, int sr, int fmax, int rmax, bool last_fwd,
+                                             int resume, int guard, const Pen p, int max_steps, BP& bp, const Grp<G> g,
+                                             int* part) {
+  const int max_antidiag = F.sv.plen + F.sv.tlen - 1;
+  int ak = 0;
+  auto step = [&](Dir& d, int s) -> int {
+    if constexpr (TILES) return tile_advance<G>(d, p, s, g, part + (&d == &R ? 2 * (G * 5) : 0), &ak);
+    else return dir_step<G, 0, TWO>(d, p, s, g, &ak);
+  };
+  while (resume == 0) {
     if (fmax + rmax >= max_antidiag) break;
     ++sf;
-    const int qf = dir_step<G, 0, TWO>(F, p, sf, g, &ak);
+    const int qf = step(F, sf);
     if (qf < 0) return WFG_ST_SCRATCH_OVERFLOW;
     if (fmax < ak) fmax = ak;
     last_fwd = true;
     if (qf) return F.status;
     if (fmax + rmax >= max_antidiag) break;
     ++sr;
-    const int qr = dir_step<G, 0, TWO>(R, p, sr, g, &ak);
+    const int qr = step(R, sr);
     if (qr < 0) return WFG_ST_SCRATCH_OVERFLOW;
     if (rmax < ak) rmax = ak;
     last_fwd = false;
@@ -956,20 +981,26 @@ __device__ __noinline__ int find_breakpoint(Dir& F, Dir& R, const PairSeqs& q, i
     if (sf > guard) return WFG_ST_UNATTAINABLE;
   }
   for (;;) {
-    if (last_fwd) {
-      const int min_sr = (sr > p.scope - 1) ? sr - (p.scope - 1) : 0;
-      if (sf + min_sr - p.go >= bp.score) break;
-      overlap<G, TWO>(F, R, sf, sr, true, bp, p, g);
+    if (last_fwd && resume != 2) {
+      if (resume == 0) {
+        const int min_sr = (sr > p.scope - 1) ? sr - (p.scope - 1) : 0;
+        if (sf + min_sr - p.go >= bp.score) break;
+        overlap<G, TWO>(F, R, sf, sr, true, bp, p, g);
+      }
+      resume = 0;
       ++sr;
-      const int q = dir_step<G, 0, TWO>(R, p, sr, g, &ak);
+      const int q = step(R, sr);
       if (q < 0) return WFG_ST_SCRATCH_OVERFLOW;
       if (q) return R.status;
     }
-    const int min_sf = (sf > p.scope - 1) ? sf - (p.scope - 1) : 0;
-    if (min_sf + sr - p.go >= bp.score) break;
-    overlap<G, TWO>(R, F, sr, sf, false, bp, p, g);
+    if (resume == 0) {
+      const int min_sf = (sf > p.scope - 1) ? sf - (p.scope - 1) : 0;
+      if (min_sf + sr - p.go >= bp.score) break;
+      overlap<G, TWO>(R, F, sr, sf, false, bp, p, g);
+    }
+    resume = 0;
     ++sf;
-    const int q = dir_step<G, 0, TWO>(F, p, sf, g, &ak);
+    const int q = step(F, sf);
     if (q < 0) return WFG_ST_SCRATCH_OVERFLOW;
     if (q) return F.status;
     if (sr + sf >= max_steps) return WFG_ST_MAX_STEPS;
@@ -977,6 +1008,180 @@ __device__ __noinline__ int find_breakpoint(Dir& F, Dir& R, const PairSeqs& q, i
     last_fwd = true;
   }
   return ST_OK;
+}
+
+// Whether direction d has row t (computing its block if need be) and the row does not touch.
+template <int G>
+__device__ __forceinline__ bool tile_ready(Dir& d, int t, const Grp<G>& g, int* part) {
+  if (t > d.ts.valid && (d.ts.touched || !tile_next<G>(d, g, part))) return false;
+  return !(d.ts.touched && t == d.ts.valid);
+}
+
+// wavefront_bialign_overlap over untouched rows: row s0 of d0 against the rows of scores s1,
+// s1 - 1, ... of d1. Cells meet where their antidiagonals add up to plen + tlen or more, so the
+// lanes first test the rows' largest ones, a row pair each, and only pairs that pass are scanned.
+// An untouched row's I and D offsets are at most M's on the same diagonal, so a scan reads M and
+// looks at D and I only where M meets. D comes first, then I, then M, the lowest diagonal of each.
+template <int G>
+__device__ __noinline__ void tile_overlap(const Dir& d0, const Dir& d1, int s0, int s1, bool fwd, BP& bp, const Pen& p,
+                                          const Grp<G> g) {
+  const int t0 = row_of(s0, p), cb0 = d0.cb, cb1 = d1.cb;
+  if (!row_exists(cb0, t0, 0)) return;
+  const int plen = d0.sv.plen, tlen = d0.sv.tlen, A = tlen - plen;
+  const int mine = s1 - g.lane();
+  unsigned todo = __ballot_sync(kFull, g.lane() < p.scope && mine >= 0 && holds_row(mine, p) &&
+                                           d0.ts.akr[row_buffer(t0)] + d1.ts.akr[row_buffer(row_of(max(mine, 0), p))] >=
+                                               plen + tlen);
+  const uint32_t mask = (uint32_t)d0.cfg.W - 1u;
+  const int pitch = d0.cfg.pitch;
+  const int32_t* r0 = d0.cfg.rdata + row_buffer(t0) * 3 * pitch;
+  while (todo) {
+    const int s = s1 - (__ffs((int)todo) - 1);
+    todo &= todo - 1;
+    if (s0 + s - p.go >= bp.score) continue;
+    const int t1 = row_of(s, p);
+    const int32_t* r1 = d1.cfg.rdata + row_buffer(t1) * 3 * pitch;
+    const int end = min(row_hi(cb0, t0), A - row_lo(cb1, t1));
+    int first[3] = {INT_MAX, INT_MAX, INT_MAX};  // lowest diagonal where M, I, D meet
+    #pragma unroll 1
+    for (int kb = max(row_lo(cb0, t0), A - row_hi(cb1, t1)) + 32 * g.warp(); kb <= end; kb += 32 * G) {
+      const int k = kb + g.lane();
+      const uint32_t i0 = (uint32_t)k & mask, i1 = (uint32_t)(A - k) & mask;
+      const bool hit = k <= end && r0[i0] + r1[i1] >= tlen;
+      if (!__any_sync(kFull, hit)) continue;
+      if (hit) {
+        first[0] = min(first[0], k);
+        if (r0[pitch + i0] + r1[pitch + i1] >= tlen) first[1] = min(first[1], k);
+        if (r0[2 * pitch + i0] + r1[2 * pitch + i1] >= tlen) first[2] = min(first[2], k);
+      }
+    }
+    const bool mn[3] = {false, false, false};
+    g.minmax(first, mn);
+    const int ci = first[2] != INT_MAX ? 2 : first[1] != INT_MAX ? 1 : 0;
+    const int k = ci == 2 ? first[2] : ci == 1 ? first[1] : first[0];
+    const int cand = ci ? s0 + s - p.o : s0 + s;
+    if (k == INT_MAX || cand >= bp.score) continue;
+    const int o0 = r0[ci * pitch + ((uint32_t)k & mask)], o1 = r1[ci * pitch + ((uint32_t)(A - k) & mask)];
+    bp.score = cand;
+    bp.comp = ci == 2 ? CD : ci == 1 ? CI : CM;
+    bp.sf = fwd ? s0 : s; bp.sr = fwd ? s : s0;
+    bp.kf = fwd ? k : A - k; bp.kr = fwd ? A - k : k;
+    bp.of = fwd ? o0 : o1; bp.orv = fwd ? o1 : o0;
+  }
+}
+
+// The breakpoint search over rows in tiles (biwfa_tiles.cuh). Both directions' blocks are computed
+// until one may hold an event: the antidiagonals add up, or a row touches an end. Its rows are then
+// replayed up to the event; the second phase scans the rows' meetings and computes further blocks
+// when it runs out of rows. A touched row, or a full ring, leaves to breakpoint_steps. Returns
+// ST_OK etc. as find_breakpoint, or INT_MAX when the first cell already touches.
+template <int G>
+__device__ __noinline__ int breakpoint_tiles(Dir& F, Dir& R, const PairSeqs& q, int pb, int pe, int tb, int te, int cb,
+                                             int ce, const Pen p, int guard, BP& bp, const Grp<G> g, int* part) {
+  const int max_antidiag = pe - pb + te - tb - 1;
+  int* part_r = part + 2 * (G * 5);
+  if (tile_start<G>(F, fwd_view(q, pb, pe, tb, te), cb, ce, g) < 0) return INT_MAX;
+  if (tile_start<G>(R, rev_view(q, pb, pe, tb, te), ce, cb, g) < 0) return INT_MAX;
+  g.sync();
+  int fmax = F.ts.akr[row_buffer(0)], rmax = R.ts.akr[row_buffer(0)];
+  int sf = 0, sr = 0, resume = 0;
+  bool last_fwd = false, steps = false;
+  if (fmax + rmax < max_antidiag) {
+    int t = 0;
+    for (;;) {
+      if (!tile_fits(F, t) || !tile_fits(R, t)) { steps = true; break; }
+      int* mf = part + ((t >> 2) & 1) * (G * 5);
+      int* mr = part_r + ((t >> 2) & 1) * (G * 5);
+      const TilePlan pf = tile_plan(cb, t, 32);
+      // one warp: both directions in one pass while half a warp holds each; else the warps take F's
+      // tiles in turn, then R's from where F's ended
+      const bool pair = G == 1 && row_hi(cb, t + 4) - (row_lo(cb, t + 4) & ~3) < 64 &&
+                        row_hi(ce, t + 4) - (row_lo(ce, t + 4) & ~3) < 64;
+      #pragma unroll 1
+      for (int d = 0; d < (pair ? 1 : 2); ++d)
+        tile_run(d ? R : F, R, pair, t, G == 1 ? 0 : d ? (g.warp() + G - pf.tiles % G) % G : g.warp(), G, nullptr, 0, 0,
+                 g.lane(), (d ? mr : mf) + g.warp() * 5, mr);
+      g.sync();
+      const int ft = tile_combine<G>(F, t, mf, g), rt = tile_combine<G>(R, t, mr, g);
+      const bool both = tile_narrow(cb, t, 16) && tile_narrow(ce, t, 16);
+      tile_done(F, t, ft, pair, pair ? both : tile_narrow(cb, t, 32));
+      tile_done(R, t, rt, pair, pair ? both : tile_narrow(ce, t, 32));
+      const int* fa = F.ts.akr + row_buffer(t + 1);
+      const int* ra = R.ts.akr + row_buffer(t + 1);
+      const int nf = max(fmax, max(max(fa[0], fa[1]), max(fa[2], fa[3])));
+      const int nr = max(rmax, max(max(ra[0], ra[1]), max(ra[2], ra[3])));
+      if (min(ft, rt) == 4 && nf + nr < max_antidiag) {
+        fmax = nf; rmax = nr;
+        t += 4;
+        if (t > guard) return WFG_ST_UNATTAINABLE;
+        continue;
+      }
+      #pragma unroll 1
+      for (int j = 0; j < 4; ++j, ++t) {
+        sf = sr = (t + 1) * p.tg;
+        last_fwd = true;
+        if (ft == j) { steps = true; break; }
+        const int f1 = max(fmax, fa[j]);
+        if (f1 + rmax >= max_antidiag) { sr = sf - 1; break; }
+        if (rt == j) { steps = true; break; }
+        const int r1 = max(rmax, ra[j]);
+        last_fwd = false;
+        if (f1 + r1 >= max_antidiag) break;
+        fmax = f1; rmax = r1;
+      }
+      break;
+    }
+    if (steps) {  // the single steps start after row t
+      sf = sr = t * p.tg;
+      last_fwd = false;
+    }
+  }
+  while (!steps) {
+    if (last_fwd) {
+      const int min_sr = (sr > p.scope - 1) ? sr - (p.scope - 1) : 0;
+      if (sf + min_sr - p.go >= bp.score) return ST_OK;
+      if (holds_row(sf, p)) tile_overlap<G>(F, R, sf, sr, true, bp, p, g);
+      if (holds_row(sr + 1, p) && !tile_ready<G>(R, row_of(sr + 1, p), g, part_r)) { resume = 1; break; }
+      ++sr;
+    }
+    const int min_sf = (sf > p.scope - 1) ? sf - (p.scope - 1) : 0;
+    if (min_sf + sr - p.go >= bp.score) return ST_OK;
+    if (holds_row(sr, p)) tile_overlap<G>(R, F, sr, sf, false, bp, p, g);
+    last_fwd = true;
+    if (holds_row(sf + 1, p) && !tile_ready<G>(F, row_of(sf + 1, p), g, part)) { resume = 2; break; }
+    ++sf;
+    if (sf > guard + 2 * p.scope || sr > guard + 2 * p.scope) return WFG_ST_UNATTAINABLE;
+  }
+  if (G > 1) g.sync();
+  tile_describe(F, sf, sf - p.scope + 1, p);
+  tile_describe(R, sr, sr - p.scope + 1, p);
+  g.sync();
+  return breakpoint_steps<G, false, true>(F, R, sf, sr, fmax, rmax, last_fwd, resume, guard, p, INT_MAX, bp, g, part);
+}
+
+// wavefront_bialign_find_breakpoint
+template <int G, bool TWO, bool TILES>
+__device__ __noinline__ int find_breakpoint(Dir& F, Dir& R, const PairSeqs& q, int pb, int pe, int tb, int te,
+                                            int cb, int ce, const Pen p, int max_steps, BP& bp, const Grp<G> g,
+                                            int* part) {
+  const int guard = score_guard(p, pe - pb, te - tb);
+  bp.score = INT_MAX;
+  g.sync();
+  if constexpr (TILES) {
+    if (p.tg) {
+      const int st = breakpoint_tiles<G>(F, R, q, pb, pe, tb, te, cb, ce, p, guard, bp, g, part);
+      if (st != INT_MAX) return st;
+      g.sync();
+    }
+  }
+  dir_init<TWO>(F, fwd_view(q, pb, pe, tb, te), cb, ce);
+  dir_init<TWO>(R, rev_view(q, pb, pe, tb, te), ce, cb);
+  F.ts.on = R.ts.on = 0;
+  g.sync();
+  int fmax = 0, rmax = 0;
+  if (dir_extend<G>(F, 0, g, &fmax)) return F.status;
+  if (dir_extend<G>(R, 0, g, &rmax)) return R.status;
+  return breakpoint_steps<G, TWO, TILES>(F, R, 0, 0, fmax, rmax, false, 0, guard, p, max_steps, bp, g, part);
 }
 
 // Forward run list of the pair (the CIGAR being assembled), with the open run in registers.
@@ -1000,24 +1205,18 @@ struct RunOut {
   }
 };
 
-// wavefront_backtrace_affine: packed (offset<<4)|type source of one step, or the
-// unshifted null when the source is absent or out of range.
-__device__ __forceinline__ long long bt_src(const DirCfg& B, int score, int ci, int kk, int add, int type) {
-  if (score < 0) return (long long)kNull;
-  const WfRef w = ref_raw<1>(B, score, ci);
-  if (w.lo <= kk && kk <= w.hi) return (long long)(w.at(kk) + add) * 16LL + type;
-  return (long long)kNull;
-}
-
 // wavefront_backtrace_affine (wavefront/wavefront_backtrace.c:320-529; TWO: the two-piece
 // distance's I2/D2 sources) or wavefront_backtrace_linear (:223-319) over the leaf store, from
 // (end_k, tlen) at score s in component ce; appends the leaf's ops to out.
-template <bool TWO>
-__device__ __forceinline__ int leaf_backtrace(const Dir& B, const Pen p, int s, int ce, RunOut& out, uint32_t* lruns,
-                                              int lruns_cap) {
+//
+// A step looks up to nine sources: each lane reads one (descriptor, then offset) and a warp
+// maximum of the packed (offset << 4) | type picks WFA2-lib's choice, so a step costs one
+// descriptor and one offset latency whatever its sources. Every warp of the group walks the
+// same path with identical writes.
+template <int G, bool TWO>
+__device__ __noinline__ int leaf_backtrace(const Dir& B, const Pen p, int s, int ce, RunOut& out, uint32_t* lruns,
+                                           int lruns_cap, const Grp<G> g) {
   const DirCfg bc = B.cfg;
-  // Backtrace from (end_k, tlen) in component ce; runs are produced end -> begin. Every
-  // thread of the group walks the same path (uniform loads, identical writes).
   const int plen = B.sv.plen, tlen = B.sv.tlen;
   int nrev = 0; int rop = -1, rlen = 0; bool rover = false;
   auto push = [&](int op, int len) {
@@ -1026,8 +1225,23 @@ __device__ __forceinline__ int leaf_backtrace(const Dir& B, const Pen p, int s, 
     if (rlen > 0) { if (nrev < lruns_cap) lruns[nrev] = ((uint32_t)rlen << 4) | (uint32_t)rop; else rover = true; ++nrev; }
     rop = op; rlen = len;
   };
+  // This lane's source: scores back, component, diagonal step, offset step, type. Lanes 0 mismatch,
+  // 1-2 I open/extend, 3-4 D open/extend, 5-8 the second gap piece. gap-affine:
+  // wavefront_backtrace_affine; edit/indel/gap-linear: wavefront_backtrace_linear, M sources only,
+  // gap-open = o, no mismatch source for indel.
   const bool lin = !TWO && p.metric != kMetricAffine;
-  constexpr bool two = TWO;
+  const int go = p.o + (lin ? 0 : p.e), go2 = bc.o2 + bc.e2;
+  const int lane = g.lane(), role = lane - 1;            // role 0.. : gap sources, two per component
+  const int gap = role >> 1;                             // 0 I, 1 D, 2 I2, 3 D2
+  const bool ext = role & 1, del = gap & 1;
+  const int my_back = lane == 0 ? p.x : gap < 2 ? (ext ? p.e : go) : (ext ? bc.e2 : go2);
+  const int my_ci = lane == 0 || !ext ? 0 : gap + 1;
+  const int my_dk = lane == 0 ? 0 : del ? 1 : -1, my_add = lane == 0 || !del ? 1 : 0;
+  const int my_type = lane == 0 ? BT_M : gap == 0 ? (ext ? BT_I_EXT : BT_I_OPEN) : gap == 1 ? (ext ? BT_D_EXT : BT_D_OPEN)
+                      : gap == 2 ? (ext ? BT_I2_EXT : BT_I2_OPEN) : (ext ? BT_D2_EXT : BT_D2_OPEN);
+  // the component that this lane's source leads to: CM walks take every source, others their own two
+  const int my_comp = gap == 0 ? CI : gap == 1 ? CD : gap == 2 ? CI2 : CD2;
+  const bool usable = lane < (TWO ? 9 : 5) && !(lane == 0 && p.metric == kMetricIndel) && !(lin && lane > 0 && ext);
   int matrix = ce, score = s, k = B.end_k;
   int32_t off = tlen;
   int h = off, v = off - k;
@@ -1038,67 +1252,29 @@ __device__ __forceinline__ int leaf_backtrace(const Dir& B, const Pen p, int s, 
   int iters = 0;
   while (v > 0 && h > 0 && score > 0) {
     if (++iters > plen + tlen + 8) return WFG_ST_UNATTAINABLE;
-    // gap-affine: wavefront_backtrace_affine; edit/indel: wavefront_backtrace_linear
-    // (wavefront/wavefront_backtrace.c:223-319): M sources only, gap-open = o, no mismatch
-    // source for indel
-    const int mm = score - p.x, go = score - p.o - (lin ? 0 : p.e), ge = score - p.e;
-    const int go2 = score - bc.o2 - bc.e2, ge2 = score - bc.e2;  // second gap piece (two-piece only)
-    long long max_all;
-    if (matrix == CM) {
-      const long long mis = (p.metric == kMetricIndel) ? (long long)kNull : bt_src(bc, mm, 0, k, 1, BT_M);
-      const long long io = bt_src(bc, go, 0, k - 1, 1, BT_I_OPEN);
-      const long long ix = lin ? (long long)kNull : bt_src(bc, ge, 1, k - 1, 1, BT_I_EXT);
-      const long long dop = bt_src(bc, go, 0, k + 1, 0, BT_D_OPEN);
-      const long long dx = lin ? (long long)kNull : bt_src(bc, ge, 2, k + 1, 0, BT_D_EXT);
-      long long mi = io >= ix ? io : ix;
-      long long md = dop >= dx ? dop : dx;
-      if (two) {
-        const long long io2 = bt_src(bc, go2, 0, k - 1, 1, BT_I2_OPEN);
-        const long long ix2 = bt_src(bc, ge2, 3, k - 1, 1, BT_I2_EXT);
-        const long long dop2 = bt_src(bc, go2, 0, k + 1, 0, BT_D2_OPEN);
-        const long long dx2 = bt_src(bc, ge2, 4, k + 1, 0, BT_D2_EXT);
-        const long long mi2 = io2 >= ix2 ? io2 : ix2;
-        const long long md2 = dop2 >= dx2 ? dop2 : dx2;
-        mi = mi >= mi2 ? mi : mi2;
-        md = md >= md2 ? md : md2;
-      }
-      const long long mid = mi >= md ? mi : md;
-      max_all = mis >= mid ? mis : mid;
-    } else if (matrix == CI) {
-      const long long io = bt_src(bc, go, 0, k - 1, 1, BT_I_OPEN);
-      const long long ix = bt_src(bc, ge, 1, k - 1, 1, BT_I_EXT);
-      max_all = io >= ix ? io : ix;
-    } else if (!TWO || matrix == CD) {
-      const long long dop = bt_src(bc, go, 0, k + 1, 0, BT_D_OPEN);
-      const long long dx = bt_src(bc, ge, 2, k + 1, 0, BT_D_EXT);
-      max_all = dop >= dx ? dop : dx;
-    } else if (matrix == CI2) {
-      const long long io = bt_src(bc, go2, 0, k - 1, 1, BT_I2_OPEN);
-      const long long ix = bt_src(bc, ge2, 3, k - 1, 1, BT_I2_EXT);
-      max_all = io >= ix ? io : ix;
-    } else {
-      const long long dop = bt_src(bc, go2, 0, k + 1, 0, BT_D2_OPEN);
-      const long long dx = bt_src(bc, ge2, 4, k + 1, 0, BT_D2_EXT);
-      max_all = dop >= dx ? dop : dx;
+    int mine = INT_MIN;
+    if (usable && (matrix == CM || (lane > 0 && matrix == my_comp)) && score >= my_back) {
+      const WfRef w = ref_raw<1>(bc, score - my_back, my_ci);
+      const int32_t o = w.get(k + my_dk);
+      if (o >= 0) mine = (o + my_add) * 16 + my_type;
     }
-    if (max_all < 0) break;
+    const int best = __reduce_max_sync(kFull, mine);
+    if (best < 0) break;
     if (matrix == CM) {
-      const int max_off = (int)(max_all >> 4);
+      const int max_off = best >> 4;
       push(WFG_OP_EQ, off - max_off);
       off = max_off;
       v = off - k; h = off;
       if (v <= 0 || h <= 0) break;
     }
-    const int type = (int)(max_all & 15);
-    if (type == BT_M) { score = mm; matrix = CM; push(WFG_OP_X, 1); --off; }
-    else if (type == BT_I_OPEN) { score = go; matrix = CM; push(WFG_OP_INS, 1); --k; --off; }
-    else if (type == BT_I_EXT) { score = ge; matrix = CI; push(WFG_OP_INS, 1); --k; --off; }
-    else if (type == BT_D_OPEN) { score = go; matrix = CM; push(WFG_OP_DEL, 1); ++k; }
-    else if (!TWO || type == BT_D_EXT) { score = ge; matrix = CD; push(WFG_OP_DEL, 1); ++k; }
-    else if (type == BT_I2_OPEN) { score = go2; matrix = CM; push(WFG_OP_INS, 1); --k; --off; }
-    else if (type == BT_I2_EXT) { score = ge2; matrix = CI2; push(WFG_OP_INS, 1); --k; --off; }
-    else if (type == BT_D2_OPEN) { score = go2; matrix = CM; push(WFG_OP_DEL, 1); ++k; }
-    else { score = ge2; matrix = CD2; push(WFG_OP_DEL, 1); ++k; }
+    const int src = __ffs((int)__ballot_sync(kFull, mine == best)) - 1;
+    score -= __shfl_sync(kFull, my_back, src);
+    const bool src_del = src > 0 && (((src - 1) >> 1) & 1);
+    const int src_comp = __shfl_sync(kFull, ext && lane > 0 ? my_comp : CM, src);
+    matrix = src_comp;
+    if (src == 0) { push(WFG_OP_X, 1); --off; }
+    else if (src_del) { push(WFG_OP_DEL, 1); ++k; }
+    else { push(WFG_OP_INS, 1); --k; --off; }
     v = off - k; h = off;
   }
   if (matrix == CM) {
@@ -1114,53 +1290,115 @@ __device__ __forceinline__ int leaf_backtrace(const Dir& B, const Pen p, int s, 
   }
   if (rlen > 0) { if (nrev < lruns_cap) lruns[nrev] = ((uint32_t)rlen << 4) | (uint32_t)rop; else rover = true; ++nrev; }
   if (rover) return WFG_ST_SCRATCH_OVERFLOW;
-  for (int i = nrev - 1; i >= 0; --i) {
-    const uint32_t r = lruns[i];
+  // Runs lie end to begin and neighbours differ, so only the first can join the open run; the
+  // threads copy the rest, and the last stays open.
+  if (nrev > 0) {
+    const uint32_t r = lruns[nrev - 1];
     out.emit((int)(r & 15u), (int)(r >> 4));
+    if (nrev > 1) {
+      out.flush();
+      for (int i = g.tid; i < nrev - 2; i += 32 * G)
+        if (out.n + i < out.cap) out.buf[out.n + i] = lruns[nrev - 2 - i];
+      out.n += nrev - 2;
+      if (out.n > out.cap) out.overflow = true;
+      const uint32_t q = lruns[0];
+      out.cur_op = (int)(q & 15u); out.cur_len = (int)(q >> 4);
+    }
   }
   return ST_OK;
 }
 
-__device__ __noinline__ int leaf_backtrace_2p(const Dir& B, const Pen p, int s, int ce, RunOut& out, uint32_t* lruns,
-                                             int lruns_cap) {
-  return leaf_backtrace<true>(B, p, s, ce, out, lruns, lruns_cap);
+// The leaf's rows in tiles, up to its end or the first touched row that is not its end. The ring
+// of direction H holds the rows that the next block reads; the leaf store gets every row. Returns
+// 0 when the first cell touches (B is left as it was), 1 when the end is reached, else 2; *s_out:
+// the last score computed.
+template <int G>
+__device__ __noinline__ int leaf_tiles(Dir& B, Dir& H, const SeqView& sv, int cb, int ce, const Pen p, int guard,
+                                       const Grp<G> g, int* part, int* s_out) {
+  const int off0 = tile_start<G>(H, sv, cb, ce, g);
+  if (off0 < 0) return 0;
+  int4* ldesc = B.cfg.ldesc;
+  int32_t* ldata = B.cfg.ldata;
+  const int lmax = B.cfg.lmax, lcap = B.lcap, ak = sv.tlen - sv.plen;
+  if (g.tid < 3) ldesc[g.tid] = g.tid == comp_index(cb) ? make_int4(0, 0, 0, 0) : make_int4(kAbsent, INT_MIN, 0, 0);
+  if (g.tid == 0) ldata[0] = off0;
+  g.sync();
+  int used = 4, last = 0;
+  bool done = false;
+  #pragma unroll 1
+  for (int t0 = 0; t0 <= guard; t0 += 4) {
+    const int lo = row_lo(cb, t0 + 4) & ~3, n = (row_hi(cb, t0 + 4) - lo + 4) & ~3;
+    if ((t0 + 4) * p.tg > lmax || used + 12 * n > lcap || !tile_fits(H, t0)) break;
+    int* mine = part + ((t0 >> 2) & 1) * (G * 5);
+    tile_run(H, H, false, t0, g.warp(), G, ldata + used, lo, n, g.lane(), mine + g.warp() * 5, nullptr);
+    #pragma unroll 1
+    for (int i = g.tid; i < 4 * p.tg * 3; i += 32 * G) {
+      const int s = t0 * p.tg + 1 + i / 3, ci = i % 3, t = row_of(s, p);
+      int4 ds = make_int4(kAbsent, INT_MIN, 0, 0);
+      if (s == t * p.tg && row_exists(cb, t, ci))
+        ds = make_int4(row_lo(cb, t), row_hi(cb, t), used + ((t - t0 - 1) * 3 + ci) * n, lo);
+      ldesc[s * 3 + ci] = ds;
+    }
+    g.sync();
+    const int touch = tile_combine<G>(H, t0, mine, g);
+    tile_done(H, t0, touch, false, tile_narrow(cb, t0, 32));
+    last = H.ts.valid;
+    if (touch < 4) {  // the end diagonal's offset in row `last`
+      const int at = used + (touch * 3 + comp_index(ce)) * n + ak - lo;
+      done = row_exists(cb, last, comp_index(ce)) && row_lo(cb, last) <= ak && ak <= row_hi(cb, last) &&
+             ldata[at] >= sv.tlen;
+    }
+    used += 12 * n;
+    if (touch < 4) break;
+  }
+  B.sv = sv; B.cb = cb; B.ce = ce;
+  B.num_null = 0;
+  B.lused = used;
+  B.status = done ? ST_END_REACHED : ST_OK; B.status_score = last * p.tg; B.end_k = ak;
+  if (G > 1) g.sync();
+  *s_out = last * p.tg;
+  return done ? 1 : 2;
 }
 
 // Leaf: wavefront_bialign_base -> unialign -> backtrace. Appends the leaf's ops to out.
-template <int G, bool TWO>
-__device__ __noinline__ int leaf_align(Dir& B, const PairSeqs& q, int pb, int pe, int tb, int te, int cb, int ce,
-                                       const Pen p, int max_steps, RunOut& out, uint32_t* lruns, int lruns_cap,
-                                       const Grp<G> g, int* max_leaf_score) {
-  g.sync();
-  dir_init<TWO>(B, fwd_view(q, pb, pe, tb, te), cb, ce);
+template <int G, bool TWO, bool TILES>
+__device__ __noinline__ int leaf_align(Dir& B, Dir& H, const PairSeqs& q, int pb, int pe, int tb, int te, int cb,
+                                       int ce, const Pen p, int max_steps, RunOut& out, uint32_t* lruns, int lruns_cap,
+                                       const Grp<G> g, int* max_leaf_score, int* part) {
   g.sync();
   const int guard = score_guard(p, pe - pb, te - tb);
-  int s = 0, ak = 0;
-  if (!dir_extend<G>(B, s, g, nullptr)) {
-    for (;;) {
-      ++s;
-      // wavefront_unialign_reached_limits checks the step count after compute, before extend
-      if (s >= max_steps) return WFG_ST_UNATTAINABLE;
-      if (s > guard) return WFG_ST_UNATTAINABLE;
-      const int q = dir_step<G, 1, TWO>(B, p, s, g, &ak);
-      if (q < 0) return WFG_ST_SCRATCH_OVERFLOW;
-      if (q) break;
-    }
+  const SeqView sv = fwd_view(q, pb, pe, tb, te);
+  int s = 0, ak = 0, state = 0;
+  if constexpr (TILES) {
+    if (p.tg) state = leaf_tiles<G>(B, H, sv, cb, ce, p, guard, g, part, &s);
+  }
+  if (state == 0) {
+    dir_init<TWO>(B, sv, cb, ce);
+    g.sync();
+    state = dir_extend<G>(B, s, g, nullptr) ? 1 : 2;
+  }
+  while (state == 2) {
+    ++s;
+    // wavefront_unialign_reached_limits checks the step count after compute, before extend
+    if (s >= max_steps) return WFG_ST_UNATTAINABLE;
+    if (s > guard) return WFG_ST_UNATTAINABLE;
+    const int q = dir_step<G, 1, TWO>(B, p, s, g, &ak);
+    if (q < 0) return WFG_ST_SCRATCH_OVERFLOW;
+    if (q) break;
   }
   if (*max_leaf_score < s) *max_leaf_score = s;
   if (B.status != ST_END_REACHED) return WFG_ST_UNATTAINABLE;
-  if (TWO) return leaf_backtrace_2p(B, p, s, ce, out, lruns, lruns_cap);
-  return leaf_backtrace<false>(B, p, s, ce, out, lruns, lruns_cap);
+  return leaf_backtrace<G, TWO>(B, p, s, ce, out, lruns, lruns_cap, g);
 }
 
 // cigar_score_gap_affine (alignment/cigar.c:277-303), cigar_score_gap_affine2p (:304-342: per
 // gap run the cheaper piece), cigar_score_gap_linear (:260-276; o is the indel penalty), or
 // cigar_score_edit (:244-259) for the edit and indel distances. The runs are maximal (adjacent
 // runs of one op are merged when emitted).
-__device__ __forceinline__ int rescore_runs(const uint32_t* runs, int n, int metric, int match, int x, int o, int e,
-                                            int o2, int e2) {
+__device__ __noinline__ int rescore_runs(const uint32_t* runs, int n, int metric, int match, int x, int o, int e,
+                                         int o2, int e2) {
   int score = 0;
-  for (int i = 0; i < n; ++i) {
+  for (int i = (int)(threadIdx.x & 31); i < n; i += 32) {  // a lane's runs
     const int op = (int)(runs[i] & 15u), len = (int)(runs[i] >> 4);
     if (metric == kMetricEdit || metric == kMetricIndel) { if (op != WFG_OP_EQ) score += len; continue; }
     if (metric == kMetricLinear) { score -= (op == WFG_OP_EQ ? match : op == WFG_OP_X ? x : o) * len; continue; }
@@ -1169,7 +1407,7 @@ __device__ __forceinline__ int rescore_runs(const uint32_t* runs, int n, int met
     else if (metric == kMetricAffine2p) score -= min(o + e * len, o2 + e2 * len);
     else score -= o + e * len;
   }
-  return score;
+  return __reduce_add_sync(kFull, score);
 }
 
 __device__ __forceinline__ int classic_score(int metric, int match_o, int plen, int tlen, int wf_score) {
@@ -1190,14 +1428,16 @@ struct GroupSmem {
   int2 rdesc[2][MS * 3];
   int rphys[2][MS];
   int red[8 * 8 + 8];
+  int part[4 * 8 * 5];  // tiles: each warp's antidiagonals and touch flag, 2 directions x 2 blocks
 };
 
 // G warps per pair, GROUPS groups per block. RING_SMEM: the two rings of each group live
 // in dynamic shared memory (sized by the host for ring_w); otherwise in the warp arena.
 // TWO: the two-piece gap-affine distance (five wavefront components); the other distances
 // run in the TWO = false instantiations. MS: the score scope cap (shared-memory ring
-// descriptors), 32 for the usual penalties and 64 for larger ones.
-template <int G, int GROUPS, bool RING_SMEM, int MINB, bool TWO, int MS>
+// descriptors), 32 for the usual penalties and 64 for larger ones. TILES: rows in tiles
+// (biwfa_tiles.cuh).
+template <int G, int GROUPS, bool RING_SMEM, int MINB, bool TWO, int MS, bool TILES>
 __global__ void __launch_bounds__(G * GROUPS * 32, MINB) biwfa_persistent_kernel(KernelParams P) {
   __shared__ GroupSmem<MS> s_grp[GROUPS];
   extern __shared__ __align__(16) int32_t s_ring_dyn[];
@@ -1210,10 +1450,11 @@ __global__ void __launch_bounds__(G * GROUPS * 32, MINB) biwfa_persistent_kernel
   const long long ggroup = (long long)blockIdx.x * GROUPS + gib;
   const int nphys = P.ring_nphys > 0 ? P.ring_nphys : P.scope;
   const int nc = TWO ? 5 : 3;
-  const ArenaLayout L = wfg_arena_layout(RING_SMEM ? 0 : nphys, P.ring_w, P.leaf_max_score, P.leaf_words,
+  constexpr int pad = TILES ? WFG_TILE_PAD : 0;
+  const ArenaLayout L = wfg_arena_layout(RING_SMEM ? 0 : nphys, P.ring_w + pad, P.leaf_max_score, P.leaf_words,
                                          P.run_cap, P.leaf_run_cap, P.stack_cap, nc);
   uint8_t* arena = P.arena + ggroup * P.arena_bytes;
-  const size_t ring_dir = (size_t)nphys * nc * P.ring_w;
+  const size_t ring_dir = (size_t)nphys * nc * (P.ring_w + pad);
   int32_t* ring = RING_SMEM ? s_ring_dyn + (size_t)gib * 2 * ring_dir : (int32_t*)(arena + L.ring_off);
   int4* ldesc = (int4*)(arena + L.ldesc_off);
   int32_t* ldata = (int32_t*)(arena + L.ldata_off);
@@ -1227,13 +1468,13 @@ __global__ void __launch_bounds__(G * GROUPS * 32, MINB) biwfa_persistent_kernel
   const uint32_t magic = (uint32_t)(0xffffffffu / (uint32_t)P.scope) + 1u;
   DirCfg fc{};
   int2* rdesc2 = (int2*)(arena + L.rdesc2_off);  // I2/D2 ring descriptors of both directions
-  fc.leaf = 0; fc.scope = P.scope; fc.magic = magic; fc.W = P.ring_w; fc.nphys = nphys; fc.lmax = 0; fc.nc = nc;
+  fc.leaf = 0; fc.scope = P.scope; fc.magic = magic; fc.W = P.ring_w; fc.pitch = P.ring_w + pad; fc.nphys = nphys; fc.lmax = 0; fc.nc = nc;
   fc.o2 = P.o2; fc.e2 = P.e2;
   fc.rdesc = S.rdesc[0]; fc.rdesc2 = rdesc2; fc.rphys = S.rphys[0]; fc.rdata = ring;
   DirCfg rc = fc;
   rc.rdesc = S.rdesc[1]; rc.rdesc2 = rdesc2 + kMaxScope2p * 2; rc.rphys = S.rphys[1]; rc.rdata = ring + ring_dir;
   DirCfg bcfg{};
-  bcfg.leaf = 1; bcfg.scope = P.scope; bcfg.magic = magic; bcfg.W = 0; bcfg.nphys = 1; bcfg.lmax = P.leaf_max_score;
+  bcfg.leaf = 1; bcfg.scope = P.scope; bcfg.magic = magic; bcfg.W = 0; bcfg.pitch = 0; bcfg.nphys = 1; bcfg.lmax = P.leaf_max_score;
   bcfg.nc = nc; bcfg.o2 = P.o2; bcfg.e2 = P.e2;
   bcfg.ldesc = ldesc; bcfg.ldata = ldata;
   F.cfg = fc; R.cfg = rc; B.cfg = bcfg;
@@ -1241,7 +1482,8 @@ __global__ void __launch_bounds__(G * GROUPS * 32, MINB) biwfa_persistent_kernel
   B.lcap = P.leaf_words; B.lused = 0;
   g.sync();
   const int go = P.metric == kMetricAffine ? P.o : P.metric == kMetricAffine2p ? max(P.o, P.o2) : 0;
-  const Pen pen = {P.x, P.o, P.e, P.scope, P.metric, go};
+  Pen pen = {P.x, P.o, P.e, P.scope, P.metric, go, 0, 0u};
+  F.ts.on = R.ts.on = B.ts.on = 0;
 
   const unsigned long long num_pairs =
       P.num_pairs_ptr ? *P.num_pairs_ptr : (unsigned long long)P.num_pairs;
@@ -1289,11 +1531,14 @@ __global__ void __launch_bounds__(G * GROUPS * 32, MINB) biwfa_persistent_kernel
       // diagonals [-plen-1, tlen+1], so a ring of next_pow2(plen+tlen+8) <= ring_w diagonals
       // never overflows; the two directions' rings are packed back to back at that width
       // (a smaller footprint per warp for short pairs).
-      const uint32_t need = (uint32_t)(pd.plen + pd.tlen + 8);
+      const uint32_t need = (uint32_t)(pd.plen + pd.tlen + 8 + (pad ? WFG_TILE_MARGIN : 0));
       const int wp = min(P.ring_w, max(64, (int)(1u << (32 - __clz((int)need - 1)))));
       F.cfg.W = wp; R.cfg.W = wp;
+      F.cfg.pitch = R.cfg.pitch = wp + pad;
       F.cfg.rdata = ring;
-      R.cfg.rdata = ring + (size_t)nphys * nc * wp;
+      R.cfg.rdata = ring + (size_t)nphys * nc * (wp + pad);
+      pen.tg = TILES && wp >= kTileMinRing ? P.tile_g : 0;
+      pen.tm = pen.tg > 1 ? 0xffffffffu / (uint32_t)pen.tg + 1u : 0u;
     }
     int status = ST_OK;
     int score = 0;
@@ -1303,7 +1548,8 @@ __global__ void __launch_bounds__(G * GROUPS * 32, MINB) biwfa_persistent_kernel
     if (P.score_only) {
       // wavefront_bialign_compute_score (wavefront/wavefront_bialign.c:662-699)
       BP bp;
-      const int st = find_breakpoint<G, TWO>(F, R, q, 0, q.plen, 0, q.tlen, CM, CM, pen, P.max_steps, bp, g);
+      const int st = find_breakpoint<G, TWO, TILES>(F, R, q, 0, q.plen, 0, q.tlen, CM, CM, pen, P.max_steps, bp, g,
+                                                       S.part);
       if (st == ST_OK || st == ST_END_REACHED) {
         const int wf = (st == ST_END_REACHED) ? (F.status == ST_END_REACHED ? F.status_score : R.status_score) : bp.score;
         score = classic_score(P.metric, P.match_o, q.plen, q.tlen, wf);
@@ -1333,19 +1579,19 @@ __global__ void __launch_bounds__(G * GROUPS * 32, MINB) biwfa_persistent_kernel
         if (tl == 0) { out.emit(WFG_OP_DEL, pl); continue; }
         if (pl == 0) { out.emit(WFG_OP_INS, tl); continue; }
         if (rem <= kFallbackMinScore) {
-          const int st = leaf_align<G, TWO>(B, q, pb, pe, tb, te, cb, ce, pen, P.max_steps, out, lruns, P.leaf_run_cap, g,
-                                       &max_leaf);
+          const int st = leaf_align<G, TWO, TILES>(B, F, q, pb, pe, tb, te, cb, ce, pen, P.max_steps, out, lruns,
+                                                 P.leaf_run_cap, g, &max_leaf, S.part);
           if (st != ST_OK) status = st;
           continue;
         }
         BP bp;
-        const int st = find_breakpoint<G, TWO>(F, R, q, pb, pe, tb, te, cb, ce, pen, P.max_steps, bp, g);
+        const int st = find_breakpoint<G, TWO, TILES>(F, R, q, pb, pe, tb, te, cb, ce, pen, P.max_steps, bp, g, S.part);
         if (st != ST_OK) {
           if (st == ST_END_REACHED) {
             const int reached = (F.status == ST_END_REACHED) ? F.status_score : R.status_score;
             if (reached <= kRecoveryMinScore) {
-              const int st2 = leaf_align<G, TWO>(B, q, pb, pe, tb, te, cb, ce, pen, P.max_steps, out, lruns,
-                                            P.leaf_run_cap, g, &max_leaf);
+              const int st2 = leaf_align<G, TWO, TILES>(B, F, q, pb, pe, tb, te, cb, ce, pen, P.max_steps, out, lruns,
+                                                   P.leaf_run_cap, g, &max_leaf, S.part);
               if (st2 != ST_OK) status = st2;
             } else {
               status = WFG_ST_UNATTAINABLE;
@@ -1461,54 +1707,57 @@ namespace {
 // Dynamic shared memory of the single-warp shape: the groups' packed-sequence slots.
 constexpr size_t kSeqSmemBytesG1 = (size_t)kG1Groups * kSeqSmemWords * sizeof(uint32_t);
 
-template <int G, int GROUPS, bool RS, int MINB, bool TWO, int MS>
+template <int G, int GROUPS, bool RS, int MINB, bool TWO, int MS, bool TILES>
 cudaError_t launch_shape(const KernelParams& p, int grid, cudaStream_t stream) {
   const size_t dyn = RS ? (size_t)GROUPS * 2 * (size_t)(p.ring_nphys > 0 ? p.ring_nphys : p.scope) * (TWO ? 5 : 3) *
                               (size_t)p.ring_w * sizeof(int32_t)
                         : (G == 1 ? kSeqSmemBytesG1 : 0);
   if (dyn > 0) {
-    const cudaError_t e = cudaFuncSetAttribute(biwfa_persistent_kernel<G, GROUPS, RS, MINB, TWO, MS>,
+    const cudaError_t e = cudaFuncSetAttribute(biwfa_persistent_kernel<G, GROUPS, RS, MINB, TWO, MS, TILES>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
     if (e != cudaSuccess) return e;
   }
-  biwfa_persistent_kernel<G, GROUPS, RS, MINB, TWO, MS><<<grid, G * GROUPS * 32, dyn, stream>>>(p);
+  biwfa_persistent_kernel<G, GROUPS, RS, MINB, TWO, MS, TILES><<<grid, G * GROUPS * 32, dyn, stream>>>(p);
   return cudaGetLastError();
 }
 
-template <int G, int GROUPS, bool RS, int MINB, bool TWO, int MS>
+template <int G, int GROUPS, bool RS, int MINB, bool TWO, int MS, bool TILES>
 cudaError_t occupancy_of(size_t dyn, int* blocks_per_sm) {
   if (dyn > 0) {
-    const cudaError_t e = cudaFuncSetAttribute(biwfa_persistent_kernel<G, GROUPS, RS, MINB, TWO, MS>,
+    const cudaError_t e = cudaFuncSetAttribute(biwfa_persistent_kernel<G, GROUPS, RS, MINB, TWO, MS, TILES>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
     if (e != cudaSuccess) return e;
   }
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm,
-                                                       biwfa_persistent_kernel<G, GROUPS, RS, MINB, TWO, MS>,
+                                                       biwfa_persistent_kernel<G, GROUPS, RS, MINB, TWO, MS, TILES>,
                                                        G * GROUPS * 32, dyn);
 }
 
-template <bool TWO, int MS>
+// The shared-memory rings of the 4- and 8-warp shapes hold a few rows, so those run without tiles.
+template <bool TWO, int MS, bool TILES>
 cudaError_t occupancy_shape(int gw, int ring_in_smem, size_t dyn, int* blocks_per_sm) {
-  if (gw <= 1) return occupancy_of<1, kG1Groups, false, g1_min_blocks<TWO>(), TWO, MS>(kSeqSmemBytesG1, blocks_per_sm);
+  if (gw <= 1)
+    return occupancy_of<1, kG1Groups, false, g1_min_blocks<TWO, TILES>(), TWO, MS, TILES>(kSeqSmemBytesG1, blocks_per_sm);
   if (gw == 8) {
-    if (ring_in_smem) return occupancy_of<8, 1, true, 1, TWO, MS>(dyn, blocks_per_sm);
-    return occupancy_of<8, 1, false, WFG_G8_MIN_BLOCKS, TWO, MS>(0, blocks_per_sm);
+    if (ring_in_smem) return occupancy_of<8, 1, true, 1, TWO, MS, false>(dyn, blocks_per_sm);
+    return occupancy_of<8, 1, false, TILES ? WFG_G8_TILES_MIN_BLOCKS : WFG_G8_MIN_BLOCKS, TWO, MS, TILES>(0, blocks_per_sm);
   }
-  if (ring_in_smem) return occupancy_of<4, 1, true, 1, TWO, MS>(dyn, blocks_per_sm);
-  return occupancy_of<4, 1, false, 3, TWO, MS>(0, blocks_per_sm);
+  if (ring_in_smem) return occupancy_of<4, 1, true, 1, TWO, MS, false>(dyn, blocks_per_sm);
+  return occupancy_of<4, 1, false, 3, TWO, MS, TILES>(0, blocks_per_sm);
 }
 
-template <bool TWO, int MS>
+template <bool TWO, int MS, bool TILES>
 cudaError_t launch_kernel(const KernelParams& p, int grid, cudaStream_t stream) {
   const int gw = p.group_warps > 0 ? p.group_warps : 1;
-  if (gw == 1) return launch_shape<1, kG1Groups, false, g1_min_blocks<TWO>(), TWO, MS>(p, grid, stream);
+  if (gw == 1)
+    return launch_shape<1, kG1Groups, false, g1_min_blocks<TWO, TILES>(), TWO, MS, TILES>(p, grid, stream);
   if (gw == 8) {
-    if (p.ring_in_smem) return launch_shape<8, 1, true, 1, TWO, MS>(p, grid, stream);
-    return launch_shape<8, 1, false, WFG_G8_MIN_BLOCKS, TWO, MS>(p, grid, stream);
+    if (p.ring_in_smem) return launch_shape<8, 1, true, 1, TWO, MS, false>(p, grid, stream);
+    return launch_shape<8, 1, false, TILES ? WFG_G8_TILES_MIN_BLOCKS : WFG_G8_MIN_BLOCKS, TWO, MS, TILES>(p, grid, stream);
   }
   if (gw == 4) {
-    if (p.ring_in_smem) return launch_shape<4, 1, true, 1, TWO, MS>(p, grid, stream);
-    return launch_shape<4, 1, false, 3, TWO, MS>(p, grid, stream);
+    if (p.ring_in_smem) return launch_shape<4, 1, true, 1, TWO, MS, false>(p, grid, stream);
+    return launch_shape<4, 1, false, 3, TWO, MS, TILES>(p, grid, stream);
   }
   return cudaErrorInvalidValue;
 }
@@ -1518,21 +1767,23 @@ cudaError_t launch_kernel(const KernelParams& p, int grid, cudaStream_t stream) 
 int biwfa_warps_per_block() { return kG1Groups; }
 
 cudaError_t biwfa_occupancy(int* blocks_per_sm) {
-  return occupancy_of<1, kG1Groups, false, g1_min_blocks<false>(), false, kMaxScope>(kSeqSmemBytesG1, blocks_per_sm);
+  return occupancy_of<1, kG1Groups, false, g1_min_blocks<false, false>(), false, kMaxScope, false>(kSeqSmemBytesG1,
+                                                                                                    blocks_per_sm);
 }
 
 // The kernel instantiation of a launch: 0 three components (scope <= 32), 1 three components
-// (scope <= 64), 2 two-piece gap-affine (scope <= 64).
-int biwfa_kernel_kind(int metric, int scope) {
-  return metric == kMetricAffine2p ? 2 : (scope > kMaxScope ? 1 : 0);
+// (scope <= 64), 2 two-piece gap-affine (scope <= 64), 3 three components with rows in tiles.
+int biwfa_kernel_kind(int metric, int scope, int tile_g) {
+  return tile_g > 0 ? 3 : metric == kMetricAffine2p ? 2 : (scope > kMaxScope ? 1 : 0);
 }
 
 // Resident blocks per SM of a shape (dyn: its dynamic shared memory in bytes; kind: as
 // biwfa_kernel_kind).
 cudaError_t biwfa_occupancy_shape(int gw, int ring_in_smem, size_t dyn, int* blocks_per_sm, int kind) {
-  if (kind == 2) return occupancy_shape<true, kMaxScope2p>(gw, ring_in_smem, dyn, blocks_per_sm);
-  if (kind == 1) return occupancy_shape<false, kMaxScope2p>(gw, ring_in_smem, dyn, blocks_per_sm);
-  return occupancy_shape<false, kMaxScope>(gw, ring_in_smem, dyn, blocks_per_sm);
+  if (kind == 3) return occupancy_shape<false, kMaxScope, true>(gw, ring_in_smem, dyn, blocks_per_sm);
+  if (kind == 2) return occupancy_shape<true, kMaxScope2p, false>(gw, ring_in_smem, dyn, blocks_per_sm);
+  if (kind == 1) return occupancy_shape<false, kMaxScope2p, false>(gw, ring_in_smem, dyn, blocks_per_sm);
+  return occupancy_shape<false, kMaxScope, false>(gw, ring_in_smem, dyn, blocks_per_sm);
 }
 
 // Groups (pairs in flight) per block of a shape.
@@ -1542,10 +1793,11 @@ int biwfa_groups_per_block(int group_warps, int ring_in_smem) {
 }
 
 cudaError_t launch_biwfa(const KernelParams& p, int grid, cudaStream_t stream) {
-  const int kind = biwfa_kernel_kind(p.metric, p.scope);
-  if (kind == 2) return launch_kernel<true, kMaxScope2p>(p, grid, stream);
-  if (kind == 1) return launch_kernel<false, kMaxScope2p>(p, grid, stream);
-  return launch_kernel<false, kMaxScope>(p, grid, stream);
+  const int kind = biwfa_kernel_kind(p.metric, p.scope, p.tile_g);
+  if (kind == 3) return launch_kernel<false, kMaxScope, true>(p, grid, stream);
+  if (kind == 2) return launch_kernel<true, kMaxScope2p, false>(p, grid, stream);
+  if (kind == 1) return launch_kernel<false, kMaxScope2p, false>(p, grid, stream);
+  return launch_kernel<false, kMaxScope, false>(p, grid, stream);
 }
 
 cudaError_t launch_pack(int n, const uint8_t* ascii, PairDesc* pairs, uint32_t* words, int num_sms,

@@ -87,6 +87,8 @@ struct KernelParams {
   int group_warps;
   int ring_in_smem;
   int ring_nphys;
+  // rows in tiles (biwfa_tiles.cuh): the spacing of the scores that hold a row, 0 for one score at a time
+  int tile_g;
 };
 
 // Score scope caps (max(x, o+e[, o2+e2]) + 1 after the match transform): the ring descriptors
@@ -94,6 +96,13 @@ struct KernelParams {
 // penalties; 64 for larger ones and for two-piece gap-affine).
 #define WFG_MAX_SCOPE 32
 #define WFG_MAX_SCOPE_2P 64
+
+// Rows in tiles: ring buffers per direction, ints between the end of a ring row and the next (a
+// pitch that is no power of two spreads the rows over the caches' sets), and the diagonals beyond
+// a pair's own that a ring row must hold (the last tile's unused lanes and the halos).
+#define WFG_TILE_BUFS 12
+#define WFG_TILE_PAD 64
+#define WFG_TILE_MARGIN 160
 
 // Physical ring buffers a direction needs: scores that can hold a wavefront are multiples of
 // g = gcd(x, o+e, e), so any window of `scope` consecutive scores holds at most ceil(scope/g)

@@ -203,6 +203,7 @@ namespace {
 struct IntPen {
   int x, o, e, scope, nphys;
   int o2 = 0, e2 = 0, nc = 3, emin = 1, g = 1;
+  int tile_g = 0;  // rows in tiles (biwfa_tiles.cuh): score spacing, 0 for one score at a time
 };
 IntPen internal_penalties(const wfg_config_t* cfg) {
   IntPen p;
@@ -270,6 +271,7 @@ int leaf_score_bound(const IntPen& p) {
 struct Launch {
   int gw = 1;            // warps per pair
   int smem = 0;          // rings in shared memory
+  int nphys = 0;         // ring buffers per direction
   int ring_w = 0, leaf_words = 0, leaf_max_score = 0, run_cap = 0, leaf_run_cap = 0, stack_cap = 0;
   int64_t groups = 0;    // pairs in flight
   bool batched = false;  // consecutive launches of `groups` pairs each instead of one persistent launch
@@ -282,7 +284,8 @@ struct Launch {
 // cap) and a small leaf store; the retry passes size rings from the longest pair.
 void size_launch(const wfg_context* c, const IntPen& p, int pass, int ring_w_hint, Launch& s) {
   const int maxsum = std::max(c->max_sum, 1);
-  const uint32_t ring_full = next_pow2((uint64_t)maxsum + 8);
+  const bool tiles = p.tile_g > 0 && !s.smem;
+  const uint32_t ring_full = next_pow2((uint64_t)maxsum + 8 + (tiles ? WFG_TILE_MARGIN : 0));
   s.leaf_max_score = leaf_score_bound(p);
   s.run_cap = maxsum + 2;
   s.leaf_run_cap = maxsum + 2;
@@ -319,7 +322,8 @@ void size_launch(const wfg_context* c, const IntPen& p, int pass, int ring_w_hin
     if (w < 64) s.smem = 0;
     else s.ring_w = std::min(s.ring_w, w);
   }
-  s.L = wfg_arena_layout(s.smem ? 0 : p.nphys, s.ring_w, s.leaf_max_score, s.leaf_words, s.run_cap, s.leaf_run_cap,
+  s.nphys = tiles && !s.smem ? WFG_TILE_BUFS : p.nphys;
+  s.L = wfg_arena_layout(s.smem ? 0 : s.nphys, s.ring_w + (tiles && !s.smem ? WFG_TILE_PAD : 0), s.leaf_max_score, s.leaf_words, s.run_cap, s.leaf_run_cap,
                          s.stack_cap, p.nc);
 }
 
@@ -327,7 +331,7 @@ void size_launch(const wfg_context* c, const IntPen& p, int pass, int ring_w_hin
 int64_t max_groups(const wfg_context* c, const IntPen& p, const Launch& l) {
   const size_t dyn = l.smem ? (size_t)2 * p.nphys * p.nc * (size_t)l.ring_w * sizeof(int32_t) : 0;
   int bps = 0;
-  if (biwfa_occupancy_shape(l.gw, l.smem, dyn, &bps, biwfa_kernel_kind(p.nc == 5 ? 4 : 0, p.scope)) != cudaSuccess ||
+  if (biwfa_occupancy_shape(l.gw, l.smem, dyn, &bps, biwfa_kernel_kind(p.nc == 5 ? 4 : 0, p.scope, l.smem ? 0 : p.tile_g)) != cudaSuccess ||
       bps < 1) {
     (void)cudaGetLastError();
     bps = 1;
@@ -366,7 +370,8 @@ KernelParams launch_params(const wfg_context* c, const wfg_config_t* cfg, const 
   kp.stats = nullptr;
   kp.group_warps = l.gw;
   kp.ring_in_smem = l.smem;
-  kp.ring_nphys = p.nphys;
+  kp.ring_nphys = l.nphys;
+  kp.tile_g = l.smem ? 0 : p.tile_g;
   kp.retry_out = (ps + 1 < kNumPasses) ? c->d_retry.ptr + (size_t)ps * n : nullptr;
   kp.retry_count = c->d_counters.ptr + ps * kCountersPerPass + 1;
   return kp;
@@ -445,6 +450,13 @@ int validate_config(wfg_context* c, const wfg_config_t* cfg, IntPen* p) {
     c->err = "max_score_scope above 64 is not supported";
     return WF_STATUS_UNSUPPORTED;
   }
+  // Rows in tiles: gap-affine penalties with x = 2e, o + e = 4e (the defaults 4/6/2 among them)
+  // within the usual kernels' score scope, the ratio that the tiles' row recurrence is written for;
+  // other ratios and distances take one score at a time. A step limit that a score can reach counts
+  // single scores. 10,000 pairs of 1 kbp: 7.7 ms one score at a time, 3.8 ms in tiles.
+  if (cfg->metric == WFG_METRIC_GAP_AFFINE && p->x == 2 * p->e && p->o == 3 * p->e && p->scope <= WFG_MAX_SCOPE &&
+      (cfg->max_alignment_steps <= 0 || cfg->max_alignment_steps >= (1 << 28)))
+    p->tile_g = p->e;
   if ((int64_t)(c->max_sum + 16) * (int64_t)std::max(p->x, std::max(p->o + p->e, p->o2 + p->e2)) >= ((int64_t)1 << 26)) {
     c->err = "pair too long for 27-bit scores";
     return WF_STATUS_UNSUPPORTED;
@@ -545,7 +557,7 @@ int wfg_run(wfg_context_t* c, const wfg_config_t* cfg, wfg_sched_t sched) {
         ++n_long;
     if (n_long > 0) {
       Launch lw; lw.gw = c->tune.retry_warps; lw.count = n_long; lw.order_off = 0;
-      lw.ring_w = (int)next_pow2((uint64_t)c->max_sum + 8);
+      lw.ring_w = (int)next_pow2((uint64_t)c->max_sum + 8);  // capped at the full width
       first.push_back(lw);
     }
     if (n - n_long > 0 || first.empty()) {
@@ -559,7 +571,7 @@ int wfg_run(wfg_context_t* c, const wfg_config_t* cfg, wfg_sched_t sched) {
   const int64_t arena_budget = arena_budget_of(c);
   int64_t pass0_bytes = 0;
   for (Launch& l : first) {
-    const int hint = l.ring_w > 0 ? l.ring_w : c->limit_ring_w;
+    const int hint = l.ring_w > 0 ? l.ring_w + (p.tile_g ? WFG_TILE_MARGIN : 0) : c->limit_ring_w;
     plan_first_pass(c, p, hint, arena_budget / (int64_t)first.size(), l);
     l.arena_off = pass0_bytes;
     pass0_bytes += l.groups * l.L.total;
@@ -920,7 +932,7 @@ int align_host_pipelined(wfg_context* c, const wfg_config_t* cfg, wfg_sched_t sc
       WFG_CHECK(c, cudaEventSynchronize(ready));
       float max_pred;
       memcpy(&max_pred, &c->h_bin_stats.ptr[4 * k + 2], sizeof(float));
-      hint = (int)(c->tune.ring_margin * max_pred / p.emin) + 64;
+      hint = (int)(c->tune.ring_margin * max_pred / p.emin) + 64 + (p.tile_g ? WFG_TILE_MARGIN : 0);
     }
     plan_first_pass(c, p, hint, budget, l);
     if (l.groups * l.L.total > region) {

@@ -1,0 +1,59 @@
+"""Rows in tiles (csrc/biwfa_tiles.cuh) against the oracle, bit for bit: wavefronts that end at and
+around the tiles' edges, rows that touch an end early (very different lengths, long gaps), pairs
+with bytes outside ACGT, every shape, and penalties of the tiles' ratio with other score spacings."""
+import numpy as np
+import pytest
+
+import biwfa_gpu_pii2025_gb300 as pkg
+from oracle import binding
+
+pytestmark = pytest.mark.gpu
+
+
+def _mutated(rng, p, edits, gap):
+    t = list(p)
+    for _ in range(edits):
+        j, kind, g = int(rng.integers(0, len(t) + 1)), rng.integers(0, 3), int(rng.integers(1, gap + 1))
+        if kind == 0:
+            t[j:j + g] = []
+        elif kind == 1:
+            t[j:j] = list(rng.choice(list(b"ACGT"), g))
+        elif j < len(t):
+            t[j] = int(rng.choice(list(b"ACGT")))
+    return bytes(np.array(t, np.uint8))
+
+
+def _batch(seed):
+    rng = np.random.default_rng(seed)
+
+    def seq(n, alphabet=b"ACGT"):
+        return bytes(rng.choice(list(alphabet), n).astype(np.uint8))
+
+    pairs = [(b"", b"ACG"), (b"A", b"A"), (b"A", b"C"), (b"ACGT" * 60, b"ACGT" * 60), (seq(700), seq(40)),
+             (seq(30), seq(900)), (seq(400), seq(400)), (b"A" * 150, b"A" * 90 + b"C" * 60)]
+    for n in (5, 31, 33, 64, 101, 130, 250, 500, 900, 1600):  # edits: wavefronts 0 - 400 diagonals wide
+        for edits in (0, 1, 3, n // 20, n // 8):
+            p = seq(n, b"ACGT" if edits != 3 else b"ACGTN")
+            pairs.append((p, _mutated(rng, p, edits, 1 + edits % 3)))
+        p = seq(n)
+        pairs.append((p, _mutated(rng, p, 4, 80)))  # long gaps
+    return pkg.PairBatch.from_lists([p for p, _ in pairs], [t for _, t in pairs])
+
+
+@pytest.mark.parametrize("pen,gw,seed", [((0, 4, 6, 2), 1, 1), ((0, 4, 6, 2), 4, 2), ((0, 4, 6, 2), 8, 3),
+                                         ((0, 2, 3, 1), 1, 4), ((0, 6, 9, 3), 1, 5), ((0, 14, 21, 7), 8, 6)])
+def test_tiles_match_oracle(batch_aligner, pen, gw, seed):
+    b = _batch(seed)
+    try:
+        batch_aligner.set_exec_shape(gw, False)
+        res = batch_aligner.align(b, penalties=pen)
+        only = batch_aligner.align(b, penalties=pen, score_only=True)
+    finally:
+        batch_aligner.set_exec_shape(1, False)
+    assert (res.status == 0).all()
+    for i in range(b.n):
+        _, score, ops, _ = binding.oracle_align(b.pattern(i), b.text(i), pen)
+        assert pkg.runs_to_ops(res.runs_of(i)) == ops, (i, b.plen[i], b.tlen[i])
+        assert res.scores[i] == (score if ops else 0), i
+        st, score, _, _ = binding.oracle_align(b.pattern(i), b.text(i), pen, score_only=True)
+        assert only.status[i] == st and (st != 0 or only.scores[i] == score), i
