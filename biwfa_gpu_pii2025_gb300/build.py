@@ -38,7 +38,7 @@ def nvcc_path() -> str:
 def _compile(src: str) -> Path:
     out = BUILD / (Path(src).stem + ".o")
     srcp = CSRC / src
-    deps = [srcp, CSRC / "biwfa_tiles.cuh", CSRC / "wfg_internal.h", CSRC / "wfg_context.h", ROOT / "include" / "wfa_gpu.h"]
+    deps = [srcp, CSRC / "biwfa_tiles.cuh", CSRC / "biwfa_tile_kernel.cuh", CSRC / "wfg_internal.h", CSRC / "wfg_context.h", ROOT / "include" / "wfa_gpu.h"]
     if out.exists() and all(out.stat().st_mtime >= d.stat().st_mtime for d in deps if d.exists()):
         return out
     lang = [] if src.endswith(".cu") else ["-x", "cu"] if src.endswith("_kernel.cpp") else []

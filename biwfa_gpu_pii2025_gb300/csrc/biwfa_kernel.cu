@@ -40,9 +40,6 @@ constexpr int kMaxScope2p = WFG_MAX_SCOPE_2P;  // the cap of the large-scope and
 #ifndef WFG_G1_WARPS5
 #define WFG_G1_WARPS5 28
 #endif
-#ifndef WFG_G1_WARPS_TILES
-#define WFG_G1_WARPS_TILES 20
-#endif
 #ifndef WFG_STEP_UNROLL
 #define WFG_STEP_UNROLL 2
 #endif
@@ -55,16 +52,9 @@ constexpr int kMaxScope2p = WFG_MAX_SCOPE_2P;  // the cap of the large-scope and
 // per block (measured equal to four: 2,457 vs 2,459 ms) lets each warp retire on its own when
 // its queue drains, so a launch that follows on another stream takes over warp slots at once
 // instead of waiting for whole blocks.
-// With rows in tiles a lane holds up to 40 offsets in registers: 20 warps per SM (96 registers).
-// Measured end to end against 24 and 28 warps (same GB300): 20,000 uneven pairs 103.7 ms (109, 119),
-// 150,000 mixture pairs 192.5 ms (205, 217), 10,000 1 kbp pairs 3.78 ms (3.71, 3.76), 200,000 150 bp
-// pairs 13.5 ms (12.7, 12.2); 16 warps (128 registers) within 1 % of 20. The 8-warp shape keeps two
-// blocks per SM (128 registers): 48 pairs of 10-20 kbp 117 ms, three blocks 130 ms, four 148 ms.
 constexpr int kG1Groups = WFG_G1_GROUPS;
-template <bool TWO, bool TILES>
-constexpr int g1_min_blocks() {
-  return (TILES ? WFG_G1_WARPS_TILES : TWO ? WFG_G1_WARPS5 : WFG_G1_WARPS3) / kG1Groups;
-}
+template <bool TWO>
+constexpr int g1_min_blocks() { return (TWO ? WFG_G1_WARPS5 : WFG_G1_WARPS3) / kG1Groups; }
 #ifndef WFG_LEAF_UNROLL
 #define WFG_LEAF_UNROLL 1
 #endif
@@ -168,9 +158,6 @@ __device__ __forceinline__ uint32_t win32(const uint32_t* w, int pos, int bshift
 // with two (127 registers, no spills).
 #ifndef WFG_G8_MIN_BLOCKS
 #define WFG_G8_MIN_BLOCKS 4
-#endif
-#ifndef WFG_G8_TILES_MIN_BLOCKS
-#define WFG_G8_TILES_MIN_BLOCKS 2
 #endif
 
 #if WFG_LCP64 >= 1
@@ -820,9 +807,10 @@ __device__ __noinline__ int dir_step(Dir& d, const Pen p, int s, const Grp<G> g,
   return 0;
 }
 
+struct BP { int score, sf, sr, kf, kr, of, orv, comp; };
+
 #include "biwfa_tiles.cuh"
 
-struct BP { int score, sf, sr, kf, kr, of, orv, comp; };
 
 // wavefront_bialign_breakpoint_indel2indel / _m2m: the first k0 (ascending) that meets,
 // found with a ballot per 32 diagonals (and the lowest hitting warp for G > 1).
@@ -951,15 +939,16 @@ __device__ __forceinline__ int score_guard(const Pen& p, int plen, int tlen) {
 }
 
 // The breakpoint search score by score from (sf, sr): resume 0 starts it, 1 and 2 enter the second
-// loop before the step of R or of F.
+// loop before the step of R or of F. TILES: one warp, rows that the tile kernel computed ahead come
+// first.
 template <int G, bool TWO, bool TILES>
 __device__ __noinline__ int breakpoint_steps(Dir& F, Dir& R, int sf, int sr, int fmax, int rmax, bool last_fwd,
-                                             int resume, int guard, const Pen p, int max_steps, BP& bp, const Grp<G> g,
-                                             int* part) {
+                                             int resume, int guard, const Pen p, int max_steps, BP& bp,
+                                             const Grp<G> g) {
   const int max_antidiag = F.sv.plen + F.sv.tlen - 1;
   int ak = 0;
   auto step = [&](Dir& d, int s) -> int {
-    if constexpr (TILES) return tile_advance<G>(d, p, s, g, part + (&d == &R ? 2 * (G * 5) : 0), &ak);
+    if constexpr (TILES) return tile_advance(d, p, s, g, &ak);
     else return dir_step<G, 0, TWO>(d, p, s, g, &ak);
   };
   while (resume == 0) {
@@ -1010,178 +999,20 @@ __device__ __noinline__ int breakpoint_steps(Dir& F, Dir& R, int sf, int sr, int
   return ST_OK;
 }
 
-// Whether direction d has row t (computing its block if need be) and the row does not touch.
-template <int G>
-__device__ __forceinline__ bool tile_ready(Dir& d, int t, const Grp<G>& g, int* part) {
-  if (t > d.ts.valid && (d.ts.touched || !tile_next<G>(d, g, part))) return false;
-  return !(d.ts.touched && t == d.ts.valid);
-}
-
-// wavefront_bialign_overlap over untouched rows: row s0 of d0 against the rows of scores s1,
-// s1 - 1, ... of d1. Cells meet where their antidiagonals add up to plen + tlen or more, so the
-// lanes first test the rows' largest ones, a row pair each, and only pairs that pass are scanned.
-// An untouched row's I and D offsets are at most M's on the same diagonal, so a scan reads M and
-// looks at D and I only where M meets. D comes first, then I, then M, the lowest diagonal of each.
-template <int G>
-__device__ __noinline__ void tile_overlap(const Dir& d0, const Dir& d1, int s0, int s1, bool fwd, BP& bp, const Pen& p,
-                                          const Grp<G> g) {
-  const int t0 = row_of(s0, p), cb0 = d0.cb, cb1 = d1.cb;
-  if (!row_exists(cb0, t0, 0)) return;
-  const int plen = d0.sv.plen, tlen = d0.sv.tlen, A = tlen - plen;
-  const int mine = s1 - g.lane();
-  unsigned todo = __ballot_sync(kFull, g.lane() < p.scope && mine >= 0 && holds_row(mine, p) &&
-                                           d0.ts.akr[row_buffer(t0)] + d1.ts.akr[row_buffer(row_of(max(mine, 0), p))] >=
-                                               plen + tlen);
-  const uint32_t mask = (uint32_t)d0.cfg.W - 1u;
-  const int pitch = d0.cfg.pitch;
-  const int32_t* r0 = d0.cfg.rdata + row_buffer(t0) * 3 * pitch;
-  while (todo) {
-    const int s = s1 - (__ffs((int)todo) - 1);
-    todo &= todo - 1;
-    if (s0 + s - p.go >= bp.score) continue;
-    const int t1 = row_of(s, p);
-    const int32_t* r1 = d1.cfg.rdata + row_buffer(t1) * 3 * pitch;
-    const int end = min(row_hi(cb0, t0), A - row_lo(cb1, t1));
-    int first[3] = {INT_MAX, INT_MAX, INT_MAX};  // lowest diagonal where M, I, D meet
-    #pragma unroll 1
-    for (int kb = max(row_lo(cb0, t0), A - row_hi(cb1, t1)) + 32 * g.warp(); kb <= end; kb += 32 * G) {
-      const int k = kb + g.lane();
-      const uint32_t i0 = (uint32_t)k & mask, i1 = (uint32_t)(A - k) & mask;
-      const bool hit = k <= end && r0[i0] + r1[i1] >= tlen;
-      if (!__any_sync(kFull, hit)) continue;
-      if (hit) {
-        first[0] = min(first[0], k);
-        if (r0[pitch + i0] + r1[pitch + i1] >= tlen) first[1] = min(first[1], k);
-        if (r0[2 * pitch + i0] + r1[2 * pitch + i1] >= tlen) first[2] = min(first[2], k);
-      }
-    }
-    const bool mn[3] = {false, false, false};
-    g.minmax(first, mn);
-    const int ci = first[2] != INT_MAX ? 2 : first[1] != INT_MAX ? 1 : 0;
-    const int k = ci == 2 ? first[2] : ci == 1 ? first[1] : first[0];
-    const int cand = ci ? s0 + s - p.o : s0 + s;
-    if (k == INT_MAX || cand >= bp.score) continue;
-    const int o0 = r0[ci * pitch + ((uint32_t)k & mask)], o1 = r1[ci * pitch + ((uint32_t)(A - k) & mask)];
-    bp.score = cand;
-    bp.comp = ci == 2 ? CD : ci == 1 ? CI : CM;
-    bp.sf = fwd ? s0 : s; bp.sr = fwd ? s : s0;
-    bp.kf = fwd ? k : A - k; bp.kr = fwd ? A - k : k;
-    bp.of = fwd ? o0 : o1; bp.orv = fwd ? o1 : o0;
-  }
-}
-
-// The breakpoint search over rows in tiles (biwfa_tiles.cuh). Both directions' blocks are computed
-// until one may hold an event: the antidiagonals add up, or a row touches an end. Its rows are then
-// replayed up to the event; the second phase scans the rows' meetings and computes further blocks
-// when it runs out of rows. A touched row, or a full ring, leaves to breakpoint_steps. Returns
-// ST_OK etc. as find_breakpoint, or INT_MAX when the first cell already touches.
-template <int G>
-__device__ __noinline__ int breakpoint_tiles(Dir& F, Dir& R, const PairSeqs& q, int pb, int pe, int tb, int te, int cb,
-                                             int ce, const Pen p, int guard, BP& bp, const Grp<G> g, int* part) {
-  const int max_antidiag = pe - pb + te - tb - 1;
-  int* part_r = part + 2 * (G * 5);
-  if (tile_start<G>(F, fwd_view(q, pb, pe, tb, te), cb, ce, g) < 0) return INT_MAX;
-  if (tile_start<G>(R, rev_view(q, pb, pe, tb, te), ce, cb, g) < 0) return INT_MAX;
-  g.sync();
-  int fmax = F.ts.akr[row_buffer(0)], rmax = R.ts.akr[row_buffer(0)];
-  int sf = 0, sr = 0, resume = 0;
-  bool last_fwd = false, steps = false;
-  if (fmax + rmax < max_antidiag) {
-    int t = 0;
-    for (;;) {
-      if (!tile_fits(F, t) || !tile_fits(R, t)) { steps = true; break; }
-      int* mf = part + ((t >> 2) & 1) * (G * 5);
-      int* mr = part_r + ((t >> 2) & 1) * (G * 5);
-      const TilePlan pf = tile_plan(cb, t, 32);
-      // one warp: both directions in one pass while half a warp holds each; else the warps take F's
-      // tiles in turn, then R's from where F's ended
-      const bool pair = G == 1 && row_hi(cb, t + 4) - (row_lo(cb, t + 4) & ~3) < 64 &&
-                        row_hi(ce, t + 4) - (row_lo(ce, t + 4) & ~3) < 64;
-      #pragma unroll 1
-      for (int d = 0; d < (pair ? 1 : 2); ++d)
-        tile_run(d ? R : F, R, pair, t, G == 1 ? 0 : d ? (g.warp() + G - pf.tiles % G) % G : g.warp(), G, nullptr, 0, 0,
-                 g.lane(), (d ? mr : mf) + g.warp() * 5, mr);
-      g.sync();
-      const int ft = tile_combine<G>(F, t, mf, g), rt = tile_combine<G>(R, t, mr, g);
-      const bool both = tile_narrow(cb, t, 16) && tile_narrow(ce, t, 16);
-      tile_done(F, t, ft, pair, pair ? both : tile_narrow(cb, t, 32));
-      tile_done(R, t, rt, pair, pair ? both : tile_narrow(ce, t, 32));
-      const int* fa = F.ts.akr + row_buffer(t + 1);
-      const int* ra = R.ts.akr + row_buffer(t + 1);
-      const int nf = max(fmax, max(max(fa[0], fa[1]), max(fa[2], fa[3])));
-      const int nr = max(rmax, max(max(ra[0], ra[1]), max(ra[2], ra[3])));
-      if (min(ft, rt) == 4 && nf + nr < max_antidiag) {
-        fmax = nf; rmax = nr;
-        t += 4;
-        if (t > guard) return WFG_ST_UNATTAINABLE;
-        continue;
-      }
-      #pragma unroll 1
-      for (int j = 0; j < 4; ++j, ++t) {
-        sf = sr = (t + 1) * p.tg;
-        last_fwd = true;
-        if (ft == j) { steps = true; break; }
-        const int f1 = max(fmax, fa[j]);
-        if (f1 + rmax >= max_antidiag) { sr = sf - 1; break; }
-        if (rt == j) { steps = true; break; }
-        const int r1 = max(rmax, ra[j]);
-        last_fwd = false;
-        if (f1 + r1 >= max_antidiag) break;
-        fmax = f1; rmax = r1;
-      }
-      break;
-    }
-    if (steps) {  // the single steps start after row t
-      sf = sr = t * p.tg;
-      last_fwd = false;
-    }
-  }
-  while (!steps) {
-    if (last_fwd) {
-      const int min_sr = (sr > p.scope - 1) ? sr - (p.scope - 1) : 0;
-      if (sf + min_sr - p.go >= bp.score) return ST_OK;
-      if (holds_row(sf, p)) tile_overlap<G>(F, R, sf, sr, true, bp, p, g);
-      if (holds_row(sr + 1, p) && !tile_ready<G>(R, row_of(sr + 1, p), g, part_r)) { resume = 1; break; }
-      ++sr;
-    }
-    const int min_sf = (sf > p.scope - 1) ? sf - (p.scope - 1) : 0;
-    if (min_sf + sr - p.go >= bp.score) return ST_OK;
-    if (holds_row(sr, p)) tile_overlap<G>(R, F, sr, sf, false, bp, p, g);
-    last_fwd = true;
-    if (holds_row(sf + 1, p) && !tile_ready<G>(F, row_of(sf + 1, p), g, part)) { resume = 2; break; }
-    ++sf;
-    if (sf > guard + 2 * p.scope || sr > guard + 2 * p.scope) return WFG_ST_UNATTAINABLE;
-  }
-  if (G > 1) g.sync();
-  tile_describe(F, sf, sf - p.scope + 1, p);
-  tile_describe(R, sr, sr - p.scope + 1, p);
-  g.sync();
-  return breakpoint_steps<G, false, true>(F, R, sf, sr, fmax, rmax, last_fwd, resume, guard, p, INT_MAX, bp, g, part);
-}
-
 // wavefront_bialign_find_breakpoint
-template <int G, bool TWO, bool TILES>
+template <int G, bool TWO>
 __device__ __noinline__ int find_breakpoint(Dir& F, Dir& R, const PairSeqs& q, int pb, int pe, int tb, int te,
-                                            int cb, int ce, const Pen p, int max_steps, BP& bp, const Grp<G> g,
-                                            int* part) {
-  const int guard = score_guard(p, pe - pb, te - tb);
+                                            int cb, int ce, const Pen p, int max_steps, BP& bp, const Grp<G> g) {
   bp.score = INT_MAX;
   g.sync();
-  if constexpr (TILES) {
-    if (p.tg) {
-      const int st = breakpoint_tiles<G>(F, R, q, pb, pe, tb, te, cb, ce, p, guard, bp, g, part);
-      if (st != INT_MAX) return st;
-      g.sync();
-    }
-  }
   dir_init<TWO>(F, fwd_view(q, pb, pe, tb, te), cb, ce);
   dir_init<TWO>(R, rev_view(q, pb, pe, tb, te), ce, cb);
-  F.ts.on = R.ts.on = 0;
   g.sync();
   int fmax = 0, rmax = 0;
   if (dir_extend<G>(F, 0, g, &fmax)) return F.status;
   if (dir_extend<G>(R, 0, g, &rmax)) return R.status;
-  return breakpoint_steps<G, TWO, TILES>(F, R, 0, 0, fmax, rmax, false, 0, guard, p, max_steps, bp, g, part);
+  return breakpoint_steps<G, TWO, false>(F, R, 0, 0, fmax, rmax, false, 0, score_guard(p, pe - pb, te - tb), p, max_steps,
+                                         bp, g);
 }
 
 // Forward run list of the pair (the CIGAR being assembled), with the open run in registers.
@@ -1308,87 +1139,37 @@ __device__ __noinline__ int leaf_backtrace(const Dir& B, const Pen p, int s, int
   return ST_OK;
 }
 
-// The leaf's rows in tiles, up to its end or the first touched row that is not its end. The ring
-// of direction H holds the rows that the next block reads; the leaf store gets every row. Returns
-// 0 when the first cell touches (B is left as it was), 1 when the end is reached, else 2; *s_out:
-// the last score computed.
-template <int G>
-__device__ __noinline__ int leaf_tiles(Dir& B, Dir& H, const SeqView& sv, int cb, int ce, const Pen p, int guard,
-                                       const Grp<G> g, int* part, int* s_out) {
-  const int off0 = tile_start<G>(H, sv, cb, ce, g);
-  if (off0 < 0) return 0;
-  int4* ldesc = B.cfg.ldesc;
-  int32_t* ldata = B.cfg.ldata;
-  const int lmax = B.cfg.lmax, lcap = B.lcap, ak = sv.tlen - sv.plen;
-  if (g.tid < 3) ldesc[g.tid] = g.tid == comp_index(cb) ? make_int4(0, 0, 0, 0) : make_int4(kAbsent, INT_MIN, 0, 0);
-  if (g.tid == 0) ldata[0] = off0;
-  g.sync();
-  int used = 4, last = 0;
-  bool done = false;
-  #pragma unroll 1
-  for (int t0 = 0; t0 <= guard; t0 += 4) {
-    const int lo = row_lo(cb, t0 + 4) & ~3, n = (row_hi(cb, t0 + 4) - lo + 4) & ~3;
-    if ((t0 + 4) * p.tg > lmax || used + 12 * n > lcap || !tile_fits(H, t0)) break;
-    int* mine = part + ((t0 >> 2) & 1) * (G * 5);
-    tile_run(H, H, false, t0, g.warp(), G, ldata + used, lo, n, g.lane(), mine + g.warp() * 5, nullptr);
-    #pragma unroll 1
-    for (int i = g.tid; i < 4 * p.tg * 3; i += 32 * G) {
-      const int s = t0 * p.tg + 1 + i / 3, ci = i % 3, t = row_of(s, p);
-      int4 ds = make_int4(kAbsent, INT_MIN, 0, 0);
-      if (s == t * p.tg && row_exists(cb, t, ci))
-        ds = make_int4(row_lo(cb, t), row_hi(cb, t), used + ((t - t0 - 1) * 3 + ci) * n, lo);
-      ldesc[s * 3 + ci] = ds;
-    }
-    g.sync();
-    const int touch = tile_combine<G>(H, t0, mine, g);
-    tile_done(H, t0, touch, false, tile_narrow(cb, t0, 32));
-    last = H.ts.valid;
-    if (touch < 4) {  // the end diagonal's offset in row `last`
-      const int at = used + (touch * 3 + comp_index(ce)) * n + ak - lo;
-      done = row_exists(cb, last, comp_index(ce)) && row_lo(cb, last) <= ak && ak <= row_hi(cb, last) &&
-             ldata[at] >= sv.tlen;
-    }
-    used += 12 * n;
-    if (touch < 4) break;
-  }
-  B.sv = sv; B.cb = cb; B.ce = ce;
-  B.num_null = 0;
-  B.lused = used;
-  B.status = done ? ST_END_REACHED : ST_OK; B.status_score = last * p.tg; B.end_k = ak;
-  if (G > 1) g.sync();
-  *s_out = last * p.tg;
-  return done ? 1 : 2;
-}
-
-// Leaf: wavefront_bialign_base -> unialign -> backtrace. Appends the leaf's ops to out.
-template <int G, bool TWO, bool TILES>
-__device__ __noinline__ int leaf_align(Dir& B, Dir& H, const PairSeqs& q, int pb, int pe, int tb, int te, int cb,
-                                       int ce, const Pen p, int max_steps, RunOut& out, uint32_t* lruns, int lruns_cap,
-                                       const Grp<G> g, int* max_leaf_score, int* part) {
-  g.sync();
-  const int guard = score_guard(p, pe - pb, te - tb);
-  const SeqView sv = fwd_view(q, pb, pe, tb, te);
-  int s = 0, ak = 0, state = 0;
-  if constexpr (TILES) {
-    if (p.tg) state = leaf_tiles<G>(B, H, sv, cb, ce, p, guard, g, part, &s);
-  }
-  if (state == 0) {
-    dir_init<TWO>(B, sv, cb, ce);
-    g.sync();
-    state = dir_extend<G>(B, s, g, nullptr) ? 1 : 2;
-  }
-  while (state == 2) {
+// The leaf's steps from score s (wavefront_bialign_base -> unialign) and its backtrace; appends the
+// leaf's ops to out.
+template <int G, bool TWO>
+__device__ __noinline__ int leaf_finish(Dir& B, bool done, int s, int guard, const Pen p, int max_steps, RunOut& out,
+                                        uint32_t* lruns, int lruns_cap, const Grp<G> g, int* max_leaf_score) {
+  int ak = 0;
+  while (!done) {
     ++s;
     // wavefront_unialign_reached_limits checks the step count after compute, before extend
     if (s >= max_steps) return WFG_ST_UNATTAINABLE;
     if (s > guard) return WFG_ST_UNATTAINABLE;
     const int q = dir_step<G, 1, TWO>(B, p, s, g, &ak);
     if (q < 0) return WFG_ST_SCRATCH_OVERFLOW;
-    if (q) break;
+    done = q != 0;
   }
   if (*max_leaf_score < s) *max_leaf_score = s;
   if (B.status != ST_END_REACHED) return WFG_ST_UNATTAINABLE;
-  return leaf_backtrace<G, TWO>(B, p, s, ce, out, lruns, lruns_cap, g);
+  return leaf_backtrace<G, TWO>(B, p, s, B.ce, out, lruns, lruns_cap, g);
+}
+
+// Leaf: wavefront_bialign_base -> unialign -> backtrace.
+template <int G, bool TWO>
+__device__ __noinline__ int leaf_align(Dir& B, const PairSeqs& q, int pb, int pe, int tb, int te, int cb, int ce,
+                                       const Pen p, int max_steps, RunOut& out, uint32_t* lruns, int lruns_cap,
+                                       const Grp<G> g, int* max_leaf_score) {
+  g.sync();
+  dir_init<TWO>(B, fwd_view(q, pb, pe, tb, te), cb, ce);
+  g.sync();
+  const bool done = dir_extend<G>(B, 0, g, nullptr) != 0;
+  return leaf_finish<G, TWO>(B, done, 0, score_guard(p, pe - pb, te - tb), p, max_steps, out, lruns, lruns_cap, g,
+                             max_leaf_score);
 }
 
 // cigar_score_gap_affine (alignment/cigar.c:277-303), cigar_score_gap_affine2p (:304-342: per
@@ -1428,16 +1209,14 @@ struct GroupSmem {
   int2 rdesc[2][MS * 3];
   int rphys[2][MS];
   int red[8 * 8 + 8];
-  int part[4 * 8 * 5];  // tiles: each warp's antidiagonals and touch flag, 2 directions x 2 blocks
 };
 
 // G warps per pair, GROUPS groups per block. RING_SMEM: the two rings of each group live
 // in dynamic shared memory (sized by the host for ring_w); otherwise in the warp arena.
 // TWO: the two-piece gap-affine distance (five wavefront components); the other distances
 // run in the TWO = false instantiations. MS: the score scope cap (shared-memory ring
-// descriptors), 32 for the usual penalties and 64 for larger ones. TILES: rows in tiles
-// (biwfa_tiles.cuh).
-template <int G, int GROUPS, bool RING_SMEM, int MINB, bool TWO, int MS, bool TILES>
+// descriptors), 32 for the usual penalties and 64 for larger ones.
+template <int G, int GROUPS, bool RING_SMEM, int MINB, bool TWO, int MS>
 __global__ void __launch_bounds__(G * GROUPS * 32, MINB) biwfa_persistent_kernel(KernelParams P) {
   __shared__ GroupSmem<MS> s_grp[GROUPS];
   extern __shared__ __align__(16) int32_t s_ring_dyn[];
@@ -1450,11 +1229,10 @@ __global__ void __launch_bounds__(G * GROUPS * 32, MINB) biwfa_persistent_kernel
   const long long ggroup = (long long)blockIdx.x * GROUPS + gib;
   const int nphys = P.ring_nphys > 0 ? P.ring_nphys : P.scope;
   const int nc = TWO ? 5 : 3;
-  constexpr int pad = TILES ? WFG_TILE_PAD : 0;
-  const ArenaLayout L = wfg_arena_layout(RING_SMEM ? 0 : nphys, P.ring_w + pad, P.leaf_max_score, P.leaf_words,
+  const ArenaLayout L = wfg_arena_layout(RING_SMEM ? 0 : nphys, P.ring_w, P.leaf_max_score, P.leaf_words,
                                          P.run_cap, P.leaf_run_cap, P.stack_cap, nc);
   uint8_t* arena = P.arena + ggroup * P.arena_bytes;
-  const size_t ring_dir = (size_t)nphys * nc * (P.ring_w + pad);
+  const size_t ring_dir = (size_t)nphys * nc * P.ring_w;
   int32_t* ring = RING_SMEM ? s_ring_dyn + (size_t)gib * 2 * ring_dir : (int32_t*)(arena + L.ring_off);
   int4* ldesc = (int4*)(arena + L.ldesc_off);
   int32_t* ldata = (int32_t*)(arena + L.ldata_off);
@@ -1468,7 +1246,7 @@ __global__ void __launch_bounds__(G * GROUPS * 32, MINB) biwfa_persistent_kernel
   const uint32_t magic = (uint32_t)(0xffffffffu / (uint32_t)P.scope) + 1u;
   DirCfg fc{};
   int2* rdesc2 = (int2*)(arena + L.rdesc2_off);  // I2/D2 ring descriptors of both directions
-  fc.leaf = 0; fc.scope = P.scope; fc.magic = magic; fc.W = P.ring_w; fc.pitch = P.ring_w + pad; fc.nphys = nphys; fc.lmax = 0; fc.nc = nc;
+  fc.leaf = 0; fc.scope = P.scope; fc.magic = magic; fc.W = P.ring_w; fc.pitch = P.ring_w; fc.nphys = nphys; fc.lmax = 0; fc.nc = nc;
   fc.o2 = P.o2; fc.e2 = P.e2;
   fc.rdesc = S.rdesc[0]; fc.rdesc2 = rdesc2; fc.rphys = S.rphys[0]; fc.rdata = ring;
   DirCfg rc = fc;
@@ -1482,8 +1260,7 @@ __global__ void __launch_bounds__(G * GROUPS * 32, MINB) biwfa_persistent_kernel
   B.lcap = P.leaf_words; B.lused = 0;
   g.sync();
   const int go = P.metric == kMetricAffine ? P.o : P.metric == kMetricAffine2p ? max(P.o, P.o2) : 0;
-  Pen pen = {P.x, P.o, P.e, P.scope, P.metric, go, 0, 0u};
-  F.ts.on = R.ts.on = B.ts.on = 0;
+  const Pen pen = {P.x, P.o, P.e, P.scope, P.metric, go, 0, 0u};
 
   const unsigned long long num_pairs =
       P.num_pairs_ptr ? *P.num_pairs_ptr : (unsigned long long)P.num_pairs;
@@ -1531,14 +1308,12 @@ __global__ void __launch_bounds__(G * GROUPS * 32, MINB) biwfa_persistent_kernel
       // diagonals [-plen-1, tlen+1], so a ring of next_pow2(plen+tlen+8) <= ring_w diagonals
       // never overflows; the two directions' rings are packed back to back at that width
       // (a smaller footprint per warp for short pairs).
-      const uint32_t need = (uint32_t)(pd.plen + pd.tlen + 8 + (pad ? WFG_TILE_MARGIN : 0));
+      const uint32_t need = (uint32_t)(pd.plen + pd.tlen + 8);
       const int wp = min(P.ring_w, max(64, (int)(1u << (32 - __clz((int)need - 1)))));
       F.cfg.W = wp; R.cfg.W = wp;
-      F.cfg.pitch = R.cfg.pitch = wp + pad;
+      F.cfg.pitch = R.cfg.pitch = wp;
       F.cfg.rdata = ring;
-      R.cfg.rdata = ring + (size_t)nphys * nc * (wp + pad);
-      pen.tg = TILES && wp >= kTileMinRing ? P.tile_g : 0;
-      pen.tm = pen.tg > 1 ? 0xffffffffu / (uint32_t)pen.tg + 1u : 0u;
+      R.cfg.rdata = ring + (size_t)nphys * nc * wp;
     }
     int status = ST_OK;
     int score = 0;
@@ -1548,8 +1323,7 @@ __global__ void __launch_bounds__(G * GROUPS * 32, MINB) biwfa_persistent_kernel
     if (P.score_only) {
       // wavefront_bialign_compute_score (wavefront/wavefront_bialign.c:662-699)
       BP bp;
-      const int st = find_breakpoint<G, TWO, TILES>(F, R, q, 0, q.plen, 0, q.tlen, CM, CM, pen, P.max_steps, bp, g,
-                                                       S.part);
+      const int st = find_breakpoint<G, TWO>(F, R, q, 0, q.plen, 0, q.tlen, CM, CM, pen, P.max_steps, bp, g);
       if (st == ST_OK || st == ST_END_REACHED) {
         const int wf = (st == ST_END_REACHED) ? (F.status == ST_END_REACHED ? F.status_score : R.status_score) : bp.score;
         score = classic_score(P.metric, P.match_o, q.plen, q.tlen, wf);
@@ -1579,19 +1353,17 @@ __global__ void __launch_bounds__(G * GROUPS * 32, MINB) biwfa_persistent_kernel
         if (tl == 0) { out.emit(WFG_OP_DEL, pl); continue; }
         if (pl == 0) { out.emit(WFG_OP_INS, tl); continue; }
         if (rem <= kFallbackMinScore) {
-          const int st = leaf_align<G, TWO, TILES>(B, F, q, pb, pe, tb, te, cb, ce, pen, P.max_steps, out, lruns,
-                                                 P.leaf_run_cap, g, &max_leaf, S.part);
+          const int st = leaf_align<G, TWO>(B, q, pb, pe, tb, te, cb, ce, pen, P.max_steps, out, lruns, P.leaf_run_cap, g, &max_leaf);
           if (st != ST_OK) status = st;
           continue;
         }
         BP bp;
-        const int st = find_breakpoint<G, TWO, TILES>(F, R, q, pb, pe, tb, te, cb, ce, pen, P.max_steps, bp, g, S.part);
+        const int st = find_breakpoint<G, TWO>(F, R, q, pb, pe, tb, te, cb, ce, pen, P.max_steps, bp, g);
         if (st != ST_OK) {
           if (st == ST_END_REACHED) {
             const int reached = (F.status == ST_END_REACHED) ? F.status_score : R.status_score;
             if (reached <= kRecoveryMinScore) {
-              const int st2 = leaf_align<G, TWO, TILES>(B, F, q, pb, pe, tb, te, cb, ce, pen, P.max_steps, out, lruns,
-                                                   P.leaf_run_cap, g, &max_leaf, S.part);
+              const int st2 = leaf_align<G, TWO>(B, q, pb, pe, tb, te, cb, ce, pen, P.max_steps, out, lruns, P.leaf_run_cap, g, &max_leaf);
               if (st2 != ST_OK) status = st2;
             } else {
               status = WFG_ST_UNATTAINABLE;
@@ -1656,6 +1428,8 @@ __global__ void __launch_bounds__(G * GROUPS * 32, MINB) biwfa_persistent_kernel
   }
 }
 
+#include "biwfa_tile_kernel.cuh"
+
 // Pack ASCII pairs into the four word arrays per pair; pure ACGT pairs use 2 bits per base,
 // anything else keeps 8 bits so the comparison stays exact for every byte value.
 __global__ void pack_pairs_kernel(int n, const uint8_t* __restrict__ ascii, PairDesc* __restrict__ pairs,
@@ -1707,57 +1481,54 @@ namespace {
 // Dynamic shared memory of the single-warp shape: the groups' packed-sequence slots.
 constexpr size_t kSeqSmemBytesG1 = (size_t)kG1Groups * kSeqSmemWords * sizeof(uint32_t);
 
-template <int G, int GROUPS, bool RS, int MINB, bool TWO, int MS, bool TILES>
+template <int G, int GROUPS, bool RS, int MINB, bool TWO, int MS>
 cudaError_t launch_shape(const KernelParams& p, int grid, cudaStream_t stream) {
   const size_t dyn = RS ? (size_t)GROUPS * 2 * (size_t)(p.ring_nphys > 0 ? p.ring_nphys : p.scope) * (TWO ? 5 : 3) *
                               (size_t)p.ring_w * sizeof(int32_t)
                         : (G == 1 ? kSeqSmemBytesG1 : 0);
   if (dyn > 0) {
-    const cudaError_t e = cudaFuncSetAttribute(biwfa_persistent_kernel<G, GROUPS, RS, MINB, TWO, MS, TILES>,
+    const cudaError_t e = cudaFuncSetAttribute(biwfa_persistent_kernel<G, GROUPS, RS, MINB, TWO, MS>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
     if (e != cudaSuccess) return e;
   }
-  biwfa_persistent_kernel<G, GROUPS, RS, MINB, TWO, MS, TILES><<<grid, G * GROUPS * 32, dyn, stream>>>(p);
+  biwfa_persistent_kernel<G, GROUPS, RS, MINB, TWO, MS><<<grid, G * GROUPS * 32, dyn, stream>>>(p);
   return cudaGetLastError();
 }
 
-template <int G, int GROUPS, bool RS, int MINB, bool TWO, int MS, bool TILES>
+template <int G, int GROUPS, bool RS, int MINB, bool TWO, int MS>
 cudaError_t occupancy_of(size_t dyn, int* blocks_per_sm) {
   if (dyn > 0) {
-    const cudaError_t e = cudaFuncSetAttribute(biwfa_persistent_kernel<G, GROUPS, RS, MINB, TWO, MS, TILES>,
+    const cudaError_t e = cudaFuncSetAttribute(biwfa_persistent_kernel<G, GROUPS, RS, MINB, TWO, MS>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
     if (e != cudaSuccess) return e;
   }
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm,
-                                                       biwfa_persistent_kernel<G, GROUPS, RS, MINB, TWO, MS, TILES>,
+                                                       biwfa_persistent_kernel<G, GROUPS, RS, MINB, TWO, MS>,
                                                        G * GROUPS * 32, dyn);
 }
 
-// The shared-memory rings of the 4- and 8-warp shapes hold a few rows, so those run without tiles.
-template <bool TWO, int MS, bool TILES>
+template <bool TWO, int MS>
 cudaError_t occupancy_shape(int gw, int ring_in_smem, size_t dyn, int* blocks_per_sm) {
-  if (gw <= 1)
-    return occupancy_of<1, kG1Groups, false, g1_min_blocks<TWO, TILES>(), TWO, MS, TILES>(kSeqSmemBytesG1, blocks_per_sm);
+  if (gw <= 1) return occupancy_of<1, kG1Groups, false, g1_min_blocks<TWO>(), TWO, MS>(kSeqSmemBytesG1, blocks_per_sm);
   if (gw == 8) {
-    if (ring_in_smem) return occupancy_of<8, 1, true, 1, TWO, MS, false>(dyn, blocks_per_sm);
-    return occupancy_of<8, 1, false, TILES ? WFG_G8_TILES_MIN_BLOCKS : WFG_G8_MIN_BLOCKS, TWO, MS, TILES>(0, blocks_per_sm);
+    if (ring_in_smem) return occupancy_of<8, 1, true, 1, TWO, MS>(dyn, blocks_per_sm);
+    return occupancy_of<8, 1, false, WFG_G8_MIN_BLOCKS, TWO, MS>(0, blocks_per_sm);
   }
-  if (ring_in_smem) return occupancy_of<4, 1, true, 1, TWO, MS, false>(dyn, blocks_per_sm);
-  return occupancy_of<4, 1, false, 3, TWO, MS, TILES>(0, blocks_per_sm);
+  if (ring_in_smem) return occupancy_of<4, 1, true, 1, TWO, MS>(dyn, blocks_per_sm);
+  return occupancy_of<4, 1, false, 3, TWO, MS>(0, blocks_per_sm);
 }
 
-template <bool TWO, int MS, bool TILES>
+template <bool TWO, int MS>
 cudaError_t launch_kernel(const KernelParams& p, int grid, cudaStream_t stream) {
   const int gw = p.group_warps > 0 ? p.group_warps : 1;
-  if (gw == 1)
-    return launch_shape<1, kG1Groups, false, g1_min_blocks<TWO, TILES>(), TWO, MS, TILES>(p, grid, stream);
+  if (gw == 1) return launch_shape<1, kG1Groups, false, g1_min_blocks<TWO>(), TWO, MS>(p, grid, stream);
   if (gw == 8) {
-    if (p.ring_in_smem) return launch_shape<8, 1, true, 1, TWO, MS, false>(p, grid, stream);
-    return launch_shape<8, 1, false, TILES ? WFG_G8_TILES_MIN_BLOCKS : WFG_G8_MIN_BLOCKS, TWO, MS, TILES>(p, grid, stream);
+    if (p.ring_in_smem) return launch_shape<8, 1, true, 1, TWO, MS>(p, grid, stream);
+    return launch_shape<8, 1, false, WFG_G8_MIN_BLOCKS, TWO, MS>(p, grid, stream);
   }
   if (gw == 4) {
-    if (p.ring_in_smem) return launch_shape<4, 1, true, 1, TWO, MS, false>(p, grid, stream);
-    return launch_shape<4, 1, false, 3, TWO, MS, TILES>(p, grid, stream);
+    if (p.ring_in_smem) return launch_shape<4, 1, true, 1, TWO, MS>(p, grid, stream);
+    return launch_shape<4, 1, false, 3, TWO, MS>(p, grid, stream);
   }
   return cudaErrorInvalidValue;
 }
@@ -1767,12 +1538,11 @@ cudaError_t launch_kernel(const KernelParams& p, int grid, cudaStream_t stream) 
 int biwfa_warps_per_block() { return kG1Groups; }
 
 cudaError_t biwfa_occupancy(int* blocks_per_sm) {
-  return occupancy_of<1, kG1Groups, false, g1_min_blocks<false, false>(), false, kMaxScope, false>(kSeqSmemBytesG1,
-                                                                                                    blocks_per_sm);
+  return occupancy_of<1, kG1Groups, false, g1_min_blocks<false>(), false, kMaxScope>(kSeqSmemBytesG1, blocks_per_sm);
 }
 
 // The kernel instantiation of a launch: 0 three components (scope <= 32), 1 three components
-// (scope <= 64), 2 two-piece gap-affine (scope <= 64), 3 three components with rows in tiles.
+// (scope <= 64), 2 two-piece gap-affine (scope <= 64), 3 the tile kernel.
 int biwfa_kernel_kind(int metric, int scope, int tile_g) {
   return tile_g > 0 ? 3 : metric == kMetricAffine2p ? 2 : (scope > kMaxScope ? 1 : 0);
 }
@@ -1780,24 +1550,29 @@ int biwfa_kernel_kind(int metric, int scope, int tile_g) {
 // Resident blocks per SM of a shape (dyn: its dynamic shared memory in bytes; kind: as
 // biwfa_kernel_kind).
 cudaError_t biwfa_occupancy_shape(int gw, int ring_in_smem, size_t dyn, int* blocks_per_sm, int kind) {
-  if (kind == 3) return occupancy_shape<false, kMaxScope, true>(gw, ring_in_smem, dyn, blocks_per_sm);
-  if (kind == 2) return occupancy_shape<true, kMaxScope2p, false>(gw, ring_in_smem, dyn, blocks_per_sm);
-  if (kind == 1) return occupancy_shape<false, kMaxScope2p, false>(gw, ring_in_smem, dyn, blocks_per_sm);
-  return occupancy_shape<false, kMaxScope, false>(gw, ring_in_smem, dyn, blocks_per_sm);
+  if (kind == 3)
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, biwfa_tile_kernel, kTileWarps * 32, 0);
+  if (kind == 2) return occupancy_shape<true, kMaxScope2p>(gw, ring_in_smem, dyn, blocks_per_sm);
+  if (kind == 1) return occupancy_shape<false, kMaxScope2p>(gw, ring_in_smem, dyn, blocks_per_sm);
+  return occupancy_shape<false, kMaxScope>(gw, ring_in_smem, dyn, blocks_per_sm);
 }
 
-// Groups (pairs in flight) per block of a shape.
-int biwfa_groups_per_block(int group_warps, int ring_in_smem) {
-  (void)ring_in_smem;
+// Groups (pairs in flight) per block of a shape. A block of the tile kernel holds a pair per warp,
+// or fewer pairs that its other warps help with.
+int biwfa_groups_per_block(int group_warps, int tile_g) {
+  if (tile_g > 0) return biwfa_owners(group_warps);
   return group_warps <= 1 ? kG1Groups : 1;
 }
 
 cudaError_t launch_biwfa(const KernelParams& p, int grid, cudaStream_t stream) {
   const int kind = biwfa_kernel_kind(p.metric, p.scope, p.tile_g);
-  if (kind == 3) return launch_kernel<false, kMaxScope, true>(p, grid, stream);
-  if (kind == 2) return launch_kernel<true, kMaxScope2p, false>(p, grid, stream);
-  if (kind == 1) return launch_kernel<false, kMaxScope2p, false>(p, grid, stream);
-  return launch_kernel<false, kMaxScope, false>(p, grid, stream);
+  if (kind == 3) {
+    biwfa_tile_kernel<<<grid, kTileWarps * 32, 0, stream>>>(p);
+    return cudaGetLastError();
+  }
+  if (kind == 2) return launch_kernel<true, kMaxScope2p>(p, grid, stream);
+  if (kind == 1) return launch_kernel<false, kMaxScope2p>(p, grid, stream);
+  return launch_kernel<false, kMaxScope>(p, grid, stream);
 }
 
 cudaError_t launch_pack(int n, const uint8_t* ascii, PairDesc* pairs, uint32_t* words, int num_sms,

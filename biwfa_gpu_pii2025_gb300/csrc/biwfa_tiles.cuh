@@ -19,9 +19,9 @@
 // What bounds it: instruction issue and fetch, then the latency of a row's two dependent rounds
 // (shuffles, then the sequence windows). One score at a time cost about 264 lane instructions per
 // diagonal and row, 40 % of them paid per step; a tile costs about 60. End to end on a GB300, one
-// score at a time -> tiles: 10,000 pairs of 1 kbp at 5 % 7.7 -> 3.8 ms, 20,000 uneven pairs
-// (100 bp - 10 kbp, 1-10 %) 320 -> 102 ms, 48 pairs of 10-20 kbp at 12 % (8 warps per pair)
-// 569 -> 135 ms, 200,000 pairs of 150 bp at 2 % 15.3 -> 13.4 ms.
+// score at a time -> tiles (and the kernel of biwfa_tile_kernel.cuh): 10,000 pairs of 1 kbp at 5 %
+// 7.7 -> 3.4 ms, 20,000 uneven pairs (100 bp - 10 kbp, 1-10 %) 320 -> 73 ms, 48 pairs of 10-20 kbp
+// at 12 % 569 -> 124 ms, 200,000 pairs of 150 bp at 2 % 15.3 -> 12.5 ms.
 //
 // Where the values are exact. WFA2-lib trims each row to its in-bounds cells and keeps
 // out-of-bounds I/D cells between them. Out-of-bounds cells arise only from a cell whose offset
@@ -198,73 +198,18 @@ __device__ __forceinline__ void tile_pass(const TileArgs& a, const SeqView& sv, 
 
 // The tiling of one block for L lanes: tiles, first diagonal, end of the last tile. One tile of
 // 4 L diagonals if they hold all of the rows' cells (the cells beside it are null), else tiles with
-// halos.
-struct TilePlan { int tiles, base, end; };
+// halos. narrow: two diagonals per lane hold the rows.
+struct TilePlan { int tiles, base, end; bool narrow; };
 __device__ __forceinline__ TilePlan tile_plan(int cb, int t0, int L) {
   TilePlan p;
   const int lo = row_lo(cb, t0 + 4) & ~3, width = row_hi(cb, t0 + 4) - lo + 1;
-  p.tiles = 1; p.base = lo;
+  p.tiles = 1; p.base = lo; p.narrow = width <= 2 * L;
   if (width > 4 * L) { p.tiles = (width + 119) / 120; p.base = lo - kTileHalo; }
   p.end = p.base + (p.tiles - 1) * 120 + 4 * L;
   return p;
 }
-
-// One warp's tiles (first, first + step, ...) of block t0 of direction d, or (pair) the tile of
-// both d and e, narrow enough for half a warp each. The warp's largest antidiagonal of each row and
-// first touched row (4: none) go to part[0..4]; with pair, e's to part_e.
-__device__ __noinline__ void tile_run(const Dir& d, const Dir& e, bool pair, int t0, int first, int step, int32_t* leaf,
-                                      int leaf_lo, int leaf_n, int lane, int* part, int* part_e) {
-  const bool upper = lane >= 16;
-  const Dir& my = pair && upper ? e : d;
-  const int L = pair ? 16 : 32, tl = lane & (L - 1);
-  const TilePlan p = tile_plan(my.cb, t0, L);
-  const SeqView sv = my.sv;
-  TileArgs a;
-  const int b = (t0 >> 2) % 3;
-  a.pitch = my.cfg.pitch;
-  a.old_rows = my.cfg.rdata + (b == 0 ? 2 : b - 1) * 12 * a.pitch;
-  a.new_rows = my.cfg.rdata + b * 12 * a.pitch;
-  a.mask = (uint32_t)my.cfg.W - 1u;
-  a.old_lo = my.ts.lo; a.old_hi = my.ts.hi;
-  a.first = tl == 0; a.last = tl == L - 1;
-  a.lane = lane;
-  a.leaf = leaf; a.leaf_lo = leaf_lo; a.leaf_n = leaf_n;
-  int ak = INT_MIN, touch = 4;
-  // two diagonals per lane while they hold the rows (in both directions of a pair)
-  const bool narrow = row_hi(my.cb, t0 + 4) - p.base < 2 * L && p.tiles == 1;
-  if (__all_sync(kFull, narrow)) {
-    a.k = p.base + tl * 2;
-    a.owner = true;
-    if (first == 0) tile_pass<2>(a, sv, 0, true, ak, touch);
-  } else {
-    a.k = p.base + tl * 4;
-    a.owner = p.tiles == 1 || !(a.first || a.last);
-    #pragma unroll 1
-    for (int i = first; i < p.tiles; i += step)
-      tile_pass<4>(a, sv, i * 120, a.owner || (i == 0 && a.first) || (i == p.tiles - 1 && a.last), ak, touch);
-  }
-  const int t_lo = __reduce_min_sync(kFull, upper ? 4 : touch), t_up = __reduce_min_sync(kFull, upper ? touch : 4);
-  const int other = __shfl_xor_sync(kFull, ak, 16);
-  if (pair) {
-    int* out = upper ? part_e : part;
-    if ((lane & 15) < 4) out[lane & 15] = ak;
-    if ((lane & 15) == 4) out[4] = upper ? t_up : t_lo;
-  } else {
-    if (lane < 4) part[lane] = max(ak, other);
-    if (lane == 4) part[4] = min(t_lo, t_up);
-  }
-}
-
-// The diagonals that block t0 writes (tile_run's choice of tiles).
-__device__ __forceinline__ void tile_span(int cb, int t0, bool pair, bool narrow, int& lo, int& hi) {
-  const TilePlan p = tile_plan(cb, t0, pair ? 16 : 32);
-  lo = p.base;
-  hi = narrow ? p.base + (pair ? 32 : 64) : p.end;
-}
-__device__ __forceinline__ bool tile_narrow(int cb, int t0, int L) {
-  return row_hi(cb, t0 + 4) - (row_lo(cb, t0 + 4) & ~3) < 2 * L;
-}
-// Whether the ring holds block t0's diagonals.
+// Whether half a warp holds block t0's rows, and whether the ring holds them.
+__device__ __forceinline__ bool tile_half(int cb, int t0) { return row_hi(cb, t0 + 4) - (row_lo(cb, t0 + 4) & ~3) < 64; }
 __device__ __forceinline__ bool tile_fits(const Dir& d, int t0) {
   const TilePlan p = tile_plan(d.cb, t0, 32);
   return p.end - p.base <= d.cfg.W;
@@ -278,9 +223,8 @@ __device__ __noinline__ int first_match(const uint32_t* pw, const uint32_t* tw, 
 }
 
 // Starts a direction over window sv in component cb: row 0 with its extension. Returns its offset,
-// or -1 when it touches (then nothing is started). The caller syncs before and after it.
-template <int G>
-__device__ __noinline__ int tile_start(Dir& d, const SeqView& sv, int cb, int ce, const Grp<G> g) {
+// or -1 when it touches (then nothing is started).
+__device__ __noinline__ int tile_start(Dir& d, const SeqView& sv, int cb, int ce, int lane) {
   const int n = min(sv.plen, sv.tlen);
   const int off0 = cb == CM ? first_match(sv.pw, sv.tw, sv.p0, sv.t0, n, sv.bshift) : 0;
   if (off0 >= n) return -1;
@@ -290,54 +234,14 @@ __device__ __noinline__ int tile_start(Dir& d, const SeqView& sv, int cb, int ce
   d.ts.lo = 0; d.ts.hi = 4;
   d.ts.akr[row_buffer(0)] = cb == CM ? 2 * off0 : 0;
   // rows -3 .. 0 on diagonals 0-3: M in buffers 8-11, I and D of row 0
-  if (g.tid < 6) {
-    const int row = g.tid < 4 ? (8 + g.tid) * 3 : 11 * 3 + g.tid - 3;
-    const int mine = g.tid < 3 ? -1 : g.tid - 3;  // the component of row 0
+  if (lane < 6) {
+    const int row = lane < 4 ? (8 + lane) * 3 : 11 * 3 + lane - 3;
+    const int mine = lane < 3 ? -1 : lane - 3;  // the component of row 0
     *reinterpret_cast<int4*>(d.cfg.rdata + row * d.cfg.pitch) =
         make_int4(mine == comp_index(cb) ? off0 : kTNull, kTNull, kTNull, kTNull);
   }
-  return off0;
-}
-
-// Combines the warps' parts of a block (after a group barrier): antidiagonals into the rows'
-// entries; returns the first touched row of the four, 4 if none.
-template <int G>
-__device__ __forceinline__ int tile_combine(Dir& d, int t0, const int* part, const Grp<G>& g) {
-  int touch = part[4];
-  #pragma unroll
-  for (int w = 1; w < G; ++w) touch = min(touch, part[w * 5 + 4]);
-  if (g.lane() < 4) {
-    int v = part[g.lane()];
-    #pragma unroll
-    for (int w = 1; w < G; ++w) v = max(v, part[w * 5 + g.lane()]);
-    d.ts.akr[((t0 >> 2) % 3) * 4 + g.lane()] = max(v, 0);
-  }
   __syncwarp();
-  return touch;
-}
-
-// The state after block t0 (touch as tile_combine gives it). Callers pass a group barrier between
-// the last read of d.ts and this.
-__device__ __forceinline__ void tile_done(Dir& d, int t0, int touch, bool pair, bool narrow) {
-  int lo, hi;
-  tile_span(d.cb, t0, pair, narrow, lo, hi);
-  d.ts.lo = lo; d.ts.hi = hi;
-  d.ts.t = t0 + 4;
-  d.ts.touched = touch < 4 ? 1 : 0;
-  d.ts.valid = touch < 4 ? t0 + 1 + touch : t0 + 4;
-}
-
-// The next block of one direction; false when the ring is full.
-template <int G>
-__device__ __noinline__ bool tile_next(Dir& d, const Grp<G> g, int* part) {
-  const int t0 = d.ts.t;
-  if (!tile_fits(d, t0)) return false;
-  int* mine = part + ((t0 >> 2) & 1) * (G * 5);
-  tile_run(d, d, false, t0, g.warp(), G, nullptr, 0, 0, g.lane(), mine + g.warp() * 5, nullptr);
-  g.sync();
-  const int touch = tile_combine<G>(d, t0, mine, g);
-  tile_done(d, t0, touch, false, tile_narrow(d.cb, t0, 32));
-  return true;
+  return off0;
 }
 
 // Descriptors of the scores from .. s from their rows (a score without a row is absent).
@@ -353,27 +257,25 @@ __device__ __noinline__ void tile_describe(Dir& d, int s, int from, const Pen& p
       c.rdesc[slot * 3 + ci] = row && row_exists(d.cb, t, ci) ? make_int2(lo, hi) : make_int2(kAbsent, INT_MIN);
     c.rphys[slot] = row_buffer(t);
   }
+  __syncwarp();
 }
 
-// Step of a direction to score s with its descriptors: from the rows computed ahead, from a new
-// block, or — once the rows have touched or the ring is full — by dir_step. Returns as dir_step.
-template <int G>
-__device__ __noinline__ int tile_advance(Dir& d, const Pen p, int s, const Grp<G> g, int* part, int* max_ak_out) {
+// Step of a direction to score s with its descriptors: from the rows computed ahead or, when these
+// end, by dir_step. Returns as dir_step.
+__device__ __noinline__ int tile_advance(Dir& d, const Pen& p, int s, const Grp<1> g, int* max_ak_out) {
   *max_ak_out = 0;
   if (d.ts.on) {
     const bool row = holds_row(s, p);
     const int t = row_of(s, p);
-    if (!row || t <= d.ts.valid || (!d.ts.touched && tile_next<G>(d, g, part))) {
-      if (G > 1) g.sync();
+    if (!row || t <= d.ts.valid) {
       tile_describe(d, s, s, p);
-      g.sync();
       if (!row) return 0;
       if (d.ts.touched && t == d.ts.valid) {
         const int ak = d.sv.tlen - d.sv.plen;
-        const WfRef w = ref_raw<0>(d.cfg, s, comp_index(d.ce));
-        if (w.lo <= ak && ak <= w.hi && w.at(ak) >= d.sv.tlen) {
-          if (G > 1) g.sync();
+        const WfRef m = ref_raw<0>(d.cfg, s, comp_index(d.ce));
+        if (m.lo <= ak && ak <= m.hi && m.at(ak) >= d.sv.tlen) {
           d.status = ST_END_REACHED; d.status_score = s; d.end_k = ak;
+          __syncwarp();
           return 1;
         }
       }
@@ -383,11 +285,63 @@ __device__ __noinline__ int tile_advance(Dir& d, const Pen p, int s, const Grp<G
     // The one-step functions take over at this row.
     int nn = 0;
     for (int q = s - 1; q > 0 && !(holds_row(q, p) && row_exists(d.cb, row_of(q, p), 0)); --q) ++nn;
-    if (G > 1) g.sync();
+    __syncwarp();
     d.ts.on = 0;
     d.num_null = nn;
     d.next_phys = row_buffer(t);
-    if (G > 1) g.sync();
+    __syncwarp();
   }
-  return dir_step<G, 0, false>(d, p, s, g, max_ak_out);
+  return dir_step<1, 0, false>(d, p, s, g, max_ak_out);
+}
+
+// wavefront_bialign_overlap over untouched rows: row s0 of d0 against the rows of scores s1,
+// s1 - 1, ... of d1. Cells meet where their antidiagonals add up to plen + tlen or more, so the
+// lanes first test the rows' largest ones, a row pair each, and only pairs that pass are scanned.
+// An untouched row's I and D offsets are at most M's on the same diagonal, so a scan reads M and
+// looks at D and I only where M meets. D comes first, then I, then M, the lowest diagonal of each.
+__device__ __noinline__ void tile_overlap(const Dir& d0, const Dir& d1, int s0, int s1, bool fwd, BP& bp, const Pen& p,
+                                          int lane) {
+  const int t0 = row_of(s0, p), cb0 = d0.cb, cb1 = d1.cb;
+  if (!row_exists(cb0, t0, 0)) return;
+  const int plen = d0.sv.plen, tlen = d0.sv.tlen, A = tlen - plen;
+  const int mine = s1 - lane;
+  unsigned todo = __ballot_sync(kFull, lane < p.scope && mine >= 0 && holds_row(mine, p) &&
+                                           d0.ts.akr[row_buffer(t0)] + d1.ts.akr[row_buffer(row_of(max(mine, 0), p))] >=
+                                               plen + tlen);
+  const uint32_t mask = (uint32_t)d0.cfg.W - 1u;
+  const int pitch = d0.cfg.pitch;
+  const int32_t* r0 = d0.cfg.rdata + row_buffer(t0) * 3 * pitch;
+  while (todo) {
+    const int s = s1 - (__ffs((int)todo) - 1);
+    todo &= todo - 1;
+    if (s0 + s - p.go >= bp.score) continue;
+    const int t1 = row_of(s, p);
+    const int32_t* r1 = d1.cfg.rdata + row_buffer(t1) * 3 * pitch;
+    const int end = min(row_hi(cb0, t0), A - row_lo(cb1, t1));
+    int first[3] = {INT_MAX, INT_MAX, INT_MAX};  // lowest diagonal where M, I, D meet
+    #pragma unroll 1
+    for (int kb = max(row_lo(cb0, t0), A - row_hi(cb1, t1)); kb <= end; kb += 32) {
+      const int k = kb + lane;
+      const uint32_t i0 = (uint32_t)k & mask, i1 = (uint32_t)(A - k) & mask;
+      const bool hit = k <= end && r0[i0] + r1[i1] >= tlen;
+      if (!__any_sync(kFull, hit)) continue;
+      if (hit) {
+        first[0] = min(first[0], k);
+        if (r0[pitch + i0] + r1[pitch + i1] >= tlen) first[1] = min(first[1], k);
+        if (r0[2 * pitch + i0] + r1[2 * pitch + i1] >= tlen) first[2] = min(first[2], k);
+      }
+    }
+    #pragma unroll
+    for (int i = 0; i < 3; ++i) first[i] = __reduce_min_sync(kFull, first[i]);
+    const int ci = first[2] != INT_MAX ? 2 : first[1] != INT_MAX ? 1 : 0;
+    const int k = ci == 2 ? first[2] : ci == 1 ? first[1] : first[0];
+    const int cand = ci ? s0 + s - p.o : s0 + s;
+    if (k == INT_MAX || cand >= bp.score) continue;
+    const int o0 = r0[ci * pitch + ((uint32_t)k & mask)], o1 = r1[ci * pitch + ((uint32_t)(A - k) & mask)];
+    bp.score = cand;
+    bp.comp = ci == 2 ? CD : ci == 1 ? CI : CM;
+    bp.sf = fwd ? s0 : s; bp.sr = fwd ? s : s0;
+    bp.kf = fwd ? k : A - k; bp.kr = fwd ? A - k : k;
+    bp.of = fwd ? o0 : o1; bp.orv = fwd ? o1 : o0;
+  }
 }

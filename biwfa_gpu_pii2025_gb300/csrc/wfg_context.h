@@ -70,7 +70,7 @@ cudaError_t biwfa_occupancy_shape(int group_warps, int ring_in_smem, size_t dyn_
                                   int kind);
 int biwfa_kernel_kind(int metric, int scope, int tile_g);
 int biwfa_warps_per_block();
-int biwfa_groups_per_block(int group_warps, int ring_in_smem);
+int biwfa_groups_per_block(int group_warps, int tile_g);
 cudaError_t launch_pack(int n, const uint8_t* ascii, PairDesc* pairs, uint32_t* words, int num_sms,
                         cudaStream_t stream);
 int mlp_param_count();

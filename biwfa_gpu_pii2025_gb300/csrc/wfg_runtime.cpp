@@ -336,7 +336,7 @@ int64_t max_groups(const wfg_context* c, const IntPen& p, const Launch& l) {
     (void)cudaGetLastError();
     bps = 1;
   }
-  return (int64_t)bps * c->num_sms * biwfa_groups_per_block(l.gw, l.smem);
+  return (int64_t)bps * c->num_sms * biwfa_groups_per_block(l.gw, l.smem ? 0 : p.tile_g);
 }
 
 // Kernel parameters of one launch of pass ps (0: first pass; the retry passes read the
@@ -385,7 +385,7 @@ int64_t plan_retry_passes(const wfg_context* c, const IntPen& p, int64_t arena_b
     Launch& l = retry[ps];
     l.gw = c->tune.retry_warps;  // pairs that overflowed the first pass are wide
     size_launch(c, p, ps, 0, l);
-    const int gpb = biwfa_groups_per_block(l.gw, l.smem);
+    const int gpb = biwfa_groups_per_block(l.gw, l.smem ? 0 : p.tile_g);
     int64_t gmax = std::min<int64_t>(max_groups(c, p, l), std::max<int64_t>(gpb, (int64_t)c->n));
     if (l.gw == 1) gmax = std::min<int64_t>(gmax, ps == 1 ? (int64_t)c->num_sms * 4 : (int64_t)c->num_sms * 2);
     const int64_t fit = arena_budget / std::max<int64_t>(l.L.total, 1);
@@ -401,10 +401,11 @@ void plan_first_pass(const wfg_context* c, const IntPen& p, int hint, int64_t ar
   if (l.gw < 1) l.gw = 1;
   if (l.gw != 1 && l.gw != 4 && l.gw != 8) l.gw = 8;
   size_launch(c, p, 0, hint, l);
-  const int64_t gmax = std::min<int64_t>(max_groups(c, p, l), std::max<int64_t>(1, l.count));
+  // Every pair of a small batch gets a block (its other warps help with the pair's tiles).
+  const int gpb = biwfa_groups_per_block(l.gw, l.smem ? 0 : p.tile_g);
+  const int64_t gmax = std::min<int64_t>(max_groups(c, p, l), std::max<int64_t>(1, l.count) * gpb);
   const int64_t fit = arena_budget / std::max<int64_t>(l.L.total, 1);
   l.groups = std::max<int64_t>(1, std::min(gmax, fit));
-  const int gpb = biwfa_groups_per_block(l.gw, l.smem);
   l.groups = std::max<int64_t>(gpb, (l.groups / gpb) * gpb);
 }
 
@@ -453,7 +454,7 @@ int validate_config(wfg_context* c, const wfg_config_t* cfg, IntPen* p) {
   // Rows in tiles: gap-affine penalties with x = 2e, o + e = 4e (the defaults 4/6/2 among them)
   // within the usual kernels' score scope, the ratio that the tiles' row recurrence is written for;
   // other ratios and distances take one score at a time. A step limit that a score can reach counts
-  // single scores. 10,000 pairs of 1 kbp: 7.7 ms one score at a time, 3.8 ms in tiles.
+  // single scores. 10,000 pairs of 1 kbp: 7.7 ms one score at a time, 3.4 ms in tiles.
   if (cfg->metric == WFG_METRIC_GAP_AFFINE && p->x == 2 * p->e && p->o == 3 * p->e && p->scope <= WFG_MAX_SCOPE &&
       (cfg->max_alignment_steps <= 0 || cfg->max_alignment_steps >= (1 << 28)))
     p->tile_g = p->e;
@@ -529,7 +530,7 @@ int wfg_run(wfg_context_t* c, const wfg_config_t* cfg, wfg_sched_t sched) {
     if (n_wide > 0) {
       Launch l; l.gw = c->tune.wide_warps; l.order_off = 0; l.count = n_wide;
       const int w_need = (int)(m * max_wide / p.emin) + 64;
-      l.smem = (c->tune.wide_smem && next_pow2((uint64_t)w_need) <= (uint32_t)kSmemRingW) ? 1 : 0;
+      l.smem = (p.tile_g == 0 && c->tune.wide_smem && next_pow2((uint64_t)w_need) <= (uint32_t)kSmemRingW) ? 1 : 0;
       l.ring_w = w_need;
       first.push_back(l);
     }
@@ -623,7 +624,7 @@ int wfg_run(wfg_context_t* c, const wfg_config_t* cfg, wfg_sched_t sched) {
       if (l.count <= 0) continue;
       if (l.batched) {
         // one launch per resident set of pairs, each waiting for its slowest pair
-        const int gpb = biwfa_groups_per_block(l.gw, l.smem);
+        const int gpb = biwfa_groups_per_block(l.gw, l.smem ? 0 : p.tile_g);
         for (int64_t b0 = 0; b0 < l.count; b0 += l.groups, ++batch_index) {
           KernelParams kp = params(l, 0);
           kp.num_pairs = (int)std::min<int64_t>(l.groups, l.count - b0);
@@ -642,7 +643,7 @@ int wfg_run(wfg_context_t* c, const wfg_config_t* cfg, wfg_sched_t sched) {
       kp.order = c->d_order.ptr + l.order_off;
       kp.queue_head = c->d_counters.ptr + (li == 0 ? 0 : 2);
       const cudaStream_t st = (fork && li > 0) ? c->aux_stream : c->stream;
-      if ((e = launch_biwfa(kp, (int)(l.groups / biwfa_groups_per_block(l.gw, l.smem)), st)) != cudaSuccess) return e;
+      if ((e = launch_biwfa(kp, (int)(l.groups / biwfa_groups_per_block(l.gw, l.smem ? 0 : p.tile_g)), st)) != cudaSuccess) return e;
       ++launches;
     }
     if (fork) {
@@ -658,7 +659,7 @@ int wfg_run(wfg_context_t* c, const wfg_config_t* cfg, wfg_sched_t sched) {
       kp.num_pairs_ptr = c->d_counters.ptr + (ps - 1) * kCountersPerPass + 1;
       kp.order = c->d_retry.ptr + (size_t)(ps - 1) * n;
       kp.queue_head = c->d_counters.ptr + ps * kCountersPerPass + 0;
-      if ((e = launch_biwfa(kp, (int)(l.groups / biwfa_groups_per_block(l.gw, l.smem)), c->stream)) != cudaSuccess)
+      if ((e = launch_biwfa(kp, (int)(l.groups / biwfa_groups_per_block(l.gw, l.smem ? 0 : p.tile_g)), c->stream)) != cudaSuccess)
         return e;
       ++launches;
     }
@@ -950,7 +951,7 @@ int align_host_pipelined(wfg_context* c, const wfg_config_t* cfg, wfg_sched_t sc
     kp.num_pairs_ptr = nullptr;
     kp.order = c->d_order.ptr + a;
     kp.queue_head = c->d_batch_heads.ptr + k;
-    WFG_CHECK(c, launch_biwfa(kp, (int)(l.groups / biwfa_groups_per_block(l.gw, l.smem)), ks));
+    WFG_CHECK(c, launch_biwfa(kp, (int)(l.groups / biwfa_groups_per_block(l.gw, l.smem ? 0 : p.tile_g)), ks));
     ++launches;
     if (k == 0) { first_warps = l.groups * l.gw; first_ring = l.ring_w; first_arena = l.L.total; }
   }
@@ -964,7 +965,7 @@ int align_host_pipelined(wfg_context* c, const wfg_config_t* cfg, wfg_sched_t sc
     kp.num_pairs_ptr = c->d_counters.ptr + (ps - 1) * kCountersPerPass + 1;
     kp.order = c->d_retry.ptr + (size_t)(ps - 1) * n;
     kp.queue_head = c->d_counters.ptr + ps * kCountersPerPass + 0;
-    WFG_CHECK(c, launch_biwfa(kp, (int)(l.groups / biwfa_groups_per_block(l.gw, l.smem)), ms));
+    WFG_CHECK(c, launch_biwfa(kp, (int)(l.groups / biwfa_groups_per_block(l.gw, l.smem ? 0 : p.tile_g)), ms));
     ++launches;
   }
   WFG_CHECK(c, cudaEventRecord(c->ev[3], ms));
