@@ -297,6 +297,7 @@ struct TileState {
   int valid;         // last row whose values hold (the first touched row, or t)
   int touched;       // row `valid` touched an end: dir_step continues after it
   int lo, hi;        // diagonals [lo, hi) that the last block wrote, in each of its rows
+  int base, end, tiles, narrow;  // tiling of the next block (tile_plan)
   int akr[kTileBufs];  // largest antidiagonal of each stored row's M
 };
 struct Dir {
@@ -809,6 +810,43 @@ __device__ __noinline__ int dir_step(Dir& d, const Pen p, int s, const Grp<G> g,
 
 struct BP { int score, sf, sr, kf, kr, of, orv, comp; };
 
+// Forward run list of the pair (the CIGAR being assembled), with the open run in registers.
+struct RunOut {
+  uint32_t* buf;
+  int n, cap;
+  int cur_op, cur_len;
+  bool overflow;
+  __device__ __forceinline__ void flush() {
+    if (cur_len > 0) {
+      if (n < cap) buf[n] = ((uint32_t)cur_len << 4) | (uint32_t)cur_op; else overflow = true;
+      ++n;
+    }
+    cur_len = 0;
+  }
+  __device__ __forceinline__ void emit(int op, int len) {
+    if (len <= 0) return;
+    if (op == cur_op && cur_len > 0) { cur_len += len; return; }
+    flush();
+    cur_op = op; cur_len = len;
+  }
+  // Appends n runs that lie end to begin and of which neighbours differ, so only the first can join
+  // the open run; the group's `threads` threads copy the rest, and the last stays open.
+  __device__ __forceinline__ void append(const uint32_t* rev, int count, int tid, int threads) {
+    if (count <= 0) return;
+    const uint32_t r = rev[count - 1];
+    emit((int)(r & 15u), (int)(r >> 4));
+    if (count == 1) return;
+    flush();
+    #pragma unroll 1
+    for (int i = tid; i < count - 2; i += threads)
+      if (n + i < cap) buf[n + i] = rev[count - 2 - i];
+    n += count - 2;
+    if (n > cap) overflow = true;
+    const uint32_t q = rev[0];
+    cur_op = (int)(q & 15u); cur_len = (int)(q >> 4);
+  }
+};
+
 #include "biwfa_tiles.cuh"
 
 
@@ -1015,27 +1053,6 @@ __device__ __noinline__ int find_breakpoint(Dir& F, Dir& R, const PairSeqs& q, i
                                          bp, g);
 }
 
-// Forward run list of the pair (the CIGAR being assembled), with the open run in registers.
-struct RunOut {
-  uint32_t* buf;
-  int n, cap;
-  int cur_op, cur_len;
-  bool overflow;
-  __device__ __forceinline__ void flush() {
-    if (cur_len > 0) {
-      if (n < cap) buf[n] = ((uint32_t)cur_len << 4) | (uint32_t)cur_op; else overflow = true;
-      ++n;
-    }
-    cur_len = 0;
-  }
-  __device__ __forceinline__ void emit(int op, int len) {
-    if (len <= 0) return;
-    if (op == cur_op && cur_len > 0) { cur_len += len; return; }
-    flush();
-    cur_op = op; cur_len = len;
-  }
-};
-
 // wavefront_backtrace_affine (wavefront/wavefront_backtrace.c:320-529; TWO: the two-piece
 // distance's I2/D2 sources) or wavefront_backtrace_linear (:223-319) over the leaf store, from
 // (end_k, tlen) at score s in component ce; appends the leaf's ops to out.
@@ -1121,42 +1138,25 @@ __device__ __noinline__ int leaf_backtrace(const Dir& B, const Pen p, int s, int
   }
   if (rlen > 0) { if (nrev < lruns_cap) lruns[nrev] = ((uint32_t)rlen << 4) | (uint32_t)rop; else rover = true; ++nrev; }
   if (rover) return WFG_ST_SCRATCH_OVERFLOW;
-  // Runs lie end to begin and neighbours differ, so only the first can join the open run; the
-  // threads copy the rest, and the last stays open.
-  if (nrev > 0) {
-    const uint32_t r = lruns[nrev - 1];
-    out.emit((int)(r & 15u), (int)(r >> 4));
-    if (nrev > 1) {
-      out.flush();
-      for (int i = g.tid; i < nrev - 2; i += 32 * G)
-        if (out.n + i < out.cap) out.buf[out.n + i] = lruns[nrev - 2 - i];
-      out.n += nrev - 2;
-      if (out.n > out.cap) out.overflow = true;
-      const uint32_t q = lruns[0];
-      out.cur_op = (int)(q & 15u); out.cur_len = (int)(q >> 4);
-    }
-  }
+  out.append(lruns, nrev, g.tid, 32 * G);
   return ST_OK;
 }
 
-// The leaf's steps from score s (wavefront_bialign_base -> unialign) and its backtrace; appends the
-// leaf's ops to out.
+// The leaf's steps from score *s_io to its end (wavefront_bialign_base -> unialign).
 template <int G, bool TWO>
-__device__ __noinline__ int leaf_finish(Dir& B, bool done, int s, int guard, const Pen p, int max_steps, RunOut& out,
-                                        uint32_t* lruns, int lruns_cap, const Grp<G> g, int* max_leaf_score) {
-  int ak = 0;
-  while (!done) {
+__device__ __noinline__ int leaf_steps(Dir& B, int* s_io, int guard, const Pen p, int max_steps, const Grp<G> g) {
+  int ak = 0, s = *s_io;
+  for (;;) {
     ++s;
     // wavefront_unialign_reached_limits checks the step count after compute, before extend
     if (s >= max_steps) return WFG_ST_UNATTAINABLE;
     if (s > guard) return WFG_ST_UNATTAINABLE;
     const int q = dir_step<G, 1, TWO>(B, p, s, g, &ak);
     if (q < 0) return WFG_ST_SCRATCH_OVERFLOW;
-    done = q != 0;
+    if (q) break;
   }
-  if (*max_leaf_score < s) *max_leaf_score = s;
-  if (B.status != ST_END_REACHED) return WFG_ST_UNATTAINABLE;
-  return leaf_backtrace<G, TWO>(B, p, s, B.ce, out, lruns, lruns_cap, g);
+  *s_io = s;
+  return B.status == ST_END_REACHED ? ST_OK : WFG_ST_UNATTAINABLE;
 }
 
 // Leaf: wavefront_bialign_base -> unialign -> backtrace.
@@ -1167,9 +1167,14 @@ __device__ __noinline__ int leaf_align(Dir& B, const PairSeqs& q, int pb, int pe
   g.sync();
   dir_init<TWO>(B, fwd_view(q, pb, pe, tb, te), cb, ce);
   g.sync();
-  const bool done = dir_extend<G>(B, 0, g, nullptr) != 0;
-  return leaf_finish<G, TWO>(B, done, 0, score_guard(p, pe - pb, te - tb), p, max_steps, out, lruns, lruns_cap, g,
-                             max_leaf_score);
+  int s = 0;
+  if (!dir_extend<G>(B, 0, g, nullptr)) {
+    const int st = leaf_steps<G, TWO>(B, &s, score_guard(p, pe - pb, te - tb), p, max_steps, g);
+    if (st != ST_OK) return st;
+  }
+  if (*max_leaf_score < s) *max_leaf_score = s;
+  if (B.status != ST_END_REACHED) return WFG_ST_UNATTAINABLE;
+  return leaf_backtrace<G, TWO>(B, p, s, ce, out, lruns, lruns_cap, g);
 }
 
 // cigar_score_gap_affine (alignment/cigar.c:277-303), cigar_score_gap_affine2p (:304-342: per
@@ -1551,7 +1556,12 @@ int biwfa_kernel_kind(int metric, int scope, int tile_g) {
 // biwfa_kernel_kind).
 cudaError_t biwfa_occupancy_shape(int gw, int ring_in_smem, size_t dyn, int* blocks_per_sm, int kind) {
   if (kind == 3)
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, biwfa_tile_kernel, kTileWarps * 32, 0);
+  {
+    const cudaError_t e = tile_kernel_attributes();
+    if (e != cudaSuccess) return e;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, biwfa_tile_kernel, kTileWarps * 32,
+                                                         sizeof(TileBlockSmem));
+  }
   if (kind == 2) return occupancy_shape<true, kMaxScope2p>(gw, ring_in_smem, dyn, blocks_per_sm);
   if (kind == 1) return occupancy_shape<false, kMaxScope2p>(gw, ring_in_smem, dyn, blocks_per_sm);
   return occupancy_shape<false, kMaxScope>(gw, ring_in_smem, dyn, blocks_per_sm);
@@ -1567,7 +1577,9 @@ int biwfa_groups_per_block(int group_warps, int tile_g) {
 cudaError_t launch_biwfa(const KernelParams& p, int grid, cudaStream_t stream) {
   const int kind = biwfa_kernel_kind(p.metric, p.scope, p.tile_g);
   if (kind == 3) {
-    biwfa_tile_kernel<<<grid, kTileWarps * 32, 0, stream>>>(p);
+    const cudaError_t e = tile_kernel_attributes();
+    if (e != cudaSuccess) return e;
+    biwfa_tile_kernel<<<grid, kTileWarps * 32, sizeof(TileBlockSmem), stream>>>(p);
     return cudaGetLastError();
   }
   if (kind == 2) return launch_kernel<true, kMaxScope2p>(p, grid, stream);

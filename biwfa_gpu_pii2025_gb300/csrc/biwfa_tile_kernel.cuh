@@ -76,7 +76,7 @@ struct TileCtl {
   bool last_fwd;
   BP bp;
   // leaf
-  int used, leaf_lo, leaf_n;
+  int leaf_end;  // words of the leaf store in use
 };
 
 struct TileGroup {
@@ -94,6 +94,10 @@ struct TileBlockSmem {
   KernelParams P;
   int active, idle;  // warps with a pair, warps that help
 };
+// The block's shared memory, named rather than passed: a function that gets a pointer to it reads it
+// with generic loads and 64-bit addresses, a third more code.
+extern __shared__ __align__(16) unsigned char s_tile_smem[];
+__device__ __forceinline__ TileBlockSmem& tile_smem() { return *reinterpret_cast<TileBlockSmem*>(s_tile_smem); }
 
 __device__ __forceinline__ int job_next(unsigned long long ticket) { return (int)(ticket & 0xffffffu); }
 __device__ __forceinline__ int job_tiles(unsigned long long ticket) { return (int)((ticket >> 24) & 0xffffffu); }
@@ -114,8 +118,8 @@ __device__ __forceinline__ int job_take(TileJob& job, int lane) {
 }
 
 // Sets the block pass of tile i of the job of warp `owner`.
-__device__ __forceinline__ void job_block(TileGroup* grp, int owner, int i, TileCtl& C) {
-  const TileJob& job = grp[owner].job;
+__device__ __forceinline__ void job_block(int owner, int i, TileCtl& C) {
+  const TileJob& job = tile_smem().grp[owner].job;
   C.owner = owner;
   C.mode = kOne;
   C.second = i >= job.d_tiles;
@@ -126,8 +130,8 @@ __device__ __forceinline__ void job_block(TileGroup* grp, int owner, int i, Tile
 }
 
 // Adds the results of a tile (C.part) to its job.
-__device__ __forceinline__ void job_add(TileGroup* grp, const TileCtl& C, int lane) {
-  TileJob& job = grp[C.owner].job;
+__device__ __forceinline__ void job_add(const TileCtl& C, int lane) {
+  TileJob& job = tile_smem().grp[C.owner].job;
   int* out = job.part + (C.second ? 5 : 0);
   if (lane < 4) atomicMax(&out[lane], C.part[lane]);
   if (lane == 4) atomicMin(&out[4], C.part[4]);
@@ -136,52 +140,66 @@ __device__ __forceinline__ void job_add(TileGroup* grp, const TileCtl& C, int la
   if (lane == 0) atomicAdd(&job.done, 1);
 }
 
-// The state of direction d after block t0: touch is its first touched row of the four, 4 if none;
-// narrow: two diagonals for each of the `lanes` lanes.
-__device__ __forceinline__ void tile_done(Dir& d, int t0, int touch, int lanes, bool narrow) {
-  const TilePlan p = tile_plan(d.cb, t0, lanes);
-  d.ts.lo = p.base;
-  d.ts.hi = narrow ? p.base + 2 * lanes : p.end;
+// The state of direction d after block t0: touch is its first touched row of the four, 4 if none.
+__device__ __forceinline__ void tile_done(Dir& d, int t0, int touch) {
+  d.ts.lo = d.ts.base;
+  d.ts.hi = d.ts.end;
   d.ts.t = t0 + 4;
   d.ts.touched = touch < 4 ? 1 : 0;
   d.ts.valid = touch < 4 ? t0 + 1 + touch : t0 + 4;
 }
 
-// Sets up block t0 of dir[d] (both: and of dir[1]) as the warp's next pass, alone or as a job that
-// the block's idle warps share. state: what follows it.
-__device__ __forceinline__ void tile_request(TileBlockSmem& B, TileGroup& S, int d, bool both, int t0, int state, int gib,
-                                             int lane) {
+// Opens block t0 of dir[d] (both: and of dir[1]), more than one tile, to the thread block's idle warps
+// and takes a tile of it as this warp's next pass. state: what follows the job.
+__device__ __noinline__ void job_open(int d, bool both, int t0, int state, int gib, int lane) {
+  TileGroup& S = tile_smem().grp[gib];
   TileCtl& C = S.ctl;
-  C.owner = gib; C.d = d; C.t0 = t0; C.tile = 0; C.step = 1;
-  C.state = state;
-  if (both && tile_half(S.dir[0].cb, t0) && tile_half(S.dir[1].cb, t0)) { C.mode = kHalves; return; }
-  C.mode = both ? kBoth : kOne;
-  if (*(volatile int*)&B.idle > 0) {
-    const int nd = tile_plan(S.dir[d].cb, t0, 32).tiles, tiles = nd + (both ? tile_plan(S.dir[1].cb, t0, 32).tiles : 0);
-    if (tiles > 1) {
-      TileJob& job = S.job;
-      if (lane < 10) job.part[lane] = lane == 4 || lane == 9 ? 4 : INT_MIN;
-      if (lane == 0) { job.d = d; job.d_tiles = nd; job.t0 = t0; job.done = 0; }
-      __syncwarp();
-      if (lane == 0) {
-        __threadfence_block();
-        const unsigned long long gen = (*(volatile unsigned long long*)&job.ticket >> 48) + 1;
-        atomicExch(&job.ticket, (gen << 48) | ((unsigned long long)tiles << 24));
-      }
-      __syncwarp();
-      C.after = state;
-      C.state = kOwnJob;
-      const int i = job_take(job, lane);
-      if (i >= 0) job_block(B.grp, gib, i, C);
-      else C.step = 0;  // the helpers took every tile: nothing to compute here
-    }
+  TileJob& job = S.job;
+  const int nd = S.dir[d].ts.tiles, tiles = nd + (both ? S.dir[1].ts.tiles : 0);
+  if (lane < 10) job.part[lane] = lane == 4 || lane == 9 ? 4 : INT_MIN;
+  if (lane == 0) { job.d = d; job.d_tiles = nd; job.t0 = t0; job.done = 0; }
+  __syncwarp();
+  if (lane == 0) {
+    __threadfence_block();
+    const unsigned long long gen = (*(volatile unsigned long long*)&job.ticket >> 48) + 1;
+    atomicExch(&job.ticket, (gen << 48) | ((unsigned long long)tiles << 24));
   }
   __syncwarp();
+  C.after = state;
+  C.state = kOwnJob;
+  const int i = job_take(job, lane);
+  if (i >= 0) job_block(gib, i, C);
+  else C.step = 0;  // the helpers took every tile: nothing to compute here
+  __syncwarp();
+}
+
+// Sets up block t0 of dir[d] (both: and of dir[1]) as the warp's next pass, alone or as a job that
+// the block's idle warps share. state: what follows it. False when a ring does not hold the block.
+__device__ __noinline__ bool tile_request(int d, bool both, int t0, int state, int gib, int lane) {
+  TileBlockSmem& B = tile_smem();
+  TileGroup& S = B.grp[gib];
+  TileCtl& C = S.ctl;
+  const bool halves = both && tile_half(S.dir[0].cb, t0) && tile_half(S.dir[1].cb, t0);
+  const int L = halves ? 16 : 32;
+  if (!tile_plan(S.dir[d], t0, L) || (both && !tile_plan(S.dir[1], t0, L))) return false;
+  if (halves && !(S.dir[0].ts.narrow && S.dir[1].ts.narrow)) {  // one width for both
+    S.dir[0].ts.narrow = S.dir[1].ts.narrow = 0;
+    S.dir[0].ts.end = S.dir[0].ts.base + 64;
+    S.dir[1].ts.end = S.dir[1].ts.base + 64;
+  }
+  C.owner = gib; C.d = d; C.t0 = t0; C.tile = 0; C.step = 1;
+  C.state = state;
+  C.mode = halves ? kHalves : both ? kBoth : kOne;
+  __syncwarp();
+  if (!halves && state != kLeaf && *(volatile int*)&B.idle > 0 && S.dir[d].ts.tiles + (both ? S.dir[1].ts.tiles : 0) > 1)
+    job_open(d, both, t0, state, gib, lane);
+  return true;
 }
 
 // Runs the warp's state machine to its next block pass (S.ctl says which); false when the launch has
 // no more work for this warp.
-__device__ __noinline__ bool tile_control(TileBlockSmem& B, int gib, int lane, int owners) {
+__device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
+  TileBlockSmem& B = tile_smem();
   TileGroup& S = B.grp[gib];
   TileCtl& C = S.ctl;
   const KernelParams& P = B.P;
@@ -215,8 +233,8 @@ __device__ __noinline__ bool tile_control(TileBlockSmem& B, int gib, int lane, i
         S.dir[C.d].ts.akr[((C.t0 >> 2) % 3) * 4 + lane] = max(C.part[lane], 0);
         if (both) R.ts.akr[((C.t0 >> 2) % 3) * 4 + lane] = max(C.part[5 + lane], 0);
       }
-      tile_done(S.dir[C.d], C.t0, C.part[4], 32, tile_plan(S.dir[C.d].cb, C.t0, 32).narrow);
-      if (both) tile_done(R, C.t0, C.part[9], 32, tile_plan(R.cb, C.t0, 32).narrow);
+      tile_done(S.dir[C.d], C.t0, C.part[4]);
+      if (both) tile_done(R, C.t0, C.part[9]);
       __syncwarp();
       if (spins >= kSpinLimit) { st = WFG_ST_UNATTAINABLE; state = kBpDone; }  // a helper was lost
       if (state == kSearch) {
@@ -224,11 +242,13 @@ __device__ __noinline__ bool tile_control(TileBlockSmem& B, int gib, int lane, i
         int nf = C.fmax, nr = C.rmax;
         #pragma unroll 1
         for (int j = 0; j < 4; ++j) { nf = max(nf, C.part[j]); nr = max(nr, C.part[5 + j]); }
-        if (min(C.part[4], C.part[9]) == 4 && nf + nr < C.max_antidiag && tile_fits(F, C.t0 + 4) &&
-            tile_fits(R, C.t0 + 4) && C.t0 <= C.guard) {
-          C.fmax = nf; C.rmax = nr;
-          tile_request(B, S, 0, true, C.t0 + 4, kSearch, gib, lane);
-          return true;
+        if (min(C.part[4], C.part[9]) == 4 && nf + nr < C.max_antidiag && C.t0 <= C.guard) {
+          const int t0 = C.t0;
+          if (tile_request(0, true, t0 + 4, kSearch, gib, lane)) {
+            C.fmax = nf; C.rmax = nr;
+            __syncwarp();
+            return true;
+          }
         }
         state = kSearchEvent;
       }
@@ -328,12 +348,11 @@ __device__ __noinline__ bool tile_control(TileBlockSmem& B, int gib, int lane, i
         __syncwarp();
         if (C.fmax + C.rmax >= C.max_antidiag) {
           state = kMet;
-        } else if (!tile_fits(F, 0) || !tile_fits(R, 0)) {
-          state = kSteps;
-        } else {
+        } else if (tile_request(0, true, 0, kSearch, gib, lane)) {
           C.out = out; C.bp = bp;
-          tile_request(B, S, 0, true, 0, kSearch, gib, lane);
           return true;
+        } else {
+          state = kSteps;
         }
       }
     }
@@ -379,11 +398,10 @@ __device__ __noinline__ bool tile_control(TileBlockSmem& B, int gib, int lane, i
         resumed = false;
         if (holds_row(s1 + 1, pen)) {
           const int t = row_of(s1 + 1, pen);
-          if (t > b.ts.valid && !b.ts.touched && tile_fits(b, b.ts.t)) {
-            __syncwarp();
+          if (t > b.ts.valid && !b.ts.touched && tile_request(last_fwd ? 1 : 0, false, b.ts.t, kMeet, gib, lane)) {
             C.sf = sf; C.sr = sr; C.last_fwd = last_fwd;
             C.out = out; C.bp = bp;
-            tile_request(B, S, last_fwd ? 1 : 0, false, b.ts.t, kMeet, gib, lane);
+            __syncwarp();
             return true;
           }
           if (t > b.ts.valid || (b.ts.touched && t == b.ts.valid)) { resume = last_fwd ? 1 : 2; state = kSteps; break; }
@@ -460,21 +478,14 @@ __device__ __noinline__ bool tile_control(TileBlockSmem& B, int gib, int lane, i
         state = kPop;
         continue;
       }
-      if (lane < 3)
-        L.cfg.ldesc[lane] = lane == comp_index(C.cb) ? make_int4(0, 0, 0, 0) : make_int4(kAbsent, INT_MIN, 0, 0);
       if (lane == 0) L.cfg.ldata[0] = off0;
       L.sv = sv; L.cb = C.cb; L.ce = C.ce; L.num_null = 0; L.status = ST_OK; L.end_k = sv.tlen - sv.plen;
-      C.used = 4;
-      C.leaf_lo = row_lo(C.cb, 4) & ~3;
-      C.leaf_n = (row_hi(C.cb, 4) - C.leaf_lo + 4) & ~3;
-      F.ts.t = 0;
+      C.leaf_end = leaf_at(0);
       __syncwarp();
       state = kLeafSteps;
       s = 0; done = false;
-      if (4 * pen.tg <= L.cfg.lmax && C.used + 12 * C.leaf_n <= L.lcap && tile_fits(F, 0)) {
+      if (4 * pen.tg <= L.cfg.lmax && leaf_at(1) <= L.lcap && tile_request(0, false, 0, kLeaf, gib, lane)) {
         C.out = out; C.bp = bp;
-        C.mode = kOne; C.owner = gib; C.d = 0; C.t0 = 0; C.tile = 0; C.step = 1;
-        C.state = kLeaf;
         __syncwarp();
         return true;
       }
@@ -486,19 +497,24 @@ __device__ __noinline__ bool tile_control(TileBlockSmem& B, int gib, int lane, i
       const int ak = L.end_k;
       s = last * pen.tg;
       if (touch < 4 && row_exists(C.cb, last, ci) && row_lo(C.cb, last) <= ak && ak <= row_hi(C.cb, last))
-        done = L.cfg.ldata[C.used - 12 * C.leaf_n + (touch * 3 + ci) * C.leaf_n + ak - C.leaf_lo] >= L.sv.tlen;
+        done = L.cfg.ldata[leaf_at(t0 >> 2) + (touch * 3 + ci) * leaf_n(t0 >> 2) + ak - leaf_lo(C.cb, t0 >> 2)] >= L.sv.tlen;
       state = kLeafSteps;
     }
 
     if (state == kLeafSteps) {
+      const int fast = s;
       __syncwarp();
-      L.lused = C.used;
+      L.lused = C.leaf_end;
       L.status = done ? ST_END_REACHED : ST_OK;
-      L.status_score = s;
       __syncwarp();
-      st = leaf_finish<1, false>(L, done, s, C.guard, pen, P.max_steps, out,
-                                 S.arena.lruns, P.leaf_run_cap, g, &C.max_leaf);
+      st = ST_OK;
+      if (!done) {
+        leaf_describe(L, s, s - pen.scope + 1, pen, lane);
+        st = leaf_steps<1, false>(L, &s, C.guard, pen, P.max_steps, g);
+      }
+      if (st == ST_OK) st = tile_backtrace(L, pen, s, fast, out, S.arena.lruns, P.leaf_run_cap, lane);
       __syncwarp();
+      C.max_leaf = max(C.max_leaf, s);
       if (st != ST_OK) C.status = st;
       __syncwarp();
       done = false;
@@ -507,7 +523,7 @@ __device__ __noinline__ bool tile_control(TileBlockSmem& B, int gib, int lane, i
     }
 
     if (state == kFinish) {
-      int status = C.status, score = C.score;
+      int status = C.status, score = P.score_only ? C.score : 0;
       const int pi = C.pi;
       if (!P.score_only) {
         out.flush();
@@ -515,13 +531,20 @@ __device__ __noinline__ bool tile_control(TileBlockSmem& B, int gib, int lane, i
         if (status == ST_OK) status = WFG_ST_COMPLETED;
         __syncwarp();
         if (status == WFG_ST_COMPLETED) {
-          score = out.n > 0 ? rescore_runs(out.buf, out.n, P.metric, P.match_o, P.x_o, P.o_o, P.e_o, P.o2_o, P.e2_o) : 0;
+          // cigar_score_gap_affine (alignment/cigar.c:277-303) over maximal runs, a lane's runs each
+          #pragma unroll 1
+          for (int i = lane; i < out.n; i += 32) {
+            const int op = (int)(out.buf[i] & 15u), len = (int)(out.buf[i] >> 4);
+            score -= op == WFG_OP_EQ ? P.match_o * len : op == WFG_OP_X ? P.x_o * len : P.o_o + P.e_o * len;
+          }
+          score = __reduce_add_sync(kFull, score);
           unsigned long long base = 0;
           if (lane == 0) base = atomicAdd(P.out_head, (unsigned long long)out.n);
           base = __shfl_sync(kFull, base, 0);
           if ((long long)base + out.n > P.out_cap) {
             status = WFG_ST_OUTPUT_OVERFLOW;
           } else {
+            #pragma unroll 1
             for (int i = lane; i < out.n; i += 32) P.out_runs[base + i] = out.buf[i];
             if (lane == 0) { P.run_off[pi] = (int64_t)base; P.run_len[pi] = out.n; }
           }
@@ -553,7 +576,7 @@ __device__ __noinline__ bool tile_control(TileBlockSmem& B, int gib, int lane, i
         for (int k = 1; k < kTileWarps; ++k) {
           const int w = gib + k < kTileWarps ? gib + k : gib + k - kTileWarps;
           const int i = job_take(B.grp[w].job, lane);
-          if (i >= 0) { job_block(B.grp, w, i, C); __syncwarp(); return true; }
+          if (i >= 0) { job_block(w, i, C); __syncwarp(); return true; }
         }
         __nanosleep(200);
       }
@@ -565,7 +588,8 @@ __device__ __noinline__ bool tile_control(TileBlockSmem& B, int gib, int lane, i
 }  // namespace
 
 __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks) biwfa_tile_kernel(KernelParams Pin) {
-  __shared__ TileBlockSmem B;
+  TileBlockSmem& B = tile_smem();
+  if (Pin.num_pairs_ptr != nullptr && *Pin.num_pairs_ptr == 0ull) return;  // a retry pass without pairs
   const int gib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int owners = biwfa_owners(Pin.group_warps);
   TileGroup& S = B.grp[gib];
@@ -609,7 +633,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks) biwfa_tile_kerne
 
   bool control = true;
   for (;;) {
-    if (control && !tile_control(B, gib, lane, owners)) break;
+    if (control && !tile_control(gib, lane, owners)) break;
     control = true;
     if (C.step == 0) continue;  // an own job whose tiles the helpers took
     // ---- the block pass
@@ -618,13 +642,12 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks) biwfa_tile_kerne
     const int L = halves ? 16 : 32, tl = lane & (L - 1), b = (t0 >> 2) % 3;
     const bool leaf = C.state == kLeaf;
     int part[2], touch[2];  // lanes 0-3: largest antidiagonal of each row; first touched row
-    bool narrow[2];
-    part[1] = INT_MIN; touch[1] = 4; narrow[1] = false;
+    part[1] = INT_MIN; touch[1] = 4;
     #pragma unroll 1
     for (int x = 0; x < (mode == kBoth ? 2 : 1); ++x) {
       const Dir& my = B.grp[C.owner].dir[(halves && upper) || x ? 1 : d0];
-      const TilePlan p = tile_plan(my.cb, t0, L);
       const SeqView sv = my.sv;
+      const int tiles = my.ts.tiles, narrow = my.ts.narrow;
       TileArgs a;
       a.pitch = my.cfg.pitch;
       a.old_rows = my.cfg.rdata + (b == 0 ? 2 : b - 1) * 12 * a.pitch;
@@ -633,20 +656,20 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks) biwfa_tile_kerne
       a.old_lo = my.ts.lo; a.old_hi = my.ts.hi;
       a.first = tl == 0; a.last = tl == L - 1;
       a.lane = lane;
-      a.leaf = leaf ? S.dir[2].cfg.ldata + C.used : nullptr;
-      a.leaf_lo = C.leaf_lo; a.leaf_n = leaf ? C.leaf_n : 0;
+      a.leaf = leaf ? S.dir[2].cfg.ldata + leaf_at(t0 >> 2) : nullptr;
+      a.leaf_lo = leaf_lo(my.cb, t0 >> 2); a.leaf_n = leaf ? leaf_n(t0 >> 2) : 0;
       int ak = INT_MIN, tch = 4;
-      narrow[x] = __all_sync(kFull, p.narrow);
-      if (narrow[x]) {  // two diagonals per lane (of both directions, in halves)
-        a.k = p.base + tl * 2;
-        a.owner = true;
-        tile_pass<2>(a, sv, 0, true, ak, tch);
-      } else {
-        a.k = p.base + tl * 4;
-        a.owner = p.tiles == 1 || !(a.first || a.last);
-        #pragma unroll 1
-        for (int i = C.tile; i < p.tiles; i += C.step)
-          tile_pass<4>(a, sv, i * 120, a.owner || (i == 0 && a.first) || (i == p.tiles - 1 && a.last), ak, tch);
+      const int step = C.step;
+      int i = C.tile;
+      a.k = my.ts.base + tl * 4;
+      a.owner = tiles == 1 || !(a.first || a.last);
+      #pragma unroll 1
+      for (; i < tiles - narrow; i += step)
+        tile_pass<4>(a, sv, i * 120, a.owner || (i == 0 && a.first) || (i == tiles - 1 && a.last), ak, tch);
+      if (i < tiles) {  // the last tile, two diagonals per lane
+        a.k = my.ts.base + tl * 2;
+        a.owner = tiles == 1 || (tl >= 2 && tl < L - 2);
+        tile_pass<2>(a, sv, i * 120, a.owner || tl >= L - 2 || i == 0, ak, tch);
       }
       const int other = __shfl_xor_sync(kFull, ak, 16);
       if (halves) {
@@ -664,9 +687,9 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks) biwfa_tile_kerne
     if (state == kHelp || state == kOwnJob) {  // the tile goes to its job; on to the next one
       __syncwarp();
       TileJob& job = B.grp[C.owner].job;
-      job_add(B.grp, C, lane);
+      job_add(C, lane);
       const int i = job_take(job, lane);
-      if (i >= 0) job_block(B.grp, C.owner, i, C);
+      if (i >= 0) job_block(C.owner, i, C);
       else C.step = 0;
       control = i < 0;
       __syncwarp();
@@ -678,38 +701,24 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks) biwfa_tile_kerne
       S.dir[d0].ts.akr[b * 4 + lane] = max(part[0], 0);
       if (both) S.dir[1].ts.akr[b * 4 + lane] = max(part[1], 0);
     }
-    tile_done(S.dir[d0], t0, touch[0], L, narrow[0]);
-    if (both) tile_done(S.dir[1], t0, touch[1], L, narrow[halves ? 0 : 1]);
+    tile_done(S.dir[d0], t0, touch[0]);
+    if (both) tile_done(S.dir[1], t0, touch[1]);
+    __syncwarp();
     if (state == kSearch) {
       const int nf = max(C.fmax, __reduce_max_sync(kFull, lane < 4 ? part[0] : INT_MIN));
       const int nr = max(C.rmax, __reduce_max_sync(kFull, lane < 4 ? part[1] : INT_MIN));
-      if (min(touch[0], touch[1]) == 4 && nf + nr < C.max_antidiag && t0 <= C.guard && tile_fits(S.dir[0], t0 + 4) &&
-          tile_fits(S.dir[1], t0 + 4)) {
-        __syncwarp();
+      if (min(touch[0], touch[1]) == 4 && nf + nr < C.max_antidiag && t0 <= C.guard &&
+          tile_request(0, true, t0 + 4, kSearch, gib, lane)) {
         C.fmax = nf; C.rmax = nr;
-        tile_request(B, S, 0, true, t0 + 4, kSearch, gib, lane);
         control = false;
       } else {
         C.state = kSearchEvent;
       }
     } else if (state == kLeaf) {
-      const Pen& pen = S.pen;
-      const int cb = C.cb, used = C.used, lo = C.leaf_lo, n = C.leaf_n;
-      int4* ldesc = S.dir[2].cfg.ldesc;
-      #pragma unroll 1
-      for (int i = lane; i < 4 * pen.tg * 3; i += 32) {
-        const int s = t0 * pen.tg + 1 + i / 3, ci = i % 3, t = row_of(s, pen);
-        int4 ds = make_int4(kAbsent, INT_MIN, 0, 0);
-        if (s == t * pen.tg && row_exists(cb, t, ci))
-          ds = make_int4(row_lo(cb, t), row_hi(cb, t), used + ((t - t0 - 1) * 3 + ci) * n, lo);
-        ldesc[s * 3 + ci] = ds;
-      }
-      __syncwarp();
-      const int lo2 = row_lo(cb, t0 + 8) & ~3, n2 = (row_hi(cb, t0 + 8) - lo2 + 4) & ~3, used2 = used + 12 * n;
-      C.used = used2;
-      if (touch[0] == 4 && t0 <= C.guard && (t0 + 8) * pen.tg <= S.dir[2].cfg.lmax && used2 + 12 * n2 <= S.dir[2].lcap &&
-          tile_fits(S.dir[0], t0 + 4)) {
-        C.leaf_lo = lo2; C.leaf_n = n2; C.t0 = t0 + 4;
+      const int end = leaf_at((t0 >> 2) + 1);
+      C.leaf_end = end;
+      if (touch[0] == 4 && t0 <= C.guard && (t0 + 8) * S.pen.tg <= S.dir[2].cfg.lmax &&
+          leaf_at((t0 >> 2) + 2) <= S.dir[2].lcap && tile_request(0, false, t0 + 4, kLeaf, gib, lane)) {
         control = false;
       } else {
         C.state = kLeafEvent;
@@ -719,3 +728,8 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks) biwfa_tile_kerne
   }
 }
 
+namespace {
+cudaError_t tile_kernel_attributes() {
+  return cudaFuncSetAttribute(biwfa_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileBlockSmem));
+}
+}  // namespace

@@ -93,8 +93,9 @@ struct TileArgs {
 // Rows t0+1 .. t0+4 of a tile's diagonals, a.k + off in this lane. Lanes j and 16 + j of ak: the
 // largest antidiagonal of row t0+1+j in the lower and the upper half warp; touch: the first of the
 // four rows (0-3) where this lane touched, else unchanged. The loop over the rows stays rolled (the
-// last four rows' registers rotate by moves): unrolled, the warps' instructions did not fit the
-// instruction caches, and waiting for them took 76 % of the issue slots.
+// last four rows' registers rotate by moves): instruction fetch bounds this kernel wherever its code
+// does not loop. 10,000 pairs of 1 kbp / 150,000 mixture pairs with the row loop rolled 3.29 / 169 ms,
+// unrolled by two 3.80 / 177 ms, by four 4.28 / 210 ms.
 template <int C>
 __device__ __forceinline__ void tile_pass(const TileArgs& a, const SeqView& sv, int off, bool store, int& ak, int& touch) {
   const int k0 = a.k + off;
@@ -138,18 +139,21 @@ __device__ __forceinline__ void tile_pass(const TileArgs& a, const SeqView& sv, 
       x[c] = __funnelshift_r(seq_word(sv.pw, wp), seq_word(sv.pw, wp + 1), (uint32_t)pp << sv.bshift) ^
              __funnelshift_r(seq_word(sv.tw, wt), seq_word(sv.tw, wt + 1), (uint32_t)tt << sv.bshift);
     }
-    uint32_t more = 0;
-    bool ends = false;
+    bool ends = false, full = false;
     #pragma unroll
     for (int c = 0; c < C; ++c) {
       const int rem = min(sv.tlen, sv.plen + k0 + c) - n[c];  // to the end of diagonal k0 + c
-      int e = x[c] ? (first_set(x[c]) >> sv.bshift) : cpw;
-      if (x[c] == 0 && rem > cpw && n[c] >= 0) more |= 1u << c;
-      e = min(e, rem);
+      const int e = min(x[c] ? (first_set(x[c]) >> sv.bshift) : cpw, rem);
+      full |= x[c] == 0;
       ends |= e >= rem;
       n[c] += e;
     }
-    // Matches longer than one window.
+    // Matches longer than one window (a null cell has none).
+    uint32_t more = 0;
+    if (full) {
+      #pragma unroll
+      for (int c = 0; c < C; ++c) if (x[c] == 0 && n[c] >= 0 && n[c] < min(sv.tlen, sv.plen + k0 + c)) more |= 1u << c;
+    }
     #pragma unroll 1
     while (more) {
       const int c = __ffs((int)more) - 1;
@@ -196,37 +200,38 @@ __device__ __forceinline__ void tile_pass(const TileArgs& a, const SeqView& sv, 
   }
 }
 
-// The tiling of one block for L lanes: tiles, first diagonal, end of the last tile. One tile of
-// 4 L diagonals if they hold all of the rows' cells (the cells beside it are null), else tiles with
-// halos. narrow: two diagonals per lane hold the rows.
-struct TilePlan { int tiles, base, end; bool narrow; };
-__device__ __forceinline__ TilePlan tile_plan(int cb, int t0, int L) {
-  TilePlan p;
-  const int lo = row_lo(cb, t0 + 4) & ~3, width = row_hi(cb, t0 + 4) - lo + 1;
-  p.tiles = 1; p.base = lo; p.narrow = width <= 2 * L;
-  if (width > 4 * L) { p.tiles = (width + 119) / 120; p.base = lo - kTileHalo; }
-  p.end = p.base + (p.tiles - 1) * 120 + 4 * L;
-  return p;
+// The tiling of block t0 for L lanes into d.ts: tiles, first diagonal, end of the last tile. One tile
+// of 4 L diagonals if they hold all of the rows' cells (the cells beside it are null), else tiles with
+// halos. narrow: the last tile has two diagonals per lane. False when the ring does not hold them.
+__device__ __forceinline__ bool tile_plan(Dir& d, int t0, int L) {
+  const int lo = row_lo(d.cb, t0 + 4) & ~3, width = row_hi(d.cb, t0 + 4) - lo + 1;
+  int tiles = 1, base = lo;
+  bool narrow = width <= 2 * L;
+  if (width > 4 * L) {
+    tiles = (int)((unsigned)(width + 119) / 120u);
+    base = lo - kTileHalo;
+    narrow = width - (tiles - 1) * 120 <= 56;
+  }
+  const int end = base + (tiles - 1) * 120 + (narrow ? 2 : 4) * L;
+  d.ts.tiles = tiles; d.ts.base = base; d.ts.end = end; d.ts.narrow = narrow;
+  return end - base <= d.cfg.W;
 }
-// Whether half a warp holds block t0's rows, and whether the ring holds them.
+// Whether half a warp holds block t0's rows.
 __device__ __forceinline__ bool tile_half(int cb, int t0) { return row_hi(cb, t0 + 4) - (row_lo(cb, t0 + 4) & ~3) < 64; }
-__device__ __forceinline__ bool tile_fits(const Dir& d, int t0) {
-  const TilePlan p = tile_plan(d.cb, t0, 32);
-  return p.end - p.base <= d.cfg.W;
-}
-
-// The first extension of a direction's diagonal 0.
-__device__ __noinline__ int first_match(const uint32_t* pw, const uint32_t* tw, int p0, int t0, int n, int bshift) {
-  SeqView v;
-  v.pw = pw; v.tw = tw; v.p0 = p0; v.t0 = t0; v.plen = n; v.tlen = n; v.bshift = bshift;
-  return lcp(v, 0, 0);
-}
 
 // Starts a direction over window sv in component cb: row 0 with its extension. Returns its offset,
 // or -1 when it touches (then nothing is started).
 __device__ __noinline__ int tile_start(Dir& d, const SeqView& sv, int cb, int ce, int lane) {
   const int n = min(sv.plen, sv.tlen);
-  const int off0 = cb == CM ? first_match(sv.pw, sv.tw, sv.p0, sv.t0, n, sv.bshift) : 0;
+  int off0 = 0;
+  if (cb == CM) {
+    const int cpw = 32 >> sv.bshift;
+    #pragma unroll 1
+    for (; off0 < n; off0 += cpw) {
+      const uint32_t x = win32(sv.pw, sv.p0 + off0, sv.bshift) ^ win32(sv.tw, sv.t0 + off0, sv.bshift);
+      if (x) { off0 += first_set(x) >> sv.bshift; break; }
+    }
+  }
   if (off0 >= n) return -1;
   d.sv = sv; d.cb = cb; d.ce = ce;
   d.num_null = 0; d.status = ST_OK; d.status_score = 0; d.end_k = INT_MAX;
@@ -294,6 +299,114 @@ __device__ __noinline__ int tile_advance(Dir& d, const Pen& p, int s, const Grp<
   return dir_step<1, 0, false>(d, p, s, g, max_ak_out);
 }
 
+// The leaf store of a leaf whose rows come in tiles: row 0's one cell at 0, then block b's four rows
+// (M, I, D each) of leaf_n(b) diagonals from leaf_lo(cb, b) at leaf_at(b), all multiples of 4 that
+// cover row_lo .. row_hi. So a row's place follows from its number, without a descriptor.
+__device__ __forceinline__ int leaf_n(int b) { return 8 * b + 8; }
+__device__ __forceinline__ int leaf_lo(int cb, int b) { return cb == CI ? -4 * b : -4 * b - 4; }
+__device__ __forceinline__ int leaf_at(int b) { return 4 + 48 * b * (b + 1); }
+
+// Leaf descriptors of the scores from .. s, for the one-step functions.
+__device__ __noinline__ void leaf_describe(Dir& d, int s, int from, const Pen& p, int lane) {
+  const int q = max(from, 0) + lane;
+  if (q <= s) {
+    const int t = row_of(q, p), b = (t - 1) >> 2;
+    #pragma unroll 1
+    for (int ci = 0; ci < 3; ++ci) {
+      int4 ds = make_int4(kAbsent, INT_MIN, 0, 0);
+      if (holds_row(q, p) && row_exists(d.cb, t, ci))
+        ds = t == 0 ? make_int4(0, 0, 0, 0)
+                    : make_int4(row_lo(d.cb, t), row_hi(d.cb, t), leaf_at(b) + (((t - 1) & 3) * 3 + ci) * leaf_n(b),
+                                leaf_lo(d.cb, b));
+      d.cfg.ldesc[q * 3 + ci] = ds;
+    }
+  }
+  __syncwarp();
+}
+
+// leaf_backtrace for gap-affine over a leaf whose rows up to score `fast` came in tiles (later ones
+// have descriptors): a lane per source (0 mismatch, 1-2 I open/extend, 3-4 D open/extend), one
+// offset latency a step, and the packed maximum picks the source.
+__device__ __noinline__ int tile_backtrace(const Dir& B, const Pen& p, int s, int fast, RunOut& out, uint32_t* lruns,
+                                           int lruns_cap, int lane) {
+  const int cb = B.cb;
+  const int32_t* ldata = B.cfg.ldata;
+  const int plen = B.sv.plen, tlen = B.sv.tlen;
+  const bool ext = lane == 2 || lane == 4, del = lane >= 3;
+  const int back = lane == 0 ? p.x : ext ? p.e : p.o + p.e;
+  const int my_ci = ext ? (del ? 2 : 1) : 0, my_dk = lane == 0 ? 0 : del ? 1 : -1, my_add = del ? 0 : 1;
+  const int my_type = lane == 0 ? BT_M : del ? (ext ? BT_D_EXT : BT_D_OPEN) : (ext ? BT_I_EXT : BT_I_OPEN);
+  int ci = comp_index(B.ce), score = s, k = B.end_k, off = tlen, nrev = 0, rop = -1, rlen = 0;
+  bool over = false;
+  int left = plen + tlen + 8;
+  // A step's match and its operation, then the start's match and gaps; the last push stores the
+  // open run.
+  int tail = 0;
+  #pragma unroll 1
+  for (;;) {
+    int eq = 0, op = -2, len = 1;
+    if (tail == 0) {
+      int mine = INT_MIN;
+      bool walk = off - k > 0 && off > 0 && score > 0;
+      if (walk) {
+        if (--left < 0) return WFG_ST_UNATTAINABLE;
+        const int sc = score - back, kk = k + my_dk;
+        if (lane < 5 && sc >= 0 && (ci == 0 || (lane > 0 && del == (ci == 2)))) {
+          int o = kTNull;
+          if (sc > fast) {
+            o = ref_raw<1>(B.cfg, sc, my_ci).get(kk);
+          } else {
+            const int t = row_of(sc, p), b = (t - 1) >> 2;
+            int at = leaf_at(b) + (((t - 1) & 3) * 3 + my_ci) * leaf_n(b) + kk - leaf_lo(cb, b);
+            if (t == 0) at = my_ci == comp_index(cb) ? 0 : -1;
+            if (sc == t * p.tg && row_lo(cb, t) <= kk && kk <= row_hi(cb, t) && at >= 0) o = ldata[at];
+          }
+          if (o >= 0) mine = (o + my_add) * 16 + my_type;
+        }
+        const int best = __reduce_max_sync(kFull, mine);
+        walk = best >= 0;
+        if (walk && ci == 0) {
+          eq = off - (best >> 4);
+          off = best >> 4;
+          walk = off - k > 0 && off > 0;
+        }
+        if (walk) {
+          const int type = best & 15;
+          const bool e = type == BT_I_EXT || type == BT_D_EXT, d = type == BT_D_EXT || type == BT_D_OPEN;
+          score -= type == BT_M ? p.x : e ? p.e : p.o + p.e;
+          ci = e ? (d ? 2 : 1) : 0;
+          op = type == BT_M ? WFG_OP_X : d ? WFG_OP_DEL : WFG_OP_INS;
+          if (type != BT_M) k += d ? 1 : -1;
+          if (!d) --off;
+        }
+      }
+      if (!walk) { tail = 1; len = 0; }
+    } else {
+      const int v = off - k, h = off, nm = v > 0 && h > 0 ? min(v, h) : 0;
+      if (ci != 0 && (v != 0 || h != 0 || score != 0)) return WFG_ST_UNATTAINABLE;  // WFA2 aborts here
+      if (tail == 1) { eq = nm; op = WFG_OP_DEL; len = v - nm; }
+      if (tail == 2) { op = WFG_OP_INS; len = h - min(max(v, 0), h); }
+      ++tail;
+    }
+    #pragma unroll 1
+    for (int x = 0; x < 2; ++x) {
+      const int o = x == 0 ? WFG_OP_EQ : op, n = x == 0 ? eq : len;
+      if (n <= 0 && !(x == 1 && tail == 4)) continue;
+      if (o == rop) { rlen += n; continue; }
+      if (rlen > 0) {
+        if (nrev < lruns_cap) lruns[nrev] = ((uint32_t)rlen << 4) | (uint32_t)rop; else over = true;
+        ++nrev;
+      }
+      rop = o; rlen = n;
+    }
+    if (tail == 4) break;
+  }
+  if (over) return WFG_ST_SCRATCH_OVERFLOW;
+  __syncwarp();
+  out.append(lruns, nrev, lane, 32);
+  return ST_OK;
+}
+
 // wavefront_bialign_overlap over untouched rows: row s0 of d0 against the rows of scores s1,
 // s1 - 1, ... of d1. Cells meet where their antidiagonals add up to plen + tlen or more, so the
 // lanes first test the rows' largest ones, a row pair each, and only pairs that pass are scanned.
@@ -320,15 +433,27 @@ __device__ __noinline__ void tile_overlap(const Dir& d0, const Dir& d1, int s0, 
     const int end = min(row_hi(cb0, t0), A - row_lo(cb1, t1));
     int first[3] = {INT_MAX, INT_MAX, INT_MAX};  // lowest diagonal where M, I, D meet
     #pragma unroll 1
-    for (int kb = max(row_lo(cb0, t0), A - row_hi(cb1, t1)); kb <= end; kb += 32) {
-      const int k = kb + lane;
-      const uint32_t i0 = (uint32_t)k & mask, i1 = (uint32_t)(A - k) & mask;
-      const bool hit = k <= end && r0[i0] + r1[i1] >= tlen;
-      if (!__any_sync(kFull, hit)) continue;
-      if (hit) {
-        first[0] = min(first[0], k);
-        if (r0[pitch + i0] + r1[pitch + i1] >= tlen) first[1] = min(first[1], k);
-        if (r0[2 * pitch + i0] + r1[2 * pitch + i1] >= tlen) first[2] = min(first[2], k);
+    for (int kb = max(row_lo(cb0, t0), A - row_hi(cb1, t1)) + lane; kb - lane <= end; kb += 128) {
+      // four diagonals per lane, their loads in flight together
+      int sum[4];
+      sum[0] = kb <= end ? r0[(uint32_t)kb & mask] + r1[(uint32_t)(A - kb) & mask] : -1;
+      sum[1] = sum[2] = sum[3] = -1;
+      if (kb - lane + 32 <= end) {
+        #pragma unroll
+        for (int u = 1; u < 4; ++u) {
+          const int k = kb + 32 * u;
+          sum[u] = k <= end ? r0[(uint32_t)k & mask] + r1[(uint32_t)(A - k) & mask] : -1;
+        }
+      }
+      #pragma unroll 1
+      for (int u = 0, k = kb; max(max(sum[0], sum[1]), max(sum[2], sum[3])) >= tlen && u < 4; ++u, k += 32) {
+        if (sum[0] >= tlen) {
+          const uint32_t i0 = (uint32_t)k & mask, i1 = (uint32_t)(A - k) & mask;
+          first[0] = min(first[0], k);
+          if (r0[pitch + i0] + r1[pitch + i1] >= tlen) first[1] = min(first[1], k);
+          if (r0[2 * pitch + i0] + r1[2 * pitch + i1] >= tlen) first[2] = min(first[2], k);
+        }
+        sum[0] = sum[1]; sum[1] = sum[2]; sum[2] = sum[3]; sum[3] = -1;
       }
     }
     #pragma unroll
