@@ -12,6 +12,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "wfg_internal.h"
@@ -80,12 +81,9 @@ struct MlpParams {
 };
 constexpr int kOffW1 = 0, kOffB1 = kIn * kHid, kOffW2 = kOffB1 + kHid, kOffB2 = kOffW2 + kHid * kHid;
 constexpr int kOffW3 = kOffB2 + kHid, kOffB3 = kOffW3 + kHid, kParamCount = kOffB3 + 1;
-// Per-warp staging floats of the train step: h1, dh2 (16 x 64 each), x (16 x 32), dy (16),
-// the bf16 input tile (16 x 32 bf16 = 256 floats).
-constexpr int kTrainWarpFloats = 32 * kHid + 16 * kIn + 16 + (16 * kIn) / 2;
-constexpr int kTrainWpb = 4;
-constexpr size_t kTrainSmemBytes =
-    sizeof(float) * ((size_t)kHid * kHid + ((kParamCount + 3) & ~3) + (size_t)kTrainWpb * kTrainWarpFloats);
+// Train step: a block of 8 warps per 16-row tile. Row pitches of the staged matrices: W2's spreads
+// eight rows' 16-byte reads over all banks.
+constexpr int kTrainWarps = 8, kW2Pitch = kHid + 4, kHPitch = kHid + 4;
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -211,133 +209,191 @@ __global__ void __launch_bounds__(WPB * 32) mlp_forward_kernel(int n, const __nv
   }
 }
 
-// Training step: forward (tensor cores) + backward (fp32) of the mean-squared error on a
-// minibatch of rows [row_begin, row_begin + rows); gradients are summed into grad (zeroed by
-// the caller). Per warp: one 16-row tile at a time, activations staged in shared memory.
-template <int WPB>
-__global__ void __launch_bounds__(WPB * 32) mlp_train_step_kernel(const __nv_bfloat16* __restrict__ x,
-                                                                 const float* __restrict__ target,
-                                                                 const int* __restrict__ rows_idx, int rows,
-                                                                 MlpParams prm, float* __restrict__ grad,
-                                                                 float* __restrict__ loss_sum) {
+// Training step: forward (tensor cores) + backward (fp32) of the mean-squared error on a minibatch of
+// `rows` rows (rows_idx); gradients and the squared error are added to grad and loss_sum. step_next,
+// if given, is advanced by one (the Adam step that follows uses *step_next - 1).
+//
+// A minibatch of 2,048 rows is 128 tiles of 16 rows: a block of 8 warps takes a tile (more when there
+// are more tiles than SMs), each warp an eighth of every layer's columns, and each thread keeps its
+// 16 + 8 sums of dW2 and dW1 in registers over the block's tiles. With a warp per tile (four per block,
+// 32 blocks on 152 SMs) and the sums in shared memory by atomics, a step took 58 us (ncu, caches
+// flushed); now 25 us. What bounds it: latency, of the parameters' load into shared memory and of the
+// chain of a tile's five products between barriers; then the 6,465 sums that each block adds to the
+// gradient. Two epochs of 16,384 rows, end to end on a GB300: 1,224 -> 667 us.
+__global__ void __launch_bounds__(kTrainWarps * 32) mlp_train_step_kernel(const __nv_bfloat16* __restrict__ x,
+                                                                          const float* __restrict__ target,
+                                                                          const int* __restrict__ rows_idx, int rows,
+                                                                          MlpParams prm, float* __restrict__ grad,
+                                                                          float* __restrict__ loss_sum,
+                                                                          int* __restrict__ step_next) {
   __shared__ __align__(16) __nv_bfloat16 s_w1t[kHid * kIn];
   __shared__ __align__(16) __nv_bfloat16 s_w2t[kHid * kHid];
   __shared__ float s_b1[kHid], s_b2[kHid], s_w3[kHid];
-  // Dynamic shared memory (train_step_smem_bytes): fp32 W2 [in][out] for dH1, the block's
-  // gradient accumulator, and per-warp staging of one 16-row tile.
-  extern __shared__ __align__(16) float s_dyn[];
-  float* s_w2 = s_dyn;                                       // kHid*kHid
-  float* s_g = s_w2 + kHid * kHid;                           // kParamCount (padded to 4)
-  float* s_warp = s_g + ((kParamCount + 3) & ~3);
-  const int wib0 = threadIdx.x >> 5;
-  float (*s_h1_w)[kHid] = reinterpret_cast<float (*)[kHid]>(s_warp + wib0 * kTrainWarpFloats);
-  float (*s_dh2_w)[kHid] = reinterpret_cast<float (*)[kHid]>(s_warp + wib0 * kTrainWarpFloats + 16 * kHid);
-  float (*s_xin_w)[kIn] = reinterpret_cast<float (*)[kIn]>(s_warp + wib0 * kTrainWarpFloats + 32 * kHid);
-  float* s_dy_w = s_warp + wib0 * kTrainWarpFloats + 32 * kHid + 16 * kIn;
-  __nv_bfloat16* s_xt_w = reinterpret_cast<__nv_bfloat16*>(s_warp + wib0 * kTrainWarpFloats + 32 * kHid + 16 * kIn + 16);
-  load_params_smem<WPB>(prm, s_w1t, s_w2t, s_b1, s_b2, s_w3);
-  for (int i = threadIdx.x; i < kHid * kHid; i += WPB * 32) s_w2[i] = prm.master[kOffW2 + i];
-  for (int i = threadIdx.x; i < kParamCount; i += WPB * 32) s_g[i] = 0.f;
-  __syncthreads();
-  const float b3 = prm.master[kOffB3];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const float inv_rows = 1.f / (float)rows;
-  float lsum = 0.f;
+  __shared__ __align__(16) float s_w2[kHid * kW2Pitch];                             // fp32 W2 [in][out]
+  __shared__ __align__(16) float s_x[16 * kIn], s_h1[16 * kHPitch], s_dh2[16 * kHPitch], s_dh1[16 * kHPitch];
+  __shared__ __align__(16) __nv_bfloat16 s_xb[16 * kIn];
+  __shared__ float s_part[kTrainWarps][16], s_dy[16];
+  const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5, g = lane >> 2, t = lane & 3;
+  load_params_smem<kTrainWarps>(prm, s_w1t, s_w2t, s_b1, s_b2, s_w3);
+  for (int i = tid; i < kHid * kHid; i += kTrainWarps * 32) s_w2[(i / kHid) * kW2Pitch + i % kHid] = prm.master[kOffW2 + i];
+  const float b3 = prm.master[kOffB3], inv_rows = 1.f / (float)rows;
+  // this thread's sums: dW2[i2 .. i2+15][j2], dW1[f1 .. f1+7][j2], db1/db2[tid], dW3 of columns c, c + 1
+  const int j2 = tid & 63, i2 = (tid >> 6) * 16, f1 = (tid >> 6) * 8, c = wib * 8 + 2 * t;
+  float dw2[16] = {}, dw1[8] = {}, db1 = 0.f, db2 = 0.f, dw3a = 0.f, dw3b = 0.f, db3 = 0.f, lsum = 0.f;
   const int tiles = (rows + 15) / 16;
-  for (int tile = blockIdx.x * WPB + wib; tile < tiles; tile += gridDim.x * WPB) {
-    // gather the tile's rows
-    for (int e = lane; e < 16 * kIn; e += 32) {
-      const int r = e / kIn, c = e % kIn;
-      const int rr = tile * 16 + r;
-      __nv_bfloat16 v = __float2bfloat16(0.f);
-      if (rr < rows) v = x[(size_t)rows_idx[rr] * kIn + c];
-      s_xt_w[e] = v;
-      s_xin_w[r][c] = __bfloat162float(v);
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    __syncthreads();
+    for (int e = tid; e < 16 * kIn; e += kTrainWarps * 32) {
+      const int rr = tile * 16 + e / kIn;
+      const __nv_bfloat16 v = rr < rows ? x[(size_t)rows_idx[rr] * kIn + e % kIn] : __float2bfloat16(0.f);
+      s_xb[e] = v;
+      s_x[e] = __bfloat162float(v);
     }
-    __syncwarp();
-    const int valid = min(16, rows - tile * 16);
-    TileAct act;
-    mlp_tile_forward(s_xt_w, 0, valid, s_w1t, s_w2t, s_b1, s_b2, s_w3, b3, lane, act);
-    // dL/dy = 2 (y - target) / rows
-    float dy0 = 0.f, dy1 = 0.f;
-    if (g < valid) { const float e0 = act.y[0] - target[rows_idx[tile * 16 + g]]; dy0 = 2.f * e0 * inv_rows; if (t == 0) lsum += e0 * e0; }
-    if (g + 8 < valid) { const float e1 = act.y[1] - target[rows_idx[tile * 16 + g + 8]]; dy1 = 2.f * e1 * inv_rows; if (t == 0) lsum += e1 * e1; }
-    if (t == 0) { s_dy_w[g] = dy0; s_dy_w[g + 8] = dy1; }
-    // stage h1 and dh2 = dy * w3 * (h2 > 0); accumulate dW3, db3
-    for (int j = 0; j < 8; ++j) {
-      const int c = j * 8 + 2 * t;
-      s_h1_w[g][c] = act.h1[j][0]; s_h1_w[g][c + 1] = act.h1[j][1];
-      s_h1_w[g + 8][c] = act.h1[j][2]; s_h1_w[g + 8][c + 1] = act.h1[j][3];
-      s_dh2_w[g][c] = act.h2[j][0] > 0.f ? dy0 * s_w3[c] : 0.f;
-      s_dh2_w[g][c + 1] = act.h2[j][1] > 0.f ? dy0 * s_w3[c + 1] : 0.f;
-      s_dh2_w[g + 8][c] = act.h2[j][2] > 0.f ? dy1 * s_w3[c] : 0.f;
-      s_dh2_w[g + 8][c + 1] = act.h2[j][3] > 0.f ? dy1 * s_w3[c + 1] : 0.f;
-      float gw0 = act.h2[j][0] * dy0 + act.h2[j][2] * dy1;
-      float gw1 = act.h2[j][1] * dy0 + act.h2[j][3] * dy1;
-      // sum over the 8 row-groups (lanes with equal t)
-      for (int off = 4; off < 32; off <<= 1) {
-        gw0 += __shfl_xor_sync(kFull, gw0, off);
-        gw1 += __shfl_xor_sync(kFull, gw1, off);
+    __syncthreads();
+    // Layer 1, this warp's 8 columns (fragment layouts: mlp_tile_forward)
+    {
+      float d[4] = {0.f, 0.f, 0.f, 0.f};
+      #pragma unroll
+      for (int ks = 0; ks < 2; ++ks) {
+        const int c0 = ks * 16 + 2 * t;
+        uint32_t a[4];
+        a[0] = *reinterpret_cast<const uint32_t*>(s_xb + g * kIn + c0);
+        a[1] = *reinterpret_cast<const uint32_t*>(s_xb + (g + 8) * kIn + c0);
+        a[2] = *reinterpret_cast<const uint32_t*>(s_xb + g * kIn + c0 + 8);
+        a[3] = *reinterpret_cast<const uint32_t*>(s_xb + (g + 8) * kIn + c0 + 8);
+        const __nv_bfloat16* w = s_w1t + (wib * 8 + g) * kIn + c0;
+        mma_bf16(d, a, *reinterpret_cast<const uint32_t*>(w), *reinterpret_cast<const uint32_t*>(w + 8));
       }
-      if (g == 0) { atomicAdd(&s_g[kOffW3 + c], gw0); atomicAdd(&s_g[kOffW3 + c + 1], gw1); }
+      #pragma unroll
+      for (int q = 0; q < 4; ++q)
+        s_h1[(g + 8 * (q >> 1)) * kHPitch + c + (q & 1)] =
+            __bfloat162float(__float2bfloat16(fmaxf(d[q] + s_b1[c + (q & 1)], 0.f)));
+    }
+    __syncthreads();
+    // Layer 2 and this warp's part of the output
+    float h2[4] = {0.f, 0.f, 0.f, 0.f};
+    #pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+      const int c0 = ks * 16 + 2 * t;
+      const float* r0 = s_h1 + g * kHPitch + c0;
+      const float* r1 = r0 + 8 * kHPitch;
+      uint32_t a[4] = {pack_bf16x2(r0[0], r0[1]), pack_bf16x2(r1[0], r1[1]), pack_bf16x2(r0[8], r0[9]),
+                       pack_bf16x2(r1[8], r1[9])};
+      const __nv_bfloat16* w = s_w2t + (wib * 8 + g) * kHid + c0;
+      mma_bf16(h2, a, *reinterpret_cast<const uint32_t*>(w), *reinterpret_cast<const uint32_t*>(w + 8));
+    }
+    #pragma unroll
+    for (int q = 0; q < 4; ++q) h2[q] = fmaxf(h2[q] + s_b2[c + (q & 1)], 0.f);
+    float y0 = h2[0] * s_w3[c] + h2[1] * s_w3[c + 1], y1 = h2[2] * s_w3[c] + h2[3] * s_w3[c + 1];
+    y0 += __shfl_xor_sync(kFull, y0, 1); y0 += __shfl_xor_sync(kFull, y0, 2);
+    y1 += __shfl_xor_sync(kFull, y1, 1); y1 += __shfl_xor_sync(kFull, y1, 2);
+    if (t == 0) { s_part[wib][g] = y0; s_part[wib][g + 8] = y1; }
+    __syncthreads();
+    if (tid < 16) {  // dL/dy = 2 (y - target) / rows
+      const int rr = tile * 16 + tid;
+      float dy = 0.f;
+      if (rr < rows) {
+        float y = 0.f;
+        #pragma unroll
+        for (int w = 0; w < kTrainWarps; ++w) y += s_part[w][tid];
+        const float e = y + b3 - target[rows_idx[rr]];
+        dy = 2.f * e * inv_rows;
+        lsum += e * e;
+        db3 += dy;
+      }
+      s_dy[tid] = dy;
+    }
+    __syncthreads();
+    // dh2 = dy * w3 * (h2 > 0), dW3
+    const float dy0 = s_dy[g], dy1 = s_dy[g + 8];
+    #pragma unroll
+    for (int q = 0; q < 4; ++q)
+      s_dh2[(g + 8 * (q >> 1)) * kHPitch + c + (q & 1)] = h2[q] > 0.f ? (q < 2 ? dy0 : dy1) * s_w3[c + (q & 1)] : 0.f;
+    dw3a += h2[0] * dy0 + h2[2] * dy1;
+    dw3b += h2[1] * dy0 + h2[3] * dy1;
+    __syncthreads();
+    // dh1[r][i] = (h1 > 0) * sum_j dh2[r][j] W2[i][j]: row tid / 16, columns tid % 16 + 16 q
+    {
+      const int r = tid >> 4, i0 = tid & 15;
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+      #pragma unroll 4
+      for (int j = 0; j < kHid; j += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(s_dh2 + r * kHPitch + j);
+        #pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float4 w = *reinterpret_cast<const float4*>(s_w2 + (i0 + 16 * q) * kW2Pitch + j);
+          acc[q] += v.x * w.x; acc[q] += v.y * w.y; acc[q] += v.z * w.z; acc[q] += v.w * w.w;
+        }
+      }
+      #pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int at = r * kHPitch + i0 + 16 * q;
+        s_dh1[at] = s_h1[at] > 0.f ? acc[q] : 0.f;
+      }
+    }
+    // dW2[i][j] = sum_r h1[r][i] dh2[r][j], db2
+    #pragma unroll 4
+    for (int r = 0; r < 16; ++r) {
+      const float dh = s_dh2[r * kHPitch + j2];
+      #pragma unroll
+      for (int q = 0; q < 16; q += 4) {
+        const float4 h = *reinterpret_cast<const float4*>(s_h1 + r * kHPitch + i2 + q);
+        dw2[q] += h.x * dh; dw2[q + 1] += h.y * dh; dw2[q + 2] += h.z * dh; dw2[q + 3] += h.w * dh;
+      }
+      if (tid < kHid) db2 += dh;
+    }
+    __syncthreads();
+    // dW1[f][i] = sum_r x[r][f] dh1[r][i], db1
+    #pragma unroll 4
+    for (int r = 0; r < 16; ++r) {
+      const float dh = s_dh1[r * kHPitch + j2];
+      #pragma unroll
+      for (int q = 0; q < 8; q += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(s_x + r * kIn + f1 + q);
+        dw1[q] += v.x * dh; dw1[q + 1] += v.y * dh; dw1[q + 2] += v.z * dh; dw1[q + 3] += v.w * dh;
+      }
+      if (tid < kHid) db1 += dh;
+    }
+  }
+  // The block's sums into the gradient.
+  #pragma unroll
+  for (int q = 0; q < 16; ++q) atomicAdd(&grad[kOffW2 + (i2 + q) * kHid + j2], dw2[q]);
+  #pragma unroll
+  for (int q = 0; q < 8; ++q) atomicAdd(&grad[kOffW1 + (f1 + q) * kHid + j2], dw1[q]);
+  if (tid < kHid) { atomicAdd(&grad[kOffB1 + tid], db1); atomicAdd(&grad[kOffB2 + tid], db2); }
+  #pragma unroll
+  for (int off = 4; off < 32; off <<= 1) {  // over the rows (lanes with equal t)
+    dw3a += __shfl_xor_sync(kFull, dw3a, off);
+    dw3b += __shfl_xor_sync(kFull, dw3b, off);
+  }
+  if (g == 0) { atomicAdd(&grad[kOffW3 + c], dw3a); atomicAdd(&grad[kOffW3 + c + 1], dw3b); }
+  if (wib == 0) {
+    #pragma unroll
+    for (int off = 8; off > 0; off >>= 1) {
+      lsum += __shfl_xor_sync(kFull, lsum, off);
+      db3 += __shfl_xor_sync(kFull, db3, off);
     }
     if (lane == 0) {
-      float db3 = 0.f;
-      for (int r = 0; r < 16; ++r) db3 += s_dy_w[r];
-      atomicAdd(&s_g[kOffB3], db3);
+      atomicAdd(&grad[kOffB3], db3);
+      if (loss_sum) atomicAdd(loss_sum, lsum);
+      if (step_next && blockIdx.x == 0) *step_next += 1;
     }
-    __syncwarp();
-    // dW2[i][j] = sum_r h1[r][i] dh2[r][j]; db2[j] = sum_r dh2[r][j]; lane owns 2 columns j
-    for (int jj = 0; jj < 2; ++jj) {
-      const int j = lane * 2 + jj;
-      float db2 = 0.f;
-      for (int r = 0; r < 16; ++r) db2 += s_dh2_w[r][j];
-      atomicAdd(&s_g[kOffB2 + j], db2);
-      for (int i = 0; i < kHid; ++i) {
-        float acc = 0.f;
-        for (int r = 0; r < 16; ++r) acc += s_h1_w[r][i] * s_dh2_w[r][j];
-        atomicAdd(&s_g[kOffW2 + i * kHid + j], acc);
-      }
-    }
-    // dh1[r][i] = (h1 > 0) * sum_j dh2[r][j] W2[i][j]; dW1[f][i] = sum_r x[r][f] dh1[r][i]
-    for (int ii = 0; ii < 2; ++ii) {
-      const int i = lane * 2 + ii;
-      float dh1[16];
-      for (int r = 0; r < 16; ++r) {
-        float acc = 0.f;
-        for (int j = 0; j < kHid; ++j) acc += s_dh2_w[r][j] * s_w2[i * kHid + j];
-        dh1[r] = s_h1_w[r][i] > 0.f ? acc : 0.f;
-      }
-      float db1 = 0.f;
-      for (int r = 0; r < 16; ++r) db1 += dh1[r];
-      atomicAdd(&s_g[kOffB1 + i], db1);
-      for (int f = 0; f < kIn; ++f) {
-        float acc = 0.f;
-        for (int r = 0; r < 16; ++r) acc += s_xin_w[r][f] * dh1[r];
-        atomicAdd(&s_g[kOffW1 + f * kHid + i], acc);
-      }
-    }
-    __syncwarp();
   }
-  lsum = __reduce_add_sync(kFull, (int)0) + lsum;  // keep warps converged
-  for (int off = 16; off > 0; off >>= 1) lsum += __shfl_xor_sync(kFull, lsum, off);
-  if (lane == 0 && loss_sum) atomicAdd(loss_sum, lsum);
-  __syncthreads();
-  for (int i = threadIdx.x; i < kParamCount; i += WPB * 32) atomicAdd(&grad[i], s_g[i]);
 }
 
 // Adam update of the fp32 master parameters, then the bf16 transposed weight copies.
-// step points at the 1-based Adam step count in device memory, so a captured training
-// epoch replays with fresh bias corrections; the last block advances it.
-__global__ void mlp_adam_kernel(float* __restrict__ master, const float* __restrict__ grad, float* __restrict__ m,
+// step_next points at the next 1-based Adam step in device memory (the train step has advanced it),
+// so a captured training epoch replays with fresh bias corrections. The gradient is zeroed for the
+// next train step.
+__global__ void mlp_adam_kernel(float* __restrict__ master, float* __restrict__ grad, float* __restrict__ m,
                                 float* __restrict__ v, float lr, float beta1, float beta2, float eps,
-                                const int* __restrict__ step, __nv_bfloat16* __restrict__ w1t,
+                                const int* __restrict__ step_next, __nv_bfloat16* __restrict__ w1t,
                                 __nv_bfloat16* __restrict__ w2t) {
-  const float t = (float)(*step);
+  const float t = (float)(*step_next - 1);
   const float bc1 = 1.f - powf(beta1, t), bc2 = 1.f - powf(beta2, t);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kParamCount; i += gridDim.x * blockDim.x) {
     const float gi = grad[i];
+    grad[i] = 0.f;
     const float mi = beta1 * m[i] + (1.f - beta1) * gi;
     const float vi = beta2 * v[i] + (1.f - beta2) * gi * gi;
     m[i] = mi;
@@ -387,34 +443,19 @@ cudaError_t launch_mlp_forward(int n, const void* feats_bf16, const float* maste
 
 cudaError_t launch_mlp_train_step(const void* feats_bf16, const float* target, const int* rows_idx, int rows,
                                   const float* master, const void* w1t, const void* w2t, float* grad, float* loss_sum,
-                                  int num_sms, cudaStream_t stream) {
+                                  int* step_next, int num_sms, cudaStream_t stream) {
   if (rows <= 0) return cudaSuccess;
-  constexpr int WPB = kTrainWpb;
-  static bool attr_set = false;
-  if (!attr_set) {
-    const cudaError_t e = cudaFuncSetAttribute(mlp_train_step_kernel<WPB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)kTrainSmemBytes);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
   MlpParams prm{master, (const __nv_bfloat16*)w1t, (const __nv_bfloat16*)w2t};
-  const int tiles = (rows + 15) / 16;
-  long long blocks = ((long long)tiles + WPB - 1) / WPB;
-  if (blocks > (long long)num_sms * 2) blocks = (long long)num_sms * 2;
-  mlp_train_step_kernel<WPB><<<(int)blocks, WPB * 32, kTrainSmemBytes, stream>>>((const __nv_bfloat16*)feats_bf16, target,
-                                                                   rows_idx, rows, prm, grad, loss_sum);
+  const int blocks = std::min((rows + 15) / 16, num_sms);
+  mlp_train_step_kernel<<<blocks, kTrainWarps * 32, 0, stream>>>((const __nv_bfloat16*)feats_bf16, target, rows_idx, rows,
+                                                                 prm, grad, loss_sum, step_next);
   return cudaGetLastError();
 }
 
-__global__ void mlp_step_advance_kernel(int* step) { *step += 1; }
-
-cudaError_t launch_mlp_adam(float* master, const float* grad, float* m, float* v, float lr, float beta1, float beta2,
-                            float eps, const int* step, void* w1t, void* w2t, cudaStream_t stream) {
-  mlp_adam_kernel<<<(kParamCount + 255) / 256, 256, 0, stream>>>(master, grad, m, v, lr, beta1, beta2, eps, step,
+cudaError_t launch_mlp_adam(float* master, float* grad, float* m, float* v, float lr, float beta1, float beta2,
+                            float eps, const int* step_next, void* w1t, void* w2t, cudaStream_t stream) {
+  mlp_adam_kernel<<<(kParamCount + 127) / 128, 128, 0, stream>>>(master, grad, m, v, lr, beta1, beta2, eps, step_next,
                                                                  (__nv_bfloat16*)w1t, (__nv_bfloat16*)w2t);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  mlp_step_advance_kernel<<<1, 1, 0, stream>>>(const_cast<int*>(step));
   return cudaGetLastError();
 }
 

@@ -80,9 +80,9 @@ cudaError_t launch_mlp_forward(int n, const void* feats_bf16, const float* maste
                                float* y_out, float* score_out, int num_sms, cudaStream_t stream);
 cudaError_t launch_mlp_train_step(const void* feats_bf16, const float* target, const int* rows_idx, int rows,
                                   const float* master, const void* w1t, const void* w2t, float* grad, float* loss_sum,
-                                  int num_sms, cudaStream_t stream);
-cudaError_t launch_mlp_adam(float* master, const float* grad, float* m, float* v, float lr, float beta1, float beta2,
-                            float eps, const int* step, void* w1t, void* w2t, cudaStream_t stream);
+                                  int* step_next, int num_sms, cudaStream_t stream);
+cudaError_t launch_mlp_adam(float* master, float* grad, float* m, float* v, float lr, float beta1, float beta2,
+                            float eps, const int* step_next, void* w1t, void* w2t, cudaStream_t stream);
 int sched_bin_words();
 cudaError_t launch_bin_order(int n, const float* pred, float wide_threshold, int wide_cap, int* work, int* stats,
                              int* order, int num_sms, cudaStream_t stream, int base = 0);

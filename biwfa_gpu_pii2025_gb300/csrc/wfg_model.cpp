@@ -147,7 +147,7 @@ int wfg_model_gradient(wfg_model_t* m, wfg_context_t* c, const float* log_target
   WFG_CHECK(c, cudaMemsetAsync(m->d_grad.ptr, 0, sizeof(float) * (size_t)m->nparams, c->stream));
   WFG_CHECK(c, cudaMemsetAsync(m->d_loss.ptr, 0, sizeof(float), c->stream));
   WFG_CHECK(c, launch_mlp_train_step(c->d_feats.ptr, m->d_targets.ptr, m->d_rows.ptr, n, m->d_master.ptr, m->d_w1t.ptr,
-                                     m->d_w2t.ptr, m->d_grad.ptr, m->d_loss.ptr, c->num_sms, c->stream));
+                                     m->d_w2t.ptr, m->d_grad.ptr, m->d_loss.ptr, nullptr, c->num_sms, c->stream));
   WFG_CHECK(c, cudaMemcpyAsync(grad, m->d_grad.ptr, sizeof(float) * (size_t)m->nparams, cudaMemcpyDeviceToHost, c->stream));
   float lsum = 0.f;
   WFG_CHECK(c, cudaMemcpyAsync(&lsum, m->d_loss.ptr, sizeof(float), cudaMemcpyDeviceToHost, c->stream));
@@ -177,12 +177,13 @@ int wfg_model_train(wfg_model_t* m, wfg_context_t* c, const int* target_scores, 
     cudaGraph_t graph;
     WFG_CHECK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t err = cudaSuccess;
-    for (int b0 = 0; b0 < n && err == cudaSuccess; b0 += batch_rows) {
-      const int rows = std::min(batch_rows, n - b0);
-      err = cudaMemsetAsync(m->d_grad.ptr, 0, sizeof(float) * (size_t)m->nparams, c->stream);
+    err = cudaMemsetAsync(m->d_grad.ptr, 0, sizeof(float) * (size_t)m->nparams, c->stream);  // Adam zeroes it from then on
+    for (int64_t b0 = 0; b0 < n && err == cudaSuccess; b0 += batch_rows) {
+      const int rows = (int)std::min<int64_t>(batch_rows, n - b0);
       if (err == cudaSuccess)
         err = launch_mlp_train_step(c->d_feats.ptr, m->d_targets.ptr, m->d_rows.ptr + b0, rows, m->d_master.ptr,
-                                    m->d_w1t.ptr, m->d_w2t.ptr, m->d_grad.ptr, m->d_loss.ptr, c->num_sms, c->stream);
+                                    m->d_w1t.ptr, m->d_w2t.ptr, m->d_grad.ptr, m->d_loss.ptr, m->d_step.ptr, c->num_sms,
+                                    c->stream);
       if (err == cudaSuccess)
         err = launch_mlp_adam(m->d_master.ptr, m->d_grad.ptr, m->d_m.ptr, m->d_v.ptr, lr, beta1, beta2, eps,
                               m->d_step.ptr, m->d_w1t.ptr, m->d_w2t.ptr, c->stream);
