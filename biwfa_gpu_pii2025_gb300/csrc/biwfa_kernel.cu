@@ -1556,12 +1556,8 @@ int biwfa_kernel_kind(int metric, int scope, int tile_g) {
 // biwfa_kernel_kind).
 cudaError_t biwfa_occupancy_shape(int gw, int ring_in_smem, size_t dyn, int* blocks_per_sm, int kind) {
   if (kind == 3)
-  {
-    const cudaError_t e = tile_kernel_attributes();
-    if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, biwfa_tile_kernel, kTileWarps * 32,
                                                          sizeof(TileBlockSmem));
-  }
   if (kind == 2) return occupancy_shape<true, kMaxScope2p>(gw, ring_in_smem, dyn, blocks_per_sm);
   if (kind == 1) return occupancy_shape<false, kMaxScope2p>(gw, ring_in_smem, dyn, blocks_per_sm);
   return occupancy_shape<false, kMaxScope>(gw, ring_in_smem, dyn, blocks_per_sm);
@@ -1577,8 +1573,6 @@ int biwfa_groups_per_block(int group_warps, int tile_g) {
 cudaError_t launch_biwfa(const KernelParams& p, int grid, cudaStream_t stream) {
   const int kind = biwfa_kernel_kind(p.metric, p.scope, p.tile_g);
   if (kind == 3) {
-    const cudaError_t e = tile_kernel_attributes();
-    if (e != cudaSuccess) return e;
     biwfa_tile_kernel<<<grid, kTileWarps * 32, sizeof(TileBlockSmem), stream>>>(p);
     return cudaGetLastError();
   }

@@ -96,6 +96,7 @@ struct TileBlockSmem {
 };
 // The block's shared memory, named rather than passed: a function that gets a pointer to it reads it
 // with generic loads and 64-bit addresses, a third more code.
+static_assert(sizeof(TileBlockSmem) <= 48 * 1024, "more shared memory than a launch gets without asking");
 extern __shared__ __align__(16) unsigned char s_tile_smem[];
 __device__ __forceinline__ TileBlockSmem& tile_smem() { return *reinterpret_cast<TileBlockSmem*>(s_tile_smem); }
 
@@ -727,9 +728,3 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks) biwfa_tile_kerne
     __syncwarp();
   }
 }
-
-namespace {
-cudaError_t tile_kernel_attributes() {
-  return cudaFuncSetAttribute(biwfa_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileBlockSmem));
-}
-}  // namespace

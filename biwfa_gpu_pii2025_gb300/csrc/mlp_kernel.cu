@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(WPB * 32) mlp_forward_kernel(int n, const __nv
 // 32 blocks on 152 SMs) and the sums in shared memory by atomics, a step took 58 us (ncu, caches
 // flushed); now 25 us. What bounds it: latency, of the parameters' load into shared memory and of the
 // chain of a tile's five products between barriers; then the 6,465 sums that each block adds to the
-// gradient. Two epochs of 16,384 rows, end to end on a GB300: 1,224 -> 667 us.
+// gradient. Two epochs of 16,384 rows, end to end on a GB300: 1,221 -> 667 us.
 __global__ void __launch_bounds__(kTrainWarps * 32) mlp_train_step_kernel(const __nv_bfloat16* __restrict__ x,
                                                                           const float* __restrict__ target,
                                                                           const int* __restrict__ rows_idx, int rows,
@@ -456,6 +456,18 @@ cudaError_t launch_mlp_adam(float* master, float* grad, float* m, float* v, floa
                             float eps, const int* step_next, void* w1t, void* w2t, cudaStream_t stream) {
   mlp_adam_kernel<<<(kParamCount + 127) / 128, 128, 0, stream>>>(master, grad, m, v, lr, beta1, beta2, eps, step_next,
                                                                  (__nv_bfloat16*)w1t, (__nv_bfloat16*)w2t);
+  return cudaGetLastError();
+}
+
+// Training targets log(1 + |score|), rounded from 64 bits.
+__global__ void mlp_targets_kernel(int n, const int* __restrict__ scores, float* __restrict__ targets) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    targets[i] = (float)log1p(fabs((double)scores[i]));
+}
+
+cudaError_t launch_mlp_targets(int n, const int* scores, float* targets, cudaStream_t stream) {
+  if (n <= 0) return cudaSuccess;
+  mlp_targets_kernel<<<std::min((n + 255) / 256, 1024), 256, 0, stream>>>(n, scores, targets);
   return cudaGetLastError();
 }
 

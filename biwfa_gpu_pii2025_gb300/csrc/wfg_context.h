@@ -83,6 +83,7 @@ cudaError_t launch_mlp_train_step(const void* feats_bf16, const float* target, c
                                   int* step_next, int num_sms, cudaStream_t stream);
 cudaError_t launch_mlp_adam(float* master, float* grad, float* m, float* v, float lr, float beta1, float beta2,
                             float eps, const int* step_next, void* w1t, void* w2t, cudaStream_t stream);
+cudaError_t launch_mlp_targets(int n, const int* scores, float* targets, cudaStream_t stream);
 int sched_bin_words();
 cudaError_t launch_bin_order(int n, const float* pred, float wide_threshold, int wide_cap, int* work, int* stats,
                              int* order, int num_sms, cudaStream_t stream, int base = 0);
@@ -156,6 +157,9 @@ struct wfg_context {
   double upload_host_ms = 0.0;
   bool uploaded = false;
   cudaGraphExec_t graph_exec = nullptr;
+  // resident blocks per SM of the launch shapes asked for so far
+  struct Occupancy { int kind, gw, smem; size_t dyn; int blocks; };
+  mutable std::vector<Occupancy> occupancy;
   wfg::PinBuf<int> h_order_pin;  // the processing order, copied by the graph's first node
 };
 

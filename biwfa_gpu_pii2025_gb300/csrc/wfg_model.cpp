@@ -20,6 +20,10 @@ struct wfg_model {
   DevBuf<float> d_master, d_grad, d_m, d_v, d_loss, d_targets;
   DevBuf<uint16_t> d_w1t, d_w2t;  // bf16 bit patterns
   DevBuf<int> d_rows, d_step;
+  // training workspaces: two epochs' row orders and the scores (pinned), each epoch's loss
+  PinBuf<int> h_rows;
+  PinBuf<float> h_loss;
+  cudaEvent_t rows_copied[2] = {};
   // captured epoch
   cudaGraphExec_t epoch_exec = nullptr;
   int graph_rows = -1, graph_batch = -1;
@@ -91,6 +95,8 @@ void wfg_model_destroy(wfg_model_t* m) {
   cudaSetDevice(m->device);
   if (m->epoch_exec) cudaGraphExecDestroy(m->epoch_exec);
   m->d_master.release(); m->d_grad.release(); m->d_m.release(); m->d_v.release(); m->d_loss.release();
+  m->h_rows.release(); m->h_loss.release();
+  for (cudaEvent_t e : m->rows_copied) if (e) cudaEventDestroy(e);
   m->d_targets.release(); m->d_w1t.release(); m->d_w2t.release(); m->d_rows.release(); m->d_step.release();
   delete m;
 }
@@ -164,11 +170,19 @@ int wfg_model_train(wfg_model_t* m, wfg_context_t* c, const int* target_scores, 
   if (n == 0) return WF_STATUS_ALG_COMPLETED;
   int st = ensure_features(c);
   if (st != WF_STATUS_ALG_COMPLETED) return st;
-  std::vector<float> tgt((size_t)n);
-  for (int i = 0; i < n; ++i) tgt[(size_t)i] = (float)std::log1p((double)std::abs((double)target_scores[i]));
   WFG_CHECK(c, m->d_targets.reserve((size_t)n));
   WFG_CHECK(c, m->d_rows.reserve((size_t)n));
-  WFG_CHECK(c, cudaMemcpyAsync(m->d_targets.ptr, tgt.data(), sizeof(float) * (size_t)n, cudaMemcpyHostToDevice, c->stream));
+  WFG_CHECK(c, m->h_rows.reserve((size_t)n * 2));
+  WFG_CHECK(c, m->h_loss.reserve((size_t)std::max(epochs, 1)));
+  for (cudaEvent_t& e : m->rows_copied)
+    if (!e) WFG_CHECK(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  // Targets log(1 + |score|), computed on the device from the scores (in 64 bits); d_rows carries the
+  // scores there and the row orders afterwards.
+  memcpy(m->h_rows.ptr + n, target_scores, sizeof(int) * (size_t)n);
+  WFG_CHECK(c, cudaMemcpyAsync(m->d_rows.ptr, m->h_rows.ptr + n, sizeof(int) * (size_t)n, cudaMemcpyHostToDevice,
+                               c->stream));
+  WFG_CHECK(c, cudaEventRecord(m->rows_copied[1], c->stream));
+  WFG_CHECK(c, launch_mlp_targets(n, m->d_rows.ptr, m->d_targets.ptr, c->stream));
   const float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
   // Capture one epoch (all minibatches) once; replays read the shuffled row order from d_rows.
   if (!m->epoch_exec || m->graph_rows != n || m->graph_batch != batch_rows || m->graph_lr != lr ||
@@ -196,23 +210,25 @@ int wfg_model_train(wfg_model_t* m, wfg_context_t* c, const int* target_scores, 
     if (inst != cudaSuccess) return wfg_fail(c, inst, "cudaGraphInstantiate");
     m->graph_rows = n; m->graph_batch = batch_rows; m->graph_lr = lr; m->graph_feats = c->d_feats.ptr;
   }
+  // The epochs run one after another on the stream; the host draws the next epoch's row order
+  // meanwhile and waits once, at the end.
   std::vector<int> rows((size_t)n);
   std::iota(rows.begin(), rows.end(), 0);
   Mix mix{seed};
-  PinBuf<int> h_rows;
-  WFG_CHECK(c, h_rows.reserve((size_t)n));
   for (int ep = 0; ep < epochs; ++ep) {
     for (int i = n - 1; i > 0; --i) std::swap(rows[(size_t)i], rows[(size_t)mix.below((uint64_t)i + 1)]);
-    memcpy(h_rows.ptr, rows.data(), sizeof(int) * (size_t)n);
-    WFG_CHECK(c, cudaMemcpyAsync(m->d_rows.ptr, h_rows.ptr, sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, c->stream));
+    int* h = m->h_rows.ptr + (size_t)(ep & 1) * (size_t)n;
+    if (ep > 0) WFG_CHECK(c, cudaEventSynchronize(m->rows_copied[ep & 1]));  // the buffer's last copy is done
+    memcpy(h, rows.data(), sizeof(int) * (size_t)n);
+    WFG_CHECK(c, cudaMemcpyAsync(m->d_rows.ptr, h, sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, c->stream));
+    WFG_CHECK(c, cudaEventRecord(m->rows_copied[ep & 1], c->stream));
     WFG_CHECK(c, cudaMemsetAsync(m->d_loss.ptr, 0, sizeof(float), c->stream));
     WFG_CHECK(c, cudaGraphLaunch(m->epoch_exec, c->stream));
-    float lsum = 0.f;
-    WFG_CHECK(c, cudaMemcpyAsync(&lsum, m->d_loss.ptr, sizeof(float), cudaMemcpyDeviceToHost, c->stream));
-    WFG_CHECK(c, cudaStreamSynchronize(c->stream));
-    if (epoch_loss) epoch_loss[ep] = lsum / (float)n;
+    WFG_CHECK(c, cudaMemcpyAsync(m->h_loss.ptr + ep, m->d_loss.ptr, sizeof(float), cudaMemcpyDeviceToHost, c->stream));
   }
-  h_rows.release();
+  WFG_CHECK(c, cudaStreamSynchronize(c->stream));
+  if (epoch_loss)
+    for (int ep = 0; ep < epochs; ++ep) epoch_loss[ep] = m->h_loss.ptr[ep] / (float)n;
   return WF_STATUS_ALG_COMPLETED;
 }
 

@@ -330,11 +330,17 @@ void size_launch(const wfg_context* c, const IntPen& p, int pass, int ring_w_hin
 // Groups that fit the device at once for a shape (persistent grid).
 int64_t max_groups(const wfg_context* c, const IntPen& p, const Launch& l) {
   const size_t dyn = l.smem ? (size_t)2 * p.nphys * p.nc * (size_t)l.ring_w * sizeof(int32_t) : 0;
+  // The device's answer for a shape does not change, so a context asks once.
+  const int kind = biwfa_kernel_kind(p.nc == 5 ? 4 : 0, p.scope, l.smem ? 0 : p.tile_g);
   int bps = 0;
-  if (biwfa_occupancy_shape(l.gw, l.smem, dyn, &bps, biwfa_kernel_kind(p.nc == 5 ? 4 : 0, p.scope, l.smem ? 0 : p.tile_g)) != cudaSuccess ||
-      bps < 1) {
-    (void)cudaGetLastError();
-    bps = 1;
+  for (const wfg_context::Occupancy& o : c->occupancy)
+    if (o.kind == kind && o.gw == l.gw && o.smem == l.smem && o.dyn == dyn) bps = o.blocks;
+  if (bps == 0) {
+    if (biwfa_occupancy_shape(l.gw, l.smem, dyn, &bps, kind) != cudaSuccess || bps < 1) {
+      (void)cudaGetLastError();
+      bps = 1;
+    }
+    if (c->occupancy.size() < 64) c->occupancy.push_back({kind, l.gw, l.smem, dyn, bps});
   }
   return (int64_t)bps * c->num_sms * biwfa_groups_per_block(l.gw, l.smem ? 0 : p.tile_g);
 }
@@ -379,7 +385,8 @@ KernelParams launch_params(const wfg_context* c, const wfg_config_t* cfg, const 
 
 // Shapes and arenas of the retry passes (1 .. kNumPasses-1), which realign the pairs that
 // overflowed the previous pass; returns the arena bytes the largest of them needs.
-int64_t plan_retry_passes(const wfg_context* c, const IntPen& p, int64_t arena_budget, Launch* retry) {
+int64_t plan_retry_passes(const wfg_context* c, const IntPen& p, int64_t arena_budget, Launch* retry,
+                          bool* short_of_memory = nullptr) {
   int64_t need = 0;
   for (int ps = 1; ps < kNumPasses; ++ps) {
     Launch& l = retry[ps];
@@ -389,6 +396,7 @@ int64_t plan_retry_passes(const wfg_context* c, const IntPen& p, int64_t arena_b
     int64_t gmax = std::min<int64_t>(max_groups(c, p, l), std::max<int64_t>(gpb, (int64_t)c->n));
     if (l.gw == 1) gmax = std::min<int64_t>(gmax, ps == 1 ? (int64_t)c->num_sms * 4 : (int64_t)c->num_sms * 2);
     const int64_t fit = arena_budget / std::max<int64_t>(l.L.total, 1);
+    if (short_of_memory && fit < gmax) *short_of_memory = true;
     l.groups = std::max<int64_t>(gpb, (std::min(gmax, fit) / gpb) * gpb);
     need = std::max(need, l.groups * l.L.total);
   }
@@ -397,7 +405,8 @@ int64_t plan_retry_passes(const wfg_context* c, const IntPen& p, int64_t arena_b
 
 // Launch sizes of the first pass over `count` pairs with ring hint `hint` (0: the plain cap):
 // groups in flight within the device's residency and the arena budget.
-void plan_first_pass(const wfg_context* c, const IntPen& p, int hint, int64_t arena_budget, Launch& l) {
+void plan_first_pass(const wfg_context* c, const IntPen& p, int hint, int64_t arena_budget, Launch& l,
+                     bool* short_of_memory = nullptr) {
   if (l.gw < 1) l.gw = 1;
   if (l.gw != 1 && l.gw != 4 && l.gw != 8) l.gw = 8;
   size_launch(c, p, 0, hint, l);
@@ -405,18 +414,21 @@ void plan_first_pass(const wfg_context* c, const IntPen& p, int hint, int64_t ar
   const int gpb = biwfa_groups_per_block(l.gw, l.smem ? 0 : p.tile_g);
   const int64_t gmax = std::min<int64_t>(max_groups(c, p, l), std::max<int64_t>(1, l.count) * gpb);
   const int64_t fit = arena_budget / std::max<int64_t>(l.L.total, 1);
+  if (short_of_memory && fit < gmax) *short_of_memory = true;
   l.groups = std::max<int64_t>(1, std::min(gmax, fit));
   l.groups = std::max<int64_t>(gpb, (l.groups / gpb) * gpb);
 }
 
 // The arena budget of a run: half of the device memory that is free or already held by the
-// arena, within [4 GiB, 96 GiB] (one GB300 has 288 GB of HBM).
+// arena, within [4 GiB, 96 GiB] (one GB300 has 288 GB of HBM). Asking for the free memory costs tens
+// of microseconds, so wfg_run plans with the least budget first.
+constexpr int64_t kLeastArenaBudget = (int64_t)4 << 30;
 int64_t arena_budget_of(const wfg_context* c) {
   int64_t budget = (int64_t)24 << 30;
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
     const int64_t avail = (int64_t)free_b + (int64_t)c->d_arena.cap;
-    budget = std::min<int64_t>((int64_t)96 << 30, std::max<int64_t>((int64_t)4 << 30, avail / 2));
+    budget = std::min<int64_t>((int64_t)96 << 30, std::max<int64_t>(kLeastArenaBudget, avail / 2));
   } else {
     (void)cudaGetLastError();
   }
@@ -551,8 +563,9 @@ int wfg_run(wfg_context_t* c, const wfg_config_t* cfg, wfg_sched_t sched) {
     // straight to a multi-warp launch with rings as wide as the batch's longest pair, on the aux
     // stream beside the single-warp launch: a single warp would take the longest of them far
     // beyond the rest of the batch, and their wavefronts outgrow the first pass's ring cap.
+    const bool by_length = sched == WFG_SCHED_SORTED && c->force_gw == 1 && !c->force_smem && c->limit_ring_w == 0;
     int n_long = 0;
-    if (sched == WFG_SCHED_SORTED && c->force_gw == 1 && !c->force_smem && c->limit_ring_w == 0)
+    if (by_length)
       while (n_long < n && c->h_plen[(size_t)order[(size_t)n_long]] + c->h_tlen[(size_t)order[(size_t)n_long]] >
                                kDirectWideSum)
         ++n_long;
@@ -569,16 +582,23 @@ int wfg_run(wfg_context_t* c, const wfg_config_t* cfg, wfg_sched_t sched) {
   }
   if (first.empty()) { Launch l; l.count = 0; first.push_back(l); }
   // ---- shapes and arena (pass-0 launches run concurrently; retry passes reuse the arena)
-  const int64_t arena_budget = arena_budget_of(c);
-  int64_t pass0_bytes = 0;
-  for (Launch& l : first) {
-    const int hint = l.ring_w > 0 ? l.ring_w + (p.tile_g ? WFG_TILE_MARGIN : 0) : c->limit_ring_w;
-    plan_first_pass(c, p, hint, arena_budget / (int64_t)first.size(), l);
-    l.arena_off = pass0_bytes;
-    pass0_bytes += l.groups * l.L.total;
-  }
+  const std::vector<Launch> planned = first;
   Launch retry[kNumPasses];
-  const int64_t arena_need = std::max(pass0_bytes, plan_retry_passes(c, p, arena_budget, retry));
+  int64_t arena_need = 0;
+  auto plan = [&](int64_t budget) {  // whether the budget holds the full launches
+    bool short_of_memory = false;
+    int64_t pass0_bytes = 0;
+    first = planned;
+    for (Launch& l : first) {
+      const int hint = l.ring_w > 0 ? l.ring_w + (p.tile_g ? WFG_TILE_MARGIN : 0) : c->limit_ring_w;
+      plan_first_pass(c, p, hint, budget / (int64_t)first.size(), l, &short_of_memory);
+      l.arena_off = pass0_bytes;
+      pass0_bytes += l.groups * l.L.total;
+    }
+    arena_need = std::max(pass0_bytes, plan_retry_passes(c, p, budget, retry, &short_of_memory));
+    return !short_of_memory;
+  };
+  if (!plan(kLeastArenaBudget)) plan(arena_budget_of(c));
   WFG_CHECK(c, c->d_arena.reserve((size_t)arena_need));
   int64_t num_batches = 0;
   for (const Launch& l : first)
