@@ -577,6 +577,21 @@ int wfg_run(wfg_context_t* c, const wfg_config_t* cfg, wfg_sched_t sched) {
     if (n - n_long > 0 || first.empty()) {
       Launch l; l.gw = c->force_gw; l.smem = c->force_smem; l.count = n - n_long; l.order_off = n_long;
       l.batched = (sched == WFG_SCHED_PLAIN);
+      // Two-piece: a wide pair on one warp can take as long as all the rest of the batch on the
+      // others. A pair's work grows with the square of its length; where the longest would take
+      // more than twice a warp's share of the batch, the first pass's rings hold 512 diagonals, so
+      // that pairs with wider wavefronts, and only those, go on to the 8-warp retry pass (their
+      // first 512 diagonals are computed twice). 4,000 pairs of 100 bp - 3 kbp, 1-8 %: 291 -> 146 ms; 500 of 5 kbp at 3-8 %: 830 -> 264 ms.
+      // A cut by length alone also sent low-error pairs, whose wavefronts are too narrow for eight
+      // warps (1,000 pairs of 1 kbp at 1 %: 6.9 ms against 4.3 ms for 2,000 on one warp each).
+      if (by_length && p.nc == 5 && c->tune.retry_warps > 1) {
+        double work = 0;
+        for (int i = 0; i < n; ++i) {
+          const double sum = (double)c->h_plen[(size_t)i] + c->h_tlen[(size_t)i];
+          work += sum * sum;
+        }
+        if ((double)c->max_sum * c->max_sum > 2.0 * work / (double)max_groups(c, p, l)) l.ring_w = kTailRingW;
+      }
       first.push_back(l);
     }
   }
