@@ -106,8 +106,9 @@ __device__ __forceinline__ WfRef absent_ref() {
 // gap-opening adjust of the overlap and its stop conditions (o for gap-affine, max(o, o2) for
 // two-piece gap-affine, 0 otherwise, wavefront/wavefront_bialign.c:396-410).
 // tg: spacing of the scores that hold a row when the rows are computed in tiles (biwfa_tiles.cuh;
-// 0: one score at a time); tm: its magic divisor.
-struct Pen { int x, o, e, scope, metric, go, tg; uint32_t tm; };
+// 0: one score at a time); tm: its magic divisor; lx, lo: one-component distances, rows back to the
+// mismatch (0: none) and the gap source, lom: lo's magic divisor.
+struct Pen { int x, o, e, scope, metric, go, tg; uint32_t tm; int lx, lo; uint32_t lom; };
 constexpr int kMetricAffine = 0, kMetricEdit = 1, kMetricIndel = 2, kMetricLinear = 3, kMetricAffine2p = 4;
 
 // Oriented window over packed words (forward arrays for the forward aligner and the
@@ -978,15 +979,15 @@ __device__ __forceinline__ int score_guard(const Pen& p, int plen, int tlen) {
 
 // The breakpoint search score by score from (sf, sr): resume 0 starts it, 1 and 2 enter the second
 // loop before the step of R or of F. TILES: one warp, rows that the tile kernel computed ahead come
-// first.
-template <int G, bool TWO, bool TILES>
+// first (1 gap-affine, 2 one component).
+template <int G, bool TWO, int TILES>
 __device__ __noinline__ int breakpoint_steps(Dir& F, Dir& R, int sf, int sr, int fmax, int rmax, bool last_fwd,
                                              int resume, int guard, const Pen p, int max_steps, BP& bp,
                                              const Grp<G> g) {
   const int max_antidiag = F.sv.plen + F.sv.tlen - 1;
   int ak = 0;
   auto step = [&](Dir& d, int s) -> int {
-    if constexpr (TILES) return tile_advance(d, p, s, g, &ak);
+    if constexpr (TILES != 0) return tile_advance<TILES == 2>(d, p, s, g, &ak);
     else return dir_step<G, 0, TWO>(d, p, s, g, &ak);
   };
   while (resume == 0) {
@@ -1049,7 +1050,7 @@ __device__ __noinline__ int find_breakpoint(Dir& F, Dir& R, const PairSeqs& q, i
   int fmax = 0, rmax = 0;
   if (dir_extend<G>(F, 0, g, &fmax)) return F.status;
   if (dir_extend<G>(R, 0, g, &rmax)) return R.status;
-  return breakpoint_steps<G, TWO, false>(F, R, 0, 0, fmax, rmax, false, 0, score_guard(p, pe - pb, te - tb), p, max_steps,
+  return breakpoint_steps<G, TWO, 0>(F, R, 0, 0, fmax, rmax, false, 0, score_guard(p, pe - pb, te - tb), p, max_steps,
                                          bp, g);
 }
 
@@ -1265,7 +1266,7 @@ __global__ void __launch_bounds__(G * GROUPS * 32, MINB) biwfa_persistent_kernel
   B.lcap = P.leaf_words; B.lused = 0;
   g.sync();
   const int go = P.metric == kMetricAffine ? P.o : P.metric == kMetricAffine2p ? max(P.o, P.o2) : 0;
-  const Pen pen = {P.x, P.o, P.e, P.scope, P.metric, go, 0, 0u};
+  const Pen pen = {P.x, P.o, P.e, P.scope, P.metric, go, 0, 0u, 0, 0, 0u};
 
   const unsigned long long num_pairs =
       P.num_pairs_ptr ? *P.num_pairs_ptr : (unsigned long long)P.num_pairs;
@@ -1547,17 +1548,19 @@ cudaError_t biwfa_occupancy(int* blocks_per_sm) {
 }
 
 // The kernel instantiation of a launch: 0 three components (scope <= 32), 1 three components
-// (scope <= 64), 2 two-piece gap-affine (scope <= 64), 3 the tile kernel.
+// (scope <= 64), 2 two-piece gap-affine (scope <= 64), 3 and 4 the tile kernel (gap-affine, one
+// component).
 int biwfa_kernel_kind(int metric, int scope, int tile_g) {
-  return tile_g > 0 ? 3 : metric == kMetricAffine2p ? 2 : (scope > kMaxScope ? 1 : 0);
+  return tile_g > 0 ? (metric == kMetricAffine ? 3 : 4) : metric == kMetricAffine2p ? 2 : (scope > kMaxScope ? 1 : 0);
 }
 
 // Resident blocks per SM of a shape (dyn: its dynamic shared memory in bytes; kind: as
 // biwfa_kernel_kind).
 cudaError_t biwfa_occupancy_shape(int gw, int ring_in_smem, size_t dyn, int* blocks_per_sm, int kind) {
-  if (kind == 3)
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, biwfa_tile_kernel, kTileWarps * 32,
-                                                         sizeof(TileBlockSmem));
+  if (kind >= 3)
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        blocks_per_sm, kind == 3 ? biwfa_tile_kernel<false> : biwfa_tile_kernel<true>, kTileWarps * 32,
+        sizeof(TileBlockSmem));
   if (kind == 2) return occupancy_shape<true, kMaxScope2p>(gw, ring_in_smem, dyn, blocks_per_sm);
   if (kind == 1) return occupancy_shape<false, kMaxScope2p>(gw, ring_in_smem, dyn, blocks_per_sm);
   return occupancy_shape<false, kMaxScope>(gw, ring_in_smem, dyn, blocks_per_sm);
@@ -1572,8 +1575,9 @@ int biwfa_groups_per_block(int group_warps, int tile_g) {
 
 cudaError_t launch_biwfa(const KernelParams& p, int grid, cudaStream_t stream) {
   const int kind = biwfa_kernel_kind(p.metric, p.scope, p.tile_g);
-  if (kind == 3) {
-    biwfa_tile_kernel<<<grid, kTileWarps * 32, sizeof(TileBlockSmem), stream>>>(p);
+  if (kind >= 3) {
+    if (kind == 3) biwfa_tile_kernel<false><<<grid, kTileWarps * 32, sizeof(TileBlockSmem), stream>>>(p);
+    else biwfa_tile_kernel<true><<<grid, kTileWarps * 32, sizeof(TileBlockSmem), stream>>>(p);
     return cudaGetLastError();
   }
   if (kind == 2) return launch_kernel<true, kMaxScope2p>(p, grid, stream);

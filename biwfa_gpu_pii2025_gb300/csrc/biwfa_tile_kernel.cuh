@@ -1,5 +1,5 @@
 // The kernel whose wavefront rows come in tiles (biwfa_tiles.cuh): score + CIGAR for gap-affine
-// penalties with x = 2g, o+e = 4g, e = g. Included by biwfa_kernel.cu inside namespace wfg.
+// penalties with x = 2g, o+e = 4g, e = g and for the one-component distances. Included by biwfa_kernel.cu inside namespace wfg.
 //
 // A warp owns a pair. Its work is a loop of blocks (four rows of one or both directions); the code
 // that computes a block stands once, in the kernel's loop, with the two common continuations (the
@@ -176,13 +176,14 @@ __device__ __noinline__ void job_open(int d, bool both, int t0, int state, int g
 
 // Sets up block t0 of dir[d] (both: and of dir[1]) as the warp's next pass, alone or as a job that
 // the block's idle warps share. state: what follows it. False when a ring does not hold the block.
+template <bool LIN>
 __device__ __noinline__ bool tile_request(int d, bool both, int t0, int state, int gib, int lane) {
   TileBlockSmem& B = tile_smem();
   TileGroup& S = B.grp[gib];
   TileCtl& C = S.ctl;
-  const bool halves = both && tile_half(S.dir[0].cb, t0) && tile_half(S.dir[1].cb, t0);
+  const bool halves = both && tile_half<LIN>(S.dir[0].cb, t0, S.pen) && tile_half<LIN>(S.dir[1].cb, t0, S.pen);
   const int L = halves ? 16 : 32;
-  if (!tile_plan(S.dir[d], t0, L) || (both && !tile_plan(S.dir[1], t0, L))) return false;
+  if (!tile_plan<LIN>(S.dir[d], t0, L, S.pen) || (both && !tile_plan<LIN>(S.dir[1], t0, L, S.pen))) return false;
   if (halves && !(S.dir[0].ts.narrow && S.dir[1].ts.narrow)) {  // one width for both
     S.dir[0].ts.narrow = S.dir[1].ts.narrow = 0;
     S.dir[0].ts.end = S.dir[0].ts.base + 64;
@@ -199,6 +200,7 @@ __device__ __noinline__ bool tile_request(int d, bool both, int t0, int state, i
 
 // Runs the warp's state machine to its next block pass (S.ctl says which); false when the launch has
 // no more work for this warp.
+template <bool LIN>
 __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
   TileBlockSmem& B = tile_smem();
   TileGroup& S = B.grp[gib];
@@ -245,7 +247,7 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
         for (int j = 0; j < 4; ++j) { nf = max(nf, C.part[j]); nr = max(nr, C.part[5 + j]); }
         if (min(C.part[4], C.part[9]) == 4 && nf + nr < C.max_antidiag && C.t0 <= C.guard) {
           const int t0 = C.t0;
-          if (tile_request(0, true, t0 + 4, kSearch, gib, lane)) {
+          if (tile_request<LIN>(0, true, t0 + 4, kSearch, gib, lane)) {
             C.fmax = nf; C.rmax = nr;
             __syncwarp();
             return true;
@@ -339,7 +341,7 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
       C.max_antidiag = C.pe - C.pb + C.te - C.tb - 1;
       bp.score = INT_MAX;
       const SeqView fv = fwd_view(C.q, C.pb, C.pe, C.tb, C.te), rv = rev_view(C.q, C.pb, C.pe, C.tb, C.te);
-      if (pen.tg == 0 || tile_start(F, fv, C.cb, C.ce, lane) < 0 || tile_start(R, rv, C.ce, C.cb, lane) < 0) {
+      if (pen.tg == 0 || tile_start<LIN>(F, fv, C.cb, C.ce, lane) < 0 || tile_start<LIN>(R, rv, C.ce, C.cb, lane) < 0) {
         st = find_breakpoint<1, false>(F, R, C.q, C.pb, C.pe, C.tb, C.te, C.cb, C.ce, pen, P.max_steps, bp, g);
         state = kBpDone;
       } else {
@@ -349,7 +351,7 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
         __syncwarp();
         if (C.fmax + C.rmax >= C.max_antidiag) {
           state = kMet;
-        } else if (tile_request(0, true, 0, kSearch, gib, lane)) {
+        } else if (tile_request<LIN>(0, true, 0, kSearch, gib, lane)) {
           C.out = out; C.bp = bp;
           return true;
         } else {
@@ -394,12 +396,12 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
         Dir& b = last_fwd ? R : F;
         if (!resumed) {
           if (s0 + max(s1 - (scope - 1), 0) - pen.go >= bp.score) { st = ST_OK; state = kBpDone; break; }
-          if (holds_row(s0, pen)) tile_overlap(last_fwd ? F : R, b, s0, s1, last_fwd, bp, pen, lane);
+          if (holds_row(s0, pen)) tile_overlap<LIN>(last_fwd ? F : R, b, s0, s1, last_fwd, bp, pen, lane);
         }
         resumed = false;
         if (holds_row(s1 + 1, pen)) {
           const int t = row_of(s1 + 1, pen);
-          if (t > b.ts.valid && !b.ts.touched && tile_request(last_fwd ? 1 : 0, false, b.ts.t, kMeet, gib, lane)) {
+          if (t > b.ts.valid && !b.ts.touched && tile_request<LIN>(last_fwd ? 1 : 0, false, b.ts.t, kMeet, gib, lane)) {
             C.sf = sf; C.sr = sr; C.last_fwd = last_fwd;
             C.out = out; C.bp = bp;
             __syncwarp();
@@ -417,9 +419,9 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
     }
 
     if (state == kSteps) {
-      tile_describe(F, C.sf, C.sf - pen.scope + 1, pen);
-      tile_describe(R, C.sr, C.sr - pen.scope + 1, pen);
-      st = breakpoint_steps<1, false, true>(F, R, C.sf, C.sr, C.fmax, C.rmax, C.last_fwd, resume, C.guard, pen, P.max_steps,
+      tile_describe<LIN>(F, C.sf, C.sf - pen.scope + 1, pen);
+      tile_describe<LIN>(R, C.sr, C.sr - pen.scope + 1, pen);
+      st = breakpoint_steps<1, false, LIN ? 2 : 1>(F, R, C.sf, C.sr, C.fmax, C.rmax, C.last_fwd, resume, C.guard, pen, P.max_steps,
                                             bp, g);
       resume = 0;
       state = kBpDone;
@@ -469,7 +471,7 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
       // ring of F holds the rows that the next block reads, the leaf store gets every row.
       const SeqView sv = fwd_view(C.q, C.pb, C.pe, C.tb, C.te);
       C.guard = score_guard(pen, C.pe - C.pb, C.te - C.tb);
-      const int off0 = pen.tg ? tile_start(F, sv, C.cb, C.ce, lane) : -1;
+      const int off0 = pen.tg ? tile_start<LIN>(F, sv, C.cb, C.ce, lane) : -1;
       if (off0 < 0) {
         st = leaf_align<1, false>(L, C.q, C.pb, C.pe, C.tb, C.te, C.cb, C.ce, pen, P.max_steps, out,
                                   S.arena.lruns, P.leaf_run_cap, g, &C.max_leaf);
@@ -481,11 +483,11 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
       }
       if (lane == 0) L.cfg.ldata[0] = off0;
       L.sv = sv; L.cb = C.cb; L.ce = C.ce; L.num_null = 0; L.status = ST_OK; L.end_k = sv.tlen - sv.plen;
-      C.leaf_end = leaf_at(0);
+      C.leaf_end = leaf_at<LIN>(0);
       __syncwarp();
       state = kLeafSteps;
       s = 0; done = false;
-      if (4 * pen.tg <= L.cfg.lmax && leaf_at(1) <= L.lcap && tile_request(0, false, 0, kLeaf, gib, lane)) {
+      if (4 * pen.tg <= L.cfg.lmax && leaf_at<LIN>(1) <= L.lcap && tile_request<LIN>(0, false, 0, kLeaf, gib, lane)) {
         C.out = out; C.bp = bp;
         __syncwarp();
         return true;
@@ -497,8 +499,9 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
       const int t0 = C.t0, touch = C.part[4], last = touch < 4 ? t0 + 1 + touch : t0 + 4, ci = comp_index(C.ce);
       const int ak = L.end_k;
       s = last * pen.tg;
-      if (touch < 4 && row_exists(C.cb, last, ci) && row_lo(C.cb, last) <= ak && ak <= row_hi(C.cb, last))
-        done = L.cfg.ldata[leaf_at(t0 >> 2) + (touch * 3 + ci) * leaf_n(t0 >> 2) + ak - leaf_lo(C.cb, t0 >> 2)] >= L.sv.tlen;
+      if (touch < 4 && row_exists<LIN>(C.cb, last, ci, pen) && row_lo<LIN>(C.cb, last, pen) <= ak &&
+          ak <= row_hi<LIN>(C.cb, last, pen))
+        done = L.cfg.ldata[leaf_cell<LIN>(C.cb, last, ci, ak)] >= L.sv.tlen;
       state = kLeafSteps;
     }
 
@@ -510,10 +513,10 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
       __syncwarp();
       st = ST_OK;
       if (!done) {
-        leaf_describe(L, s, s - pen.scope + 1, pen, lane);
+        leaf_describe<LIN>(L, s, s - pen.scope + 1, pen, lane);
         st = leaf_steps<1, false>(L, &s, C.guard, pen, P.max_steps, g);
       }
-      if (st == ST_OK) st = tile_backtrace(L, pen, s, fast, out, S.arena.lruns, P.leaf_run_cap, lane);
+      if (st == ST_OK) st = tile_backtrace<LIN>(L, pen, s, fast, out, S.arena.lruns, P.leaf_run_cap, lane);
       __syncwarp();
       C.max_leaf = max(C.max_leaf, s);
       if (st != ST_OK) C.status = st;
@@ -533,12 +536,14 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
         __syncwarp();
         if (status == WFG_ST_COMPLETED) {
           // cigar_score_gap_affine (alignment/cigar.c:277-303) over maximal runs, a lane's runs each
+          if (LIN && out.n > 0)
+            score = rescore_runs(out.buf, out.n, P.metric, P.match_o, P.x_o, P.o_o, P.e_o, P.o2_o, P.e2_o);
           #pragma unroll 1
-          for (int i = lane; i < out.n; i += 32) {
+          for (int i = lane; !LIN && i < out.n; i += 32) {
             const int op = (int)(out.buf[i] & 15u), len = (int)(out.buf[i] >> 4);
             score -= op == WFG_OP_EQ ? P.match_o * len : op == WFG_OP_X ? P.x_o * len : P.o_o + P.e_o * len;
           }
-          score = __reduce_add_sync(kFull, score);
+          if (!LIN) score = __reduce_add_sync(kFull, score);
           unsigned long long base = 0;
           if (lane == 0) base = atomicAdd(P.out_head, (unsigned long long)out.n);
           base = __shfl_sync(kFull, base, 0);
@@ -588,6 +593,8 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
 
 }  // namespace
 
+// LIN: the one-component distances (edit, indel, gap-linear); else gap-affine.
+template <bool LIN>
 __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks) biwfa_tile_kernel(KernelParams Pin) {
   TileBlockSmem& B = tile_smem();
   if (Pin.num_pairs_ptr != nullptr && *Pin.num_pairs_ptr == 0ull) return;  // a retry pass without pairs
@@ -621,8 +628,13 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks) biwfa_tile_kerne
     }
     if (lane == 0) {
       S.arena = A;
-      S.pen = {Pin.x, Pin.o, Pin.e, Pin.scope, Pin.metric, Pin.o, 0,
+      S.pen = {Pin.x, Pin.o, Pin.e, Pin.scope, Pin.metric, LIN ? 0 : Pin.o, 0,
                Pin.tile_g > 1 ? 0xffffffffu / (uint32_t)Pin.tile_g + 1u : 0u};
+      if (LIN) {
+        S.pen.lx = Pin.metric == kMetricIndel ? 0 : Pin.x / Pin.tile_g;
+        S.pen.lo = Pin.o / Pin.tile_g;
+        S.pen.lom = 0xffffffffu / (uint32_t)S.pen.lo + 1u;
+      }
       S.job.ticket = 0ull;
       C.state = gib < owners ? kFetch : kHelp;
       C.first = true;
@@ -634,7 +646,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks) biwfa_tile_kerne
 
   bool control = true;
   for (;;) {
-    if (control && !tile_control(gib, lane, owners)) break;
+    if (control && !tile_control<LIN>(gib, lane, owners)) break;
     control = true;
     if (C.step == 0) continue;  // an own job whose tiles the helpers took
     // ---- the block pass
@@ -657,8 +669,9 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks) biwfa_tile_kerne
       a.old_lo = my.ts.lo; a.old_hi = my.ts.hi;
       a.first = tl == 0; a.last = tl == L - 1;
       a.lane = lane;
-      a.leaf = leaf ? S.dir[2].cfg.ldata + leaf_at(t0 >> 2) : nullptr;
-      a.leaf_lo = leaf_lo(my.cb, t0 >> 2); a.leaf_n = leaf ? leaf_n(t0 >> 2) : 0;
+      if (LIN) { a.lx = S.pen.lx; a.lo = S.pen.lo; }
+      a.leaf = leaf ? S.dir[2].cfg.ldata + leaf_at<LIN>(t0 >> 2) : nullptr;
+      a.leaf_lo = leaf_lo<LIN>(my.cb, t0 >> 2); a.leaf_n = leaf ? leaf_n<LIN>(t0 >> 2) : 0;
       int ak = INT_MIN, tch = 4;
       const int step = C.step;
       int i = C.tile;
@@ -666,11 +679,11 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks) biwfa_tile_kerne
       a.owner = tiles == 1 || !(a.first || a.last);
       #pragma unroll 1
       for (; i < tiles - narrow; i += step)
-        tile_pass<4>(a, sv, i * 120, a.owner || (i == 0 && a.first) || (i == tiles - 1 && a.last), ak, tch);
+        tile_pass<4, LIN>(a, sv, i * 120, a.owner || (i == 0 && a.first) || (i == tiles - 1 && a.last), ak, tch);
       if (i < tiles) {  // the last tile, two diagonals per lane
         a.k = my.ts.base + tl * 2;
         a.owner = tiles == 1 || (tl >= 2 && tl < L - 2);
-        tile_pass<2>(a, sv, i * 120, a.owner || tl >= L - 2 || i == 0, ak, tch);
+        tile_pass<2, LIN>(a, sv, i * 120, a.owner || tl >= L - 2 || i == 0, ak, tch);
       }
       const int other = __shfl_xor_sync(kFull, ak, 16);
       if (halves) {
@@ -709,17 +722,17 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks) biwfa_tile_kerne
       const int nf = max(C.fmax, __reduce_max_sync(kFull, lane < 4 ? part[0] : INT_MIN));
       const int nr = max(C.rmax, __reduce_max_sync(kFull, lane < 4 ? part[1] : INT_MIN));
       if (min(touch[0], touch[1]) == 4 && nf + nr < C.max_antidiag && t0 <= C.guard &&
-          tile_request(0, true, t0 + 4, kSearch, gib, lane)) {
+          tile_request<LIN>(0, true, t0 + 4, kSearch, gib, lane)) {
         C.fmax = nf; C.rmax = nr;
         control = false;
       } else {
         C.state = kSearchEvent;
       }
     } else if (state == kLeaf) {
-      const int end = leaf_at((t0 >> 2) + 1);
+      const int end = leaf_at<LIN>((t0 >> 2) + 1);
       C.leaf_end = end;
       if (touch[0] == 4 && t0 <= C.guard && (t0 + 8) * S.pen.tg <= S.dir[2].cfg.lmax &&
-          leaf_at((t0 >> 2) + 2) <= S.dir[2].lcap && tile_request(0, false, t0 + 4, kLeaf, gib, lane)) {
+          leaf_at<LIN>((t0 >> 2) + 2) <= S.dir[2].lcap && tile_request<LIN>(0, false, t0 + 4, kLeaf, gib, lane)) {
         control = false;
       } else {
         C.state = kLeafEvent;

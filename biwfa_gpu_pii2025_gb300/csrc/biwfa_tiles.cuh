@@ -41,16 +41,28 @@ __device__ __forceinline__ int row_of(int s, const Pen& p) { return p.tg == 1 ? 
 __device__ __forceinline__ bool holds_row(int s, const Pen& p) { return s == row_of(s, p) * p.tg; }
 
 // Diagonals that can hold a non-null cell in row t of a direction that starts in component cb
-// (the rows of all components lie inside; both bounds widen monotonically).
-__device__ __forceinline__ int row_lo(int cb, int t) {
-  return cb == CM ? (t < kTO ? 0 : kTO - 1 - t) : cb == CI ? min(0, kTO + 1 - t) : -t;
-}
-__device__ __forceinline__ int row_hi(int cb, int t) {
+// (the rows of all components lie inside; both bounds widen monotonically). LIN: one component, rows
+// p.lx (mismatch) and p.lo (gap) back, so a row is at most t / p.lo diagonals wide on each side.
+template <bool LIN>
+__device__ __forceinline__ int row_hi(int cb, int t, const Pen& p) {
+  if (LIN) return p.lo == 1 ? t : (int)__umulhi((uint32_t)t, p.lom);
   return cb == CM ? (t < kTO ? 0 : t - kTO + 1) : cb == CI ? t : max(0, t - kTO - 1);
 }
+template <bool LIN>
+__device__ __forceinline__ int row_lo(int cb, int t, const Pen& p) {
+  if (LIN) return -row_hi<true>(cb, t, p);
+  return cb == CM ? (t < kTO ? 0 : kTO - 1 - t) : cb == CI ? min(0, kTO + 1 - t) : -t;
+}
 // Whether component ci (0 M, 1 I, 2 D) of row t exists: some cell of it is not null.
-__device__ __forceinline__ bool row_exists(int cb, int t, int ci) {
+template <bool LIN>
+__device__ __forceinline__ bool row_exists(int cb, int t, int ci, const Pen& p) {
   if (t < 0) return false;
+  if (LIN) {  // sums of lx and lo (each at most 4, without a common factor): all numbers from 6 on
+    if (ci != 0) return false;
+    for (int r = t; t < 6 && p.lo > 1 && r >= 0; r -= p.lo)
+      if (r % p.lx == 0) return true;
+    return t >= 6 || p.lo == 1;
+  }
   if (cb == CM) return ci == 0 ? (t >= kTO || t % kTX == 0) : t >= kTO;
   if (ci == 0) return t >= 1;
   return ci == (cb == CI ? 1 : 2) ? true : t >= kTO + 1;
@@ -88,6 +100,7 @@ struct TileArgs {
   bool first, last;    // this lane is the first or last one of its tile
   bool owner;          // this lane's diagonals are not halo
   int lane;
+  int lx, lo;          // one-component distances: rows back to the mismatch and the gap source (lx 0: none)
 };
 
 // Rows t0+1 .. t0+4 of a tile's diagonals, a.k + off in this lane. Lanes j and 16 + j of ak: the
@@ -96,7 +109,7 @@ struct TileArgs {
 // last four rows' registers rotate by moves): instruction fetch bounds this kernel wherever its code
 // does not loop. 10,000 pairs of 1 kbp / 150,000 mixture pairs with the row loop rolled 3.29 / 169 ms,
 // unrolled by two 3.80 / 177 ms, by four 4.28 / 210 ms.
-template <int C>
+template <int C, bool LIN>
 __device__ __forceinline__ void tile_pass(const TileArgs& a, const SeqView& sv, int off, bool store, int& ak, int& touch) {
   const int k0 = a.k + off;
   const uint32_t idx = (uint32_t)k0 & a.mask;
@@ -105,8 +118,10 @@ __device__ __forceinline__ void tile_pass(const TileArgs& a, const SeqView& sv, 
   if (k0 >= a.old_lo && k0 < a.old_hi) {
     #pragma unroll
     for (int j = 0; j < 4; ++j) tile_load<C>(a.old_rows + j * p3 + idx, m[j]);
-    tile_load<C>(a.old_rows + 3 * p3 + a.pitch + idx, vi);
-    tile_load<C>(a.old_rows + 3 * p3 + 2 * a.pitch + idx, vd);
+    if (!LIN) {
+      tile_load<C>(a.old_rows + 3 * p3 + a.pitch + idx, vi);
+      tile_load<C>(a.old_rows + 3 * p3 + 2 * a.pitch + idx, vd);
+    }
   } else {
     #pragma unroll
     for (int c = 0; c < C; ++c) m[0][c] = m[1][c] = m[2][c] = m[3][c] = vi[c] = vd[c] = kTNull;
@@ -117,19 +132,36 @@ __device__ __forceinline__ void tile_pass(const TileArgs& a, const SeqView& sv, 
   int32_t* leaf = a.leaf + (k0 - a.leaf_lo);
   #pragma unroll 1
   for (int j = 0; j < 4; ++j) {
-    // I = max(M[t-4], I[t-1])[k-1] + 1, D = max(M[t-4], D[t-1])[k+1], M = max(M[t-2] + 1, I, D)
-    int fi[C], fd[C], n[C];
+    int n[C];
     uint32_t x[C];
-    #pragma unroll
-    for (int c = 0; c < C; ++c) { fi[c] = max(m[4 - kTO][c], vi[c]); fd[c] = max(m[4 - kTO][c], vd[c]); }
-    int left = __shfl_up_sync(kFull, fi[C - 1], 1), right = __shfl_down_sync(kFull, fd[0], 1);
-    if (a.first) left = kTNull;
-    if (a.last) right = kTNull;
-    #pragma unroll
-    for (int c = 0; c < C; ++c) {
-      vi[c] = (c == 0 ? left : fi[c > 0 ? c - 1 : 0]) + 1;
-      vd[c] = (c == C - 1 ? right : fd[c < C - 1 ? c + 1 : C - 1]);
-      n[c] = max(m[4 - kTX][c] + 1, max(vi[c], vd[c]));
+    if constexpr (LIN) {
+      // M = max(M[t-lx] + 1, M[t-lo][k-1] + 1, M[t-lo][k+1]), null beyond its diagonal's end
+      int gap[C];
+      #pragma unroll
+      for (int c = 0; c < C; ++c) gap[c] = a.lo == 1 ? m[3][c] : a.lo == 2 ? m[2][c] : a.lo == 3 ? m[1][c] : m[0][c];
+      int left = __shfl_up_sync(kFull, gap[C - 1], 1), right = __shfl_down_sync(kFull, gap[0], 1);
+      if (a.first) left = kTNull;
+      if (a.last) right = kTNull;
+      #pragma unroll
+      for (int c = 0; c < C; ++c) {
+        const int sub = a.lx == 1 ? m[3][c] : a.lx == 2 ? m[2][c] : a.lx == 3 ? m[1][c] : a.lx == 4 ? m[0][c] : kTNull;
+        n[c] = max(max(sub, c == 0 ? left : gap[c > 0 ? c - 1 : 0]) + 1, c == C - 1 ? right : gap[c < C - 1 ? c + 1 : C - 1]);
+        if (n[c] > min(sv.tlen, sv.plen + k0 + c)) n[c] = kTNull;
+      }
+    } else {
+      // I = max(M[t-4], I[t-1])[k-1] + 1, D = max(M[t-4], D[t-1])[k+1], M = max(M[t-2] + 1, I, D)
+      int fi[C], fd[C];
+      #pragma unroll
+      for (int c = 0; c < C; ++c) { fi[c] = max(m[4 - kTO][c], vi[c]); fd[c] = max(m[4 - kTO][c], vd[c]); }
+      int left = __shfl_up_sync(kFull, fi[C - 1], 1), right = __shfl_down_sync(kFull, fd[0], 1);
+      if (a.first) left = kTNull;
+      if (a.last) right = kTNull;
+      #pragma unroll
+      for (int c = 0; c < C; ++c) {
+        vi[c] = (c == 0 ? left : fi[c > 0 ? c - 1 : 0]) + 1;
+        vd[c] = (c == C - 1 ? right : fd[c < C - 1 ? c + 1 : C - 1]);
+        n[c] = max(m[4 - kTX][c] + 1, max(vi[c], vd[c]));
+      }
     }
     // First windows of all cells (a null cell reads the sequences' starts).
     #pragma unroll
@@ -145,7 +177,7 @@ __device__ __forceinline__ void tile_pass(const TileArgs& a, const SeqView& sv, 
       const int rem = min(sv.tlen, sv.plen + k0 + c) - n[c];  // to the end of diagonal k0 + c
       const int e = min(x[c] ? (first_set(x[c]) >> sv.bshift) : cpw, rem);
       full |= x[c] == 0;
-      ends |= e >= rem;
+      ends |= e >= rem && (!LIN || k0 + c == sv.tlen - sv.plen);
       n[c] += e;
     }
     // Matches longer than one window (a null cell has none).
@@ -172,7 +204,7 @@ __device__ __forceinline__ void tile_pass(const TileArgs& a, const SeqView& sv, 
         cur += cpw;
       }
       cur = min(cur, end);
-      ends |= cur >= end;
+      ends |= cur >= end && (!LIN || k0 + c == sv.tlen - sv.plen);
       #pragma unroll
       for (int i = 0; i < C; ++i) if (c == i) n[i] = cur;
     }
@@ -188,23 +220,26 @@ __device__ __forceinline__ void tile_pass(const TileArgs& a, const SeqView& sv, 
     for (int c = 0; c < C; ++c) { m[0][c] = m[1][c]; m[1][c] = m[2][c]; m[2][c] = m[3][c]; m[3][c] = n[c]; }
     if (store) {
       tile_store<C>(ring, n);
-      if (a.leaf_n == 0 || j == 3) { tile_store<C>(ring + a.pitch, vi); tile_store<C>(ring + 2 * a.pitch, vd); }
+      if (!LIN && (a.leaf_n == 0 || j == 3)) { tile_store<C>(ring + a.pitch, vi); tile_store<C>(ring + 2 * a.pitch, vd); }
     }
     ring += p3;
     if (leafw) {
       tile_store<C>(leaf, n);
-      tile_store<C>(leaf + a.leaf_n, vi);
-      tile_store<C>(leaf + 2 * a.leaf_n, vd);
+      if (!LIN) {
+        tile_store<C>(leaf + a.leaf_n, vi);
+        tile_store<C>(leaf + 2 * a.leaf_n, vd);
+      }
     }
-    leaf += 3 * a.leaf_n;
+    leaf += (LIN ? 1 : 3) * a.leaf_n;
   }
 }
 
 // The tiling of block t0 for L lanes into d.ts: tiles, first diagonal, end of the last tile. One tile
 // of 4 L diagonals if they hold all of the rows' cells (the cells beside it are null), else tiles with
 // halos. narrow: the last tile has two diagonals per lane. False when the ring does not hold them.
-__device__ __forceinline__ bool tile_plan(Dir& d, int t0, int L) {
-  const int lo = row_lo(d.cb, t0 + 4) & ~3, width = row_hi(d.cb, t0 + 4) - lo + 1;
+template <bool LIN>
+__device__ __forceinline__ bool tile_plan(Dir& d, int t0, int L, const Pen& pen) {
+  const int hi = row_hi<LIN>(d.cb, t0 + 4, pen), lo = row_lo<LIN>(d.cb, t0 + 4, pen) & ~3, width = hi - lo + 1;
   int tiles = 1, base = lo;
   bool narrow = width <= 2 * L;
   if (width > 4 * L) {
@@ -214,13 +249,19 @@ __device__ __forceinline__ bool tile_plan(Dir& d, int t0, int L) {
   }
   const int end = base + (tiles - 1) * 120 + (narrow ? 2 : 4) * L;
   d.ts.tiles = tiles; d.ts.base = base; d.ts.end = end; d.ts.narrow = narrow;
+  // WFA2-lib prunes edit wavefronts of 1,000 diagonals and more: the one-step function's part
+  if (LIN && pen.metric == kMetricEdit && 2 * hi + 1 >= 1000) return false;
   return end - base <= d.cfg.W;
 }
 // Whether half a warp holds block t0's rows.
-__device__ __forceinline__ bool tile_half(int cb, int t0) { return row_hi(cb, t0 + 4) - (row_lo(cb, t0 + 4) & ~3) < 64; }
+template <bool LIN>
+__device__ __forceinline__ bool tile_half(int cb, int t0, const Pen& p) {
+  return row_hi<LIN>(cb, t0 + 4, p) - (row_lo<LIN>(cb, t0 + 4, p) & ~3) < 64;
+}
 
 // Starts a direction over window sv in component cb: row 0 with its extension. Returns its offset,
 // or -1 when it touches (then nothing is started).
+template <bool LIN>
 __device__ __noinline__ int tile_start(Dir& d, const SeqView& sv, int cb, int ce, int lane) {
   const int n = min(sv.plen, sv.tlen);
   int off0 = 0;
@@ -232,7 +273,10 @@ __device__ __noinline__ int tile_start(Dir& d, const SeqView& sv, int cb, int ce
       if (x) { off0 += first_set(x) >> sv.bshift; break; }
     }
   }
-  if (off0 >= n) return -1;
+  if (off0 >= n) {
+    if (!LIN || sv.plen == sv.tlen) return -1;
+    off0 = n;  // one component: an end that is not the window's corner is an ordinary cell
+  }
   d.sv = sv; d.cb = cb; d.ce = ce;
   d.num_null = 0; d.status = ST_OK; d.status_score = 0; d.end_k = INT_MAX;
   d.ts.on = 1; d.ts.t = 0; d.ts.valid = 0; d.ts.touched = 0;
@@ -250,16 +294,17 @@ __device__ __noinline__ int tile_start(Dir& d, const SeqView& sv, int cb, int ce
 }
 
 // Descriptors of the scores from .. s from their rows (a score without a row is absent).
+template <bool LIN>
 __device__ __noinline__ void tile_describe(Dir& d, int s, int from, const Pen& p) {
   const DirCfg c = d.cfg;
   #pragma unroll 1
   for (int q = max(from, 0); q <= s; ++q) {
     const int slot = slot_of(c, q), t = row_of(q, p);
     const bool row = holds_row(q, p);
-    const int lo = row_lo(d.cb, t), hi = row_hi(d.cb, t);
+    const int lo = row_lo<LIN>(d.cb, t, p), hi = row_hi<LIN>(d.cb, t, p);
     #pragma unroll 1
     for (int ci = 0; ci < 3; ++ci)
-      c.rdesc[slot * 3 + ci] = row && row_exists(d.cb, t, ci) ? make_int2(lo, hi) : make_int2(kAbsent, INT_MIN);
+      c.rdesc[slot * 3 + ci] = row && row_exists<LIN>(d.cb, t, ci, p) ? make_int2(lo, hi) : make_int2(kAbsent, INT_MIN);
     c.rphys[slot] = row_buffer(t);
   }
   __syncwarp();
@@ -267,13 +312,14 @@ __device__ __noinline__ void tile_describe(Dir& d, int s, int from, const Pen& p
 
 // Step of a direction to score s with its descriptors: from the rows computed ahead or, when these
 // end, by dir_step. Returns as dir_step.
+template <bool LIN>
 __device__ __noinline__ int tile_advance(Dir& d, const Pen& p, int s, const Grp<1> g, int* max_ak_out) {
   *max_ak_out = 0;
   if (d.ts.on) {
     const bool row = holds_row(s, p);
     const int t = row_of(s, p);
     if (!row || t <= d.ts.valid) {
-      tile_describe(d, s, s, p);
+      tile_describe<LIN>(d, s, s, p);
       if (!row) return 0;
       if (d.ts.touched && t == d.ts.valid) {
         const int ak = d.sv.tlen - d.sv.plen;
@@ -289,7 +335,7 @@ __device__ __noinline__ int tile_advance(Dir& d, const Pen& p, int s, const Grp<
     }
     // The one-step functions take over at this row.
     int nn = 0;
-    for (int q = s - 1; q > 0 && !(holds_row(q, p) && row_exists(d.cb, row_of(q, p), 0)); --q) ++nn;
+    for (int q = s - 1; q > 0 && !(holds_row(q, p) && row_exists<LIN>(d.cb, row_of(q, p), 0, p)); --q) ++nn;
     __syncwarp();
     d.ts.on = 0;
     d.num_null = nn;
@@ -300,13 +346,23 @@ __device__ __noinline__ int tile_advance(Dir& d, const Pen& p, int s, const Grp<
 }
 
 // The leaf store of a leaf whose rows come in tiles: row 0's one cell at 0, then block b's four rows
-// (M, I, D each) of leaf_n(b) diagonals from leaf_lo(cb, b) at leaf_at(b), all multiples of 4 that
-// cover row_lo .. row_hi. So a row's place follows from its number, without a descriptor.
-__device__ __forceinline__ int leaf_n(int b) { return 8 * b + 8; }
-__device__ __forceinline__ int leaf_lo(int cb, int b) { return cb == CI ? -4 * b : -4 * b - 4; }
-__device__ __forceinline__ int leaf_at(int b) { return 4 + 48 * b * (b + 1); }
+// (M, I, D each, or M alone) of leaf_n(b) diagonals from leaf_lo(cb, b) at leaf_at(b), all multiples
+// of 4 that cover row_lo .. row_hi. So a row's place follows from its number, without a descriptor.
+template <bool LIN>
+__device__ __forceinline__ int leaf_n(int b) { return 8 * b + (LIN ? 12 : 8); }
+template <bool LIN>
+__device__ __forceinline__ int leaf_lo(int cb, int b) { return !LIN && cb == CI ? -4 * b : -4 * b - 4; }
+template <bool LIN>
+__device__ __forceinline__ int leaf_at(int b) { return LIN ? 4 + 16 * b * (b + 2) : 4 + 48 * b * (b + 1); }
+// Row t's component ci on diagonal k (t >= 1).
+template <bool LIN>
+__device__ __forceinline__ int leaf_cell(int cb, int t, int ci, int k) {
+  const int b = (t - 1) >> 2, j = (t - 1) & 3;
+  return leaf_at<LIN>(b) + (LIN ? j : j * 3 + ci) * leaf_n<LIN>(b) + k - leaf_lo<LIN>(cb, b);
+}
 
 // Leaf descriptors of the scores from .. s, for the one-step functions.
+template <bool LIN>
 __device__ __noinline__ void leaf_describe(Dir& d, int s, int from, const Pen& p, int lane) {
   const int q = max(from, 0) + lane;
   if (q <= s) {
@@ -314,26 +370,28 @@ __device__ __noinline__ void leaf_describe(Dir& d, int s, int from, const Pen& p
     #pragma unroll 1
     for (int ci = 0; ci < 3; ++ci) {
       int4 ds = make_int4(kAbsent, INT_MIN, 0, 0);
-      if (holds_row(q, p) && row_exists(d.cb, t, ci))
+      if (holds_row(q, p) && row_exists<LIN>(d.cb, t, ci, p))
         ds = t == 0 ? make_int4(0, 0, 0, 0)
-                    : make_int4(row_lo(d.cb, t), row_hi(d.cb, t), leaf_at(b) + (((t - 1) & 3) * 3 + ci) * leaf_n(b),
-                                leaf_lo(d.cb, b));
+                    : make_int4(row_lo<LIN>(d.cb, t, p), row_hi<LIN>(d.cb, t, p),
+                                leaf_cell<LIN>(d.cb, t, ci, leaf_lo<LIN>(d.cb, b)), leaf_lo<LIN>(d.cb, b));
       d.cfg.ldesc[q * 3 + ci] = ds;
     }
   }
   __syncwarp();
 }
 
-// leaf_backtrace for gap-affine over a leaf whose rows up to score `fast` came in tiles (later ones
+// leaf_backtrace over a leaf whose rows up to score `fast` came in tiles (later ones
 // have descriptors): a lane per source (0 mismatch, 1-2 I open/extend, 3-4 D open/extend), one
 // offset latency a step, and the packed maximum picks the source.
+template <bool LIN>
 __device__ __noinline__ int tile_backtrace(const Dir& B, const Pen& p, int s, int fast, RunOut& out, uint32_t* lruns,
                                            int lruns_cap, int lane) {
   const int cb = B.cb;
   const int32_t* ldata = B.cfg.ldata;
   const int plen = B.sv.plen, tlen = B.sv.tlen;
   const bool ext = lane == 2 || lane == 4, del = lane >= 3;
-  const int back = lane == 0 ? p.x : ext ? p.e : p.o + p.e;
+  const int open = LIN ? p.o : p.o + p.e, back = lane == 0 ? p.x : ext ? p.e : open;
+  const bool usable = LIN ? (lane == 0 ? p.metric != kMetricIndel : lane == 1 || lane == 3) : lane < 5;
   const int my_ci = ext ? (del ? 2 : 1) : 0, my_dk = lane == 0 ? 0 : del ? 1 : -1, my_add = del ? 0 : 1;
   const int my_type = lane == 0 ? BT_M : del ? (ext ? BT_D_EXT : BT_D_OPEN) : (ext ? BT_I_EXT : BT_I_OPEN);
   int ci = comp_index(B.ce), score = s, k = B.end_k, off = tlen, nrev = 0, rop = -1, rlen = 0;
@@ -351,15 +409,14 @@ __device__ __noinline__ int tile_backtrace(const Dir& B, const Pen& p, int s, in
       if (walk) {
         if (--left < 0) return WFG_ST_UNATTAINABLE;
         const int sc = score - back, kk = k + my_dk;
-        if (lane < 5 && sc >= 0 && (ci == 0 || (lane > 0 && del == (ci == 2)))) {
+        if (usable && sc >= 0 && (ci == 0 || (lane > 0 && del == (ci == 2)))) {
           int o = kTNull;
           if (sc > fast) {
             o = ref_raw<1>(B.cfg, sc, my_ci).get(kk);
           } else {
-            const int t = row_of(sc, p), b = (t - 1) >> 2;
-            int at = leaf_at(b) + (((t - 1) & 3) * 3 + my_ci) * leaf_n(b) + kk - leaf_lo(cb, b);
-            if (t == 0) at = my_ci == comp_index(cb) ? 0 : -1;
-            if (sc == t * p.tg && row_lo(cb, t) <= kk && kk <= row_hi(cb, t) && at >= 0) o = ldata[at];
+            const int t = row_of(sc, p);
+            const int at = t == 0 ? (my_ci == comp_index(cb) ? 0 : -1) : leaf_cell<LIN>(cb, t, my_ci, kk);
+            if (sc == t * p.tg && row_lo<LIN>(cb, t, p) <= kk && kk <= row_hi<LIN>(cb, t, p) && at >= 0) o = ldata[at];
           }
           if (o >= 0) mine = (o + my_add) * 16 + my_type;
         }
@@ -373,7 +430,7 @@ __device__ __noinline__ int tile_backtrace(const Dir& B, const Pen& p, int s, in
         if (walk) {
           const int type = best & 15;
           const bool e = type == BT_I_EXT || type == BT_D_EXT, d = type == BT_D_EXT || type == BT_D_OPEN;
-          score -= type == BT_M ? p.x : e ? p.e : p.o + p.e;
+          score -= type == BT_M ? p.x : e ? p.e : open;
           ci = e ? (d ? 2 : 1) : 0;
           op = type == BT_M ? WFG_OP_X : d ? WFG_OP_DEL : WFG_OP_INS;
           if (type != BT_M) k += d ? 1 : -1;
@@ -412,10 +469,11 @@ __device__ __noinline__ int tile_backtrace(const Dir& B, const Pen& p, int s, in
 // lanes first test the rows' largest ones, a row pair each, and only pairs that pass are scanned.
 // An untouched row's I and D offsets are at most M's on the same diagonal, so a scan reads M and
 // looks at D and I only where M meets. D comes first, then I, then M, the lowest diagonal of each.
+template <bool LIN>
 __device__ __noinline__ void tile_overlap(const Dir& d0, const Dir& d1, int s0, int s1, bool fwd, BP& bp, const Pen& p,
                                           int lane) {
   const int t0 = row_of(s0, p), cb0 = d0.cb, cb1 = d1.cb;
-  if (!row_exists(cb0, t0, 0)) return;
+  if (!row_exists<LIN>(cb0, t0, 0, p)) return;
   const int plen = d0.sv.plen, tlen = d0.sv.tlen, A = tlen - plen;
   const int mine = s1 - lane;
   unsigned todo = __ballot_sync(kFull, lane < p.scope && mine >= 0 && holds_row(mine, p) &&
@@ -430,10 +488,10 @@ __device__ __noinline__ void tile_overlap(const Dir& d0, const Dir& d1, int s0, 
     if (s0 + s - p.go >= bp.score) continue;
     const int t1 = row_of(s, p);
     const int32_t* r1 = d1.cfg.rdata + row_buffer(t1) * 3 * pitch;
-    const int end = min(row_hi(cb0, t0), A - row_lo(cb1, t1));
+    const int end = min(row_hi<LIN>(cb0, t0, p), A - row_lo<LIN>(cb1, t1, p));
     int first[3] = {INT_MAX, INT_MAX, INT_MAX};  // lowest diagonal where M, I, D meet
     #pragma unroll 1
-    for (int kb = max(row_lo(cb0, t0), A - row_hi(cb1, t1)) + lane; kb - lane <= end; kb += 128) {
+    for (int kb = max(row_lo<LIN>(cb0, t0, p), A - row_hi<LIN>(cb1, t1, p)) + lane; kb - lane <= end; kb += 128) {
       // four diagonals per lane, their loads in flight together
       int sum[4];
       sum[0] = kb <= end ? r0[(uint32_t)kb & mask] + r1[(uint32_t)(A - kb) & mask] : -1;
@@ -450,8 +508,8 @@ __device__ __noinline__ void tile_overlap(const Dir& d0, const Dir& d1, int s0, 
         if (sum[0] >= tlen) {
           const uint32_t i0 = (uint32_t)k & mask, i1 = (uint32_t)(A - k) & mask;
           first[0] = min(first[0], k);
-          if (r0[pitch + i0] + r1[pitch + i1] >= tlen) first[1] = min(first[1], k);
-          if (r0[2 * pitch + i0] + r1[2 * pitch + i1] >= tlen) first[2] = min(first[2], k);
+          if (!LIN && r0[pitch + i0] + r1[pitch + i1] >= tlen) first[1] = min(first[1], k);
+          if (!LIN && r0[2 * pitch + i0] + r1[2 * pitch + i1] >= tlen) first[2] = min(first[2], k);
         }
         sum[0] = sum[1]; sum[1] = sum[2]; sum[2] = sum[3]; sum[3] = -1;
       }

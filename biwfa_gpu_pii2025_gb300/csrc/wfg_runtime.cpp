@@ -203,6 +203,7 @@ namespace {
 struct IntPen {
   int x, o, e, scope, nphys;
   int o2 = 0, e2 = 0, nc = 3, emin = 1, g = 1;
+  int metric = WFG_METRIC_GAP_AFFINE;
   int tile_g = 0;  // rows in tiles (biwfa_tiles.cuh): score spacing, 0 for one score at a time
 };
 IntPen internal_penalties(const wfg_config_t* cfg) {
@@ -331,7 +332,7 @@ void size_launch(const wfg_context* c, const IntPen& p, int pass, int ring_w_hin
 int64_t max_groups(const wfg_context* c, const IntPen& p, const Launch& l) {
   const size_t dyn = l.smem ? (size_t)2 * p.nphys * p.nc * (size_t)l.ring_w * sizeof(int32_t) : 0;
   // The device's answer for a shape does not change, so a context asks once.
-  const int kind = biwfa_kernel_kind(p.nc == 5 ? 4 : 0, p.scope, l.smem ? 0 : p.tile_g);
+  const int kind = biwfa_kernel_kind(p.metric, p.scope, l.smem ? 0 : p.tile_g);
   int bps = 0;
   for (const wfg_context::Occupancy& o : c->occupancy)
     if (o.kind == kind && o.gw == l.gw && o.smem == l.smem && o.dyn == dyn) bps = o.blocks;
@@ -459,6 +460,7 @@ int validate_config(wfg_context* c, const wfg_config_t* cfg, IntPen* p) {
     return WF_STATUS_UNSUPPORTED;
   }
   *p = internal_penalties(cfg);
+  p->metric = cfg->metric;
   if (p->scope > WFG_MAX_SCOPE_2P) {
     c->err = "max_score_scope above 64 is not supported";
     return WF_STATUS_UNSUPPORTED;
@@ -470,6 +472,16 @@ int validate_config(wfg_context* c, const wfg_config_t* cfg, IntPen* p) {
   if (cfg->metric == WFG_METRIC_GAP_AFFINE && p->x == 2 * p->e && p->o == 3 * p->e && p->scope <= WFG_MAX_SCOPE &&
       (cfg->max_alignment_steps <= 0 || cfg->max_alignment_steps >= (1 << 28)))
     p->tile_g = p->e;
+  // And the one-component distances whose mismatch and gap lie at most four rows back: 20,000 uneven
+  // pairs of edit distance 18.7 ms end to end one score at a time, 9.1 ms in tiles; 5,000 of 5 kbp at
+  // 3-8 %: edit 12.4 and 7.2 ms, indel 17.4 and 10.0, gap-linear 4/2 24.9 and 11.0. Batches whose
+  // longest pair has 128 bp a side keep single scores for edit and indel (20,000 pairs of 100 bp: 0.51
+  // and 0.56 ms; of 200 bp 1.18 and 1.11).
+  const bool edits = cfg->metric == WFG_METRIC_EDIT || cfg->metric == WFG_METRIC_INDEL;
+  if (((edits && c->max_sum > kEditTilesMinSum) ||
+       (cfg->metric == WFG_METRIC_GAP_LINEAR && p->x <= 4 * p->g && p->o <= 4 * p->g && p->scope <= WFG_MAX_SCOPE)) &&
+      (cfg->max_alignment_steps <= 0 || cfg->max_alignment_steps >= (1 << 28)))
+    p->tile_g = p->g;
   if ((int64_t)(c->max_sum + 16) * (int64_t)std::max(p->x, std::max(p->o + p->e, p->o2 + p->e2)) >= ((int64_t)1 << 26)) {
     c->err = "pair too long for 27-bit scores";
     return WF_STATUS_UNSUPPORTED;

@@ -57,3 +57,32 @@ def test_tiles_match_oracle(batch_aligner, pen, gw, seed):
         assert res.scores[i] == (score if ops else 0), i
         st, score, _, _ = binding.oracle_align(b.pattern(i), b.text(i), pen, score_only=True)
         assert only.status[i] == st and (st != 0 or only.scores[i] == score), i
+
+
+@pytest.mark.parametrize("metric,pen,gw,seed", [
+    (binding.METRIC_EDIT, (0, 1, 0, 0), 1, 11), (binding.METRIC_EDIT, (0, 1, 0, 0), 8, 12),
+    (binding.METRIC_INDEL, (0, 1, 0, 0), 1, 13), (binding.METRIC_LINEAR, (0, 4, 2, 0), 1, 14),
+    (binding.METRIC_LINEAR, (0, 4, 6, 0), 4, 15), (binding.METRIC_LINEAR, (0, 9, 12, 0), 1, 16),
+    (binding.METRIC_LINEAR, (0, 1, 4, 0), 1, 17)])
+def test_one_component_tiles_match_oracle(batch_aligner, metric, pen, gw, seed):
+    """One component: rows go on past touched ends, up to edit's wavefronts of 1,000 diagonals."""
+    b = _batch(seed)
+    if metric == binding.METRIC_EDIT:
+        rng = np.random.default_rng(seed)
+        far = [(bytes(rng.choice(list(b"ACGT"), n).astype(np.uint8)), bytes(rng.choice(list(b"ACGT"), m).astype(np.uint8)))
+               for n, m in ((2500, 2500), (3000, 700))]
+        b = pkg.PairBatch.from_lists([b.pattern(i) for i in range(b.n)] + [p for p, _ in far],
+                                     [b.text(i) for i in range(b.n)] + [t for _, t in far])
+    try:
+        batch_aligner.set_exec_shape(gw, False)
+        res = batch_aligner.align(b, penalties=pen, metric=metric)
+        only = batch_aligner.align(b, penalties=pen, metric=metric, score_only=True)
+    finally:
+        batch_aligner.set_exec_shape(1, False)
+    assert (res.status == 0).all()
+    for i in range(b.n):
+        _, score, ops, _ = binding.oracle_align(b.pattern(i), b.text(i), pen, metric=metric)
+        assert pkg.runs_to_ops(res.runs_of(i)) == ops, (i, b.plen[i], b.tlen[i])
+        assert res.scores[i] == (score if ops else 0), i
+        st, score, _, _ = binding.oracle_align(b.pattern(i), b.text(i), pen, True, metric=metric)
+        assert only.status[i] == st and (st != 0 or only.scores[i] == score), i
