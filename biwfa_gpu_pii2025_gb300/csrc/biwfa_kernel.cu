@@ -299,6 +299,7 @@ struct TileState {
   int touched;       // row `valid` touched an end: dir_step continues after it
   int lo, hi;        // diagonals [lo, hi) that the last block wrote, in each of its rows
   int base, end, tiles, narrow;  // tiling of the next block (tile_plan)
+  int gaps;          // its I and D rows are all stored (else the last ones)
   int akr[kTileBufs];  // largest antidiagonal of each stored row's M
 };
 struct Dir {

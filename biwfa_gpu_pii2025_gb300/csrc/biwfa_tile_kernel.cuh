@@ -66,11 +66,11 @@ struct TileCtl {
   int part[10];                 // results of the block, as TileJob's
   // pair
   bool first;
-  int pi, status, score, sp, max_leaf, max_depth;
+  int pi, status, score, sp;
   PairSeqs q;
   RunOut out;
   // window
-  int pb, pe, tb, te, cb, ce, lvl, rem;
+  int pb, pe, tb, te, cb, ce, rem;
   // search
   int guard, max_antidiag, fmax, rmax, sf, sr;
   bool last_fwd;
@@ -190,12 +190,26 @@ __device__ __noinline__ bool tile_request(int d, bool both, int t0, int state, i
     S.dir[1].ts.end = S.dir[1].ts.base + 64;
   }
   C.owner = gib; C.d = d; C.t0 = t0; C.tile = 0; C.step = 1;
+  if (!LIN) {  // which rows' I and D go to the ring (TileArgs::gaps)
+    S.dir[d].ts.gaps = state == kMeet || (state == kSearch && S.dir[d].ts.tiles <= kGapTiles);
+    if (both) S.dir[1].ts.gaps = S.dir[1].ts.tiles <= kGapTiles;
+  }
   C.state = state;
   C.mode = halves ? kHalves : both ? kBoth : kOne;
   __syncwarp();
   if (!halves && state != kLeaf && *(volatile int*)&B.idle > 0 && S.dir[d].ts.tiles + (both ? S.dir[1].ts.tiles : 0) > 1)
     job_open(d, both, t0, state, gib, lane);
   return true;
+}
+
+// I and D of the last two blocks of both directions of a search, where their passes did not store them.
+__device__ __noinline__ void search_gaps(int gib, int lane) {
+  TileGroup& S = tile_smem().grp[gib];
+  #pragma unroll 1
+  for (int i = 0; i < 4; ++i) {
+    const int t0 = S.ctl.t0 - (i < 2 ? 4 : 0);
+    if (t0 >= 0 && tile_wide(S.dir[i & 1].cb, t0, S.pen)) tile_gaps(S.dir[i & 1], t0, S.pen, lane);
+  }
 }
 
 // Runs the warp's state machine to its next block pass (S.ctl says which); false when the launch has
@@ -295,9 +309,9 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
       F.cfg.rdata = A.ring;
       R.cfg.rdata = A.ring + (size_t)P.ring_nphys * 3 * (wp + WFG_TILE_PAD);
       S.pen.tg = wp >= kTileMinRing ? P.tile_g : 0;
-      C.status = ST_OK; C.score = 0; C.max_leaf = -1; C.max_depth = 0;
+      C.status = ST_OK; C.score = 0;
       out.buf = A.runs; out.n = 0; out.cap = P.run_cap; out.cur_op = -1; out.cur_len = 0; out.overflow = false;
-      C.pb = 0; C.pe = pd.plen; C.tb = 0; C.te = pd.tlen; C.cb = CM; C.ce = CM; C.lvl = 0;
+      C.pb = 0; C.pe = pd.plen; C.tb = 0; C.te = pd.tlen; C.cb = CM; C.ce = CM;
       C.rem = max(pd.plen, pd.tlen) <= kFallbackMinLength ? 0 : INT_MAX;  // short pairs take the leaf
       C.sp = 0;
       __syncwarp();
@@ -320,8 +334,7 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
           __syncwarp();
           C.sp = sp;
           C.pb = a.x; C.pe = a.y; C.tb = a.z; C.te = a.w;
-          C.cb = b.x; C.ce = b.y; C.rem = b.z; C.lvl = b.w;
-          C.max_depth = max(C.max_depth, b.w);
+          C.cb = b.x; C.ce = b.y; C.rem = b.z;
         } else {
           C.sp = 0;
         }
@@ -363,6 +376,7 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
     if (state == kSearchEvent) {
       // Replay of the block's rows up to the event; a touched row, or a full ring, leaves to the
       // single steps after the last row before it.
+      if (!LIN && C.t0 >= kGapFirst) search_gaps(gib, lane);
       int t = C.t0, fmax = C.fmax, rmax = C.rmax, sf = 0, sr = 0;
       const int ft = C.part[4], rt = C.part[9];
       bool steps = true, last_fwd = false;
@@ -447,9 +461,9 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
         } else {
           int4* e = reinterpret_cast<int4*>(S.arena.stack + sp * 8);
           e[0] = make_int4(C.pb + bv, C.pe, C.tb + bh, C.te);
-          e[1] = make_int4(bp.comp, C.ce, bp.sr, C.lvl + 1);
+          e[1] = make_int4(bp.comp, C.ce, bp.sr, 0);
           e[2] = make_int4(C.pb, C.pb + bv, C.tb, C.tb + bh);
-          e[3] = make_int4(C.cb, bp.comp, bp.sf, C.lvl + 1);
+          e[3] = make_int4(C.cb, bp.comp, bp.sf, 0);
           __syncwarp();
           C.sp = sp + 2;
         }
@@ -474,7 +488,7 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
       const int off0 = pen.tg ? tile_start<LIN>(F, sv, C.cb, C.ce, lane) : -1;
       if (off0 < 0) {
         st = leaf_align<1, false>(L, C.q, C.pb, C.pe, C.tb, C.te, C.cb, C.ce, pen, P.max_steps, out,
-                                  S.arena.lruns, P.leaf_run_cap, g, &C.max_leaf);
+                                  S.arena.lruns, P.leaf_run_cap, g, &s);
         __syncwarp();
         if (st != ST_OK) C.status = st;
         __syncwarp();
@@ -518,7 +532,6 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
       }
       if (st == ST_OK) st = tile_backtrace<LIN>(L, pen, s, fast, out, S.arena.lruns, P.leaf_run_cap, lane);
       __syncwarp();
-      C.max_leaf = max(C.max_leaf, s);
       if (st != ST_OK) C.status = st;
       __syncwarp();
       done = false;
@@ -563,12 +576,6 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
         P.scores[pi] = score;
         P.status[pi] = status;
         if (status != WFG_ST_COMPLETED || P.score_only) { P.run_off[pi] = 0; P.run_len[pi] = 0; }
-        if (P.stats) {
-          P.stats[pi * 4 + 0] = 0;
-          P.stats[pi * 4 + 1] = C.max_leaf;
-          P.stats[pi * 4 + 2] = C.max_depth;
-          P.stats[pi * 4 + 3] = 0;
-        }
       }
       __syncwarp();
       state = kFetch;
@@ -669,6 +676,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks) biwfa_tile_kerne
       a.old_lo = my.ts.lo; a.old_hi = my.ts.hi;
       a.first = tl == 0; a.last = tl == L - 1;
       a.lane = lane;
+      a.gaps = my.ts.gaps;
       if (LIN) { a.lx = S.pen.lx; a.lo = S.pen.lo; }
       a.leaf = leaf ? S.dir[2].cfg.ldata + leaf_at<LIN>(t0 >> 2) : nullptr;
       a.leaf_lo = leaf_lo<LIN>(my.cb, t0 >> 2); a.leaf_n = leaf ? leaf_n<LIN>(t0 >> 2) : 0;

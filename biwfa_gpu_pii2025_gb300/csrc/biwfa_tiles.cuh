@@ -20,8 +20,8 @@
 // (shuffles, then the sequence windows). One score at a time cost about 264 lane instructions per
 // diagonal and row, 40 % of them paid per step; a tile costs about 60. End to end on a GB300, one
 // score at a time -> tiles (and the kernel of biwfa_tile_kernel.cuh): 10,000 pairs of 1 kbp at 5 %
-// 7.7 -> 3.4 ms, 20,000 uneven pairs (100 bp - 10 kbp, 1-10 %) 320 -> 73 ms, 48 pairs of 10-20 kbp
-// at 12 % 569 -> 124 ms, 200,000 pairs of 150 bp at 2 % 15.3 -> 12.5 ms.
+// 7.7 -> 3.2 ms, 20,000 uneven pairs (100 bp - 10 kbp, 1-10 %) 320 -> 64 ms, 48 pairs of 10-20 kbp
+// at 12 % 560 -> 123 ms, 200,000 pairs of 150 bp at 2 % 15.4 -> 12.3 ms.
 //
 // Where the values are exact. WFA2-lib trims each row to its in-bounds cells and keeps
 // out-of-bounds I/D cells between them. Out-of-bounds cells arise only from a cell whose offset
@@ -99,6 +99,7 @@ struct TileArgs {
   int k;               // this lane's first diagonal in the first tile
   bool first, last;    // this lane is the first or last one of its tile
   bool owner;          // this lane's diagonals are not halo
+  bool gaps;           // I and D go to the ring for every row (else for the last one)
   int lane;
   int lx, lo;          // one-component distances: rows back to the mismatch and the gap source (lx 0: none)
 };
@@ -220,7 +221,7 @@ __device__ __forceinline__ void tile_pass(const TileArgs& a, const SeqView& sv, 
     for (int c = 0; c < C; ++c) { m[0][c] = m[1][c]; m[1][c] = m[2][c]; m[2][c] = m[3][c]; m[3][c] = n[c]; }
     if (store) {
       tile_store<C>(ring, n);
-      if (!LIN && (a.leaf_n == 0 || j == 3)) { tile_store<C>(ring + a.pitch, vi); tile_store<C>(ring + 2 * a.pitch, vd); }
+      if (!LIN && (a.gaps || j == 3)) { tile_store<C>(ring + a.pitch, vi); tile_store<C>(ring + 2 * a.pitch, vd); }
     }
     ring += p3;
     if (leafw) {
@@ -291,6 +292,56 @@ __device__ __noinline__ int tile_start(Dir& d, const SeqView& sv, int cb, int ce
   }
   __syncwarp();
   return off0;
+}
+
+// Whether block t0 has more than kGapTiles tiles: below that its rows fit the caches anyway. The
+// diagonals grow by at most two per row, so no block before kGapFirst has.
+constexpr int kGapTiles = 3, kGapFirst = (kGapTiles * 120) / 2 - 12;
+__device__ __forceinline__ bool tile_wide(int cb, int t0, const Pen& p) {
+  return row_hi<false>(cb, t0 + 4, p) - (row_lo<false>(cb, t0 + 4, p) & ~3) + 1 > kGapTiles * 120;
+}
+// I and D of rows t0+1 .. t0+3 of a wide block, which its pass did not store: most blocks of a search
+// are read again only as the next block's last row, and the rows' footprint and traffic in L2 and
+// HBM are half with that alone. The last two blocks before the second phase get them here, from M
+// (nothing is extended again). All rows stored -> this, on one GB300: 150,000 mixture pairs 160-164 ->
+// 152-154 ms (L2 hits 37 % of the rows' sectors before), 20,000 uneven pairs 68.6 -> 64.2 ms, scores only
+// of 10,000 pairs of 200 bp - 5 kbp 6.25 -> 5.90 ms; 1 kbp pairs, never as wide, are equal.
+__device__ __noinline__ void tile_gaps(const Dir& d, int t0, const Pen& p, int lane) {
+  const int lo = row_lo<false>(d.cb, t0 + 4, p) & ~3, hi = row_hi<false>(d.cb, t0 + 4, p);
+  const int old_lo = row_lo<false>(d.cb, t0, p) & ~3, old_hi = (row_hi<false>(d.cb, t0, p) + 4) & ~3;
+  const int b = (t0 >> 2) % 3, pitch = d.cfg.pitch;
+  const int32_t* old_rows = d.cfg.rdata + (b == 0 ? 2 : b - 1) * 12 * pitch;
+  int32_t* new_rows = d.cfg.rdata + b * 12 * pitch;
+  #pragma unroll 1
+  for (int base = lo - 4; base < hi; base += 120) {  // a halo of four diagonals per side
+    const int k = base + lane * 4;
+    const uint32_t idx = (uint32_t)k & ((uint32_t)d.cfg.W - 1u);
+    int vi[4], vd[4], m[4];
+    #pragma unroll
+    for (int c = 0; c < 4; ++c) vi[c] = vd[c] = m[c] = kTNull;
+    const bool in = k >= old_lo && k < old_hi;
+    if (in) {
+      tile_load<4>(old_rows + 10 * pitch + idx, vi);
+      tile_load<4>(old_rows + 11 * pitch + idx, vd);
+    }
+    #pragma unroll 1
+    for (int j = 0; j < 3; ++j) {
+      if (in) tile_load<4>(old_rows + j * 3 * pitch + idx, m);
+      int fi[4], fd[4];
+      #pragma unroll
+      for (int c = 0; c < 4; ++c) { fi[c] = max(m[c], vi[c]); fd[c] = max(m[c], vd[c]); }
+      int left = __shfl_up_sync(kFull, fi[3], 1), right = __shfl_down_sync(kFull, fd[0], 1);
+      if (lane == 0) left = kTNull;
+      if (lane == 31) right = kTNull;
+      #pragma unroll
+      for (int c = 0; c < 4; ++c) { vi[c] = (c == 0 ? left : fi[c > 0 ? c - 1 : 0]) + 1; vd[c] = c == 3 ? right : fd[c < 3 ? c + 1 : 3]; }
+      if (lane > 0 && lane < 31 && k <= hi) {
+        tile_store<4>(new_rows + (j * 3 + 1) * pitch + idx, vi);
+        tile_store<4>(new_rows + (j * 3 + 2) * pitch + idx, vd);
+      }
+    }
+  }
+  __syncwarp();
 }
 
 // Descriptors of the scores from .. s from their rows (a score without a row is absent).

@@ -80,7 +80,7 @@ struct KernelParams {
   uint32_t* out_runs;
   int64_t out_cap;
   unsigned long long* out_head;  // dense output cursor (shared by all passes)
-  // statistics (optional, may be null): per pair {n_steps, max_leaf_score, max_depth, n_cells}
+  // statistics (optional, may be null; not from the tile kernel): per pair {n_steps, max_leaf_score, max_depth, n_cells}
   int* stats;
   // execution shape (0 = defaults): warps cooperating on one pair, rings in shared memory,
   // physical ring buffers per direction (<= scope; see ring_buffers())

@@ -86,3 +86,30 @@ def test_one_component_tiles_match_oracle(batch_aligner, metric, pen, gw, seed):
         assert res.scores[i] == (score if ops else 0), i
         st, score, _, _ = binding.oracle_align(b.pattern(i), b.text(i), pen, True, metric=metric)
         assert only.status[i] == st and (st != 0 or only.scores[i] == score), i
+
+
+@pytest.mark.parametrize("pen,gw,seed", [((0, 4, 6, 2), 1, 21), ((0, 4, 6, 2), 8, 22), ((0, 2, 3, 1), 1, 23)])
+def test_wide_searches_match_oracle(batch_aligner, pen, gw, seed):
+    """Searches whose two directions meet in blocks of 300 - 1,500 diagonals, whose I and D rows are
+    completed only then: meetings inside long gaps (I and D breakpoints), rows that touch an end."""
+    rng = np.random.default_rng(seed)
+
+    def seq(n):
+        return bytes(rng.choice(list(b"ACGT"), n).astype(np.uint8))
+
+    pairs = [(seq(600), seq(600)), (seq(2200), seq(1300)), (seq(1200), seq(1900))]
+    for n in range(700, 2400, 170):
+        p = seq(n)
+        t = _mutated(rng, p, n // 10, 3)
+        gap, at = int(rng.integers(60, 300)), len(t) // 2 + int(rng.integers(-40, 40))
+        pairs += [(p, t), (p, t[:at] + seq(gap) + t[at:]), (p, t[:at] + t[at + gap:])]
+    b = pkg.PairBatch.from_lists([p for p, _ in pairs], [t for _, t in pairs])
+    try:
+        batch_aligner.set_exec_shape(gw, False)
+        res = batch_aligner.align(b, penalties=pen)
+    finally:
+        batch_aligner.set_exec_shape(1, False)
+    assert (res.status == 0).all()
+    for i in range(b.n):
+        _, score, ops, _ = binding.oracle_align(b.pattern(i), b.text(i), pen)
+        assert res.scores[i] == score and pkg.runs_to_ops(res.runs_of(i)) == ops, (i, b.plen[i], b.tlen[i])
