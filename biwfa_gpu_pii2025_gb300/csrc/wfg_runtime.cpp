@@ -581,6 +581,11 @@ int wfg_run(wfg_context_t* c, const wfg_config_t* cfg, wfg_sched_t sched) {
       while (n_long < n && c->h_plen[(size_t)order[(size_t)n_long]] + c->h_tlen[(size_t)order[(size_t)n_long]] >
                                kDirectWideSum)
         ++n_long;
+    // So do all pairs of a batch in tiles that has a block of the GPU for each of them, if the first
+    // pass's ring cap could stop one: the pair would run the same way there (one pair a block, 15
+    // helpers) until its wavefronts outgrow the cap, and then again in the retry pass. 48 pairs of
+    // 10-20 kbp at 12 %, 37 of which outgrow it: 123 -> 73 ms; one 10 kbp pair that does not: 8.45 and 8.42.
+    if (by_length && p.tile_g && n <= c->num_sms && c->max_sum + 8 + WFG_TILE_MARGIN > (int)kPlainRingCap) n_long = n;
     if (n_long > 0) {
       Launch lw; lw.gw = c->tune.retry_warps; lw.count = n_long; lw.order_off = 0;
       lw.ring_w = (int)next_pow2((uint64_t)c->max_sum + 8);  // capped at the full width

@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 import biwfa_gpu_pii2025_gb300 as pkg
+from biwfa_gpu_pii2025_gb300 import _capi
 from oracle import binding
 
 pytestmark = pytest.mark.gpu
@@ -113,3 +114,24 @@ def test_wide_searches_match_oracle(batch_aligner, pen, gw, seed):
     for i in range(b.n):
         _, score, ops, _ = binding.oracle_align(b.pattern(i), b.text(i), pen)
         assert res.scores[i] == score and pkg.runs_to_ops(res.runs_of(i)) == ops, (i, b.plen[i], b.tlen[i])
+
+
+def test_small_batch_of_wide_pairs(batch_aligner):
+    """A batch with a block for each pair starts in rings of full width: no pair is aligned twice, and
+    the results are those of the first pass's capped rings with their retry pass."""
+    rng = np.random.default_rng(31)
+
+    def seq(n):
+        return bytes(rng.choice(list(b"ACGT"), n).astype(np.uint8))
+
+    p = seq(4000)
+    pairs = [(seq(6000), seq(6000)), (p, _mutated(rng, p, 700, 3)), (seq(5000), b"A"), (seq(40), seq(50))]
+    b = pkg.PairBatch.from_lists([p for p, _ in pairs], [t for _, t in pairs])
+    res = batch_aligner.align(b)
+    assert batch_aligner.stats().retried_pairs == 0
+    capped = batch_aligner.align(b, sched=_capi.SCHED_PLAIN)
+    assert batch_aligner.stats().retried_pairs > 0
+    for i in range(b.n):
+        _, score, ops, _ = binding.oracle_align(b.pattern(i), b.text(i))
+        assert res.status[i] == capped.status[i] == 0 and res.scores[i] == capped.scores[i] == score, i
+        assert pkg.runs_to_ops(res.runs_of(i)) == ops == pkg.runs_to_ops(capped.runs_of(i)), i
