@@ -483,7 +483,7 @@ def run_ours(args):
                                                              "warps_active_per_sm", "dram_throughput_pct",
                                                              "pairs", "launch", "command") if k in counters}
                                    if counters else None),
-                         "kernel": "biwfa_persistent_kernel (3 passes)", "kernel_ms": k_ms,
+                         "kernel": "biwfa_tile_kernel (3 passes)", "kernel_ms": k_ms,
                          "alg_bytes_per_launch": alg_bytes,
                          "note": "integer/latency-bound kernel: algorithmic bytes are 2-bit inputs + score + "
                                  "CIGAR runs; the issue figures (ncu, one launch) show the binding limit"},

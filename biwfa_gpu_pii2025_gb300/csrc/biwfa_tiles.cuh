@@ -21,7 +21,7 @@
 // diagonal and row, 40 % of them paid per step; a tile costs about 60. End to end on a GB300, one
 // score at a time -> tiles (and the kernel of biwfa_tile_kernel.cuh): 10,000 pairs of 1 kbp at 5 %
 // 7.7 -> 3.2 ms, 20,000 uneven pairs (100 bp - 10 kbp, 1-10 %) 320 -> 64 ms, 48 pairs of 10-20 kbp
-// at 12 % 560 -> 123 ms, 200,000 pairs of 150 bp at 2 % 15.4 -> 12.3 ms.
+// at 12 % 560 -> 73 ms, 200,000 pairs of 150 bp at 2 % 15.4 -> 12.3 ms.
 //
 // Where the values are exact. WFA2-lib trims each row to its in-bounds cells and keeps
 // out-of-bounds I/D cells between them. Out-of-bounds cells arise only from a cell whose offset

