@@ -48,7 +48,7 @@ enum { kOne, kHalves, kBoth };
 struct TileJob {
   unsigned long long ticket;  // generation << 48 | tiles << 24 | next tile
   int done;                   // tiles computed
-  int t0, d_tiles;            // tiles 0 .. d_tiles - 1 are dir[d]'s, the rest dir[1]'s
+  int t0, d_tiles, tiles;     // tiles 0 .. d_tiles - 1 are dir[d]'s, the rest dir[1]'s
   int d;
   int part[10];               // results: d's antidiagonals of four rows and first touched row, then e's
 };
@@ -103,6 +103,12 @@ __device__ __forceinline__ TileBlockSmem& tile_smem() { return *reinterpret_cast
 __device__ __forceinline__ int job_next(unsigned long long ticket) { return (int)(ticket & 0xffffffu); }
 __device__ __forceinline__ int job_tiles(unsigned long long ticket) { return (int)((ticket >> 24) & 0xffffffu); }
 
+// A word that other warps write while this one decides by it: one lane reads it for all, as lanes
+// that read it one after another could decide differently and part at the next shuffle.
+__device__ __forceinline__ int warp_read(const int& word, int lane) {
+  return __shfl_sync(kFull, lane == 0 ? *(const volatile int*)&word : 0, 0);
+}
+
 // Takes a tile of the job for this warp: its number, or -1.
 __device__ __forceinline__ int job_take(TileJob& job, int lane) {
   int i = -1;
@@ -114,7 +120,7 @@ __device__ __forceinline__ int job_take(TileJob& job, int lane) {
     }
   }
   i = __shfl_sync(kFull, i, 0);
-  if (i >= 0) __threadfence_block();
+  if (i >= 0) { __threadfence_block(); __syncwarp(); }
   return i;
 }
 
@@ -158,7 +164,7 @@ __device__ __noinline__ void job_open(int d, bool both, int t0, int state, int g
   TileJob& job = S.job;
   const int nd = S.dir[d].ts.tiles, tiles = nd + (both ? S.dir[1].ts.tiles : 0);
   if (lane < 10) job.part[lane] = lane == 4 || lane == 9 ? 4 : INT_MIN;
-  if (lane == 0) { job.d = d; job.d_tiles = nd; job.t0 = t0; job.done = 0; }
+  if (lane == 0) { job.d = d; job.d_tiles = nd; job.tiles = tiles; job.t0 = t0; job.done = 0; }
   __syncwarp();
   if (lane == 0) {
     __threadfence_block();
@@ -197,7 +203,7 @@ __device__ __noinline__ bool tile_request(int d, bool both, int t0, int state, i
   C.state = state;
   C.mode = halves ? kHalves : both ? kBoth : kOne;
   __syncwarp();
-  if (!halves && state != kLeaf && *(volatile int*)&B.idle > 0 && S.dir[d].ts.tiles + (both ? S.dir[1].ts.tiles : 0) > 1)
+  if (!halves && state != kLeaf && S.dir[d].ts.tiles + (both ? S.dir[1].ts.tiles : 0) > 1 && warp_read(B.idle, lane) > 0)
     job_open(d, both, t0, state, gib, lane);
   return true;
 }
@@ -235,9 +241,9 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
 
   if (state == kHelp || state == kOwnJob) {
     if (state == kOwnJob) {  // no tile is left to take: wait for the helpers'
-      const int tiles = job_tiles(*(volatile unsigned long long*)&S.job.ticket);
+      const int tiles = S.job.tiles;
       int spins = 0;
-      while (*(volatile int*)&S.job.done < tiles && spins < kSpinLimit) { ++spins; __nanosleep(20); }
+      while (warp_read(S.job.done, lane) < tiles && spins < kSpinLimit) { ++spins; __nanosleep(20); }
       __threadfence_block();
       __syncwarp();
       if (lane < 10) C.part[lane] = *(volatile int*)&S.job.part[lane];
@@ -584,7 +590,7 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
 
     if (state == kHelp) {
       // Queue empty: tiles of the block's other warps until none has a pair.
-      for (int spins = 0; spins < kSpinLimit && *(volatile int*)&B.active > 0; ++spins) {
+      for (int spins = 0; spins < kSpinLimit && warp_read(B.active, lane) > 0; ++spins) {
         #pragma unroll 1
         for (int k = 1; k < kTileWarps; ++k) {
           const int w = gib + k < kTileWarps ? gib + k : gib + k - kTileWarps;

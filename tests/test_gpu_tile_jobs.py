@@ -1,0 +1,44 @@
+"""Tiles that a thread block's idle warps take (csrc/biwfa_tile_kernel.cuh) against the oracle, bit for
+bit: several owners per block with jobs open at once, pairs of very different width beside each other,
+one owner with all other warps helping."""
+import numpy as np
+import pytest
+
+import biwfa_gpu_pii2025_gb300 as pkg
+from oracle import binding
+
+pytestmark = pytest.mark.gpu
+
+
+def _pairs(rng, n):
+    """Every eighth pair is wide (unrelated sequences of 300 - 1,200 bases), the others narrow or empty."""
+    pairs = []
+    for i in range(n):
+        if i % 8 == 0:
+            a, b = (rng.choice(list(b"ACGT"), int(rng.integers(300, 1200))).astype(np.uint8) for _ in range(2))
+        else:
+            a = rng.choice(list(b"ACGT"), int(rng.integers(0, 700))).astype(np.uint8)
+            b = a.copy()
+            for at in rng.integers(0, max(1, a.size), a.size // 25):
+                b[at] = rng.choice(list(b"ACGT"))
+            b = np.delete(b, rng.integers(0, a.size, a.size // 40)) if a.size else b
+        pairs.append((bytes(a), bytes(b)))
+    return pairs
+
+
+@pytest.mark.parametrize("n,gw,seed", [(3, 1, 1), (200, 1, 2), (700, 1, 3), (400, 4, 4), (170, 8, 5)])
+@pytest.mark.parametrize("metric,pen", [(binding.METRIC_AFFINE, (0, 4, 6, 2)), (binding.METRIC_LINEAR, (0, 4, 2, 0))])
+def test_several_owners_share_helpers(batch_aligner, n, gw, seed, metric, pen):
+    pairs = _pairs(np.random.default_rng(seed), n)
+    b = pkg.PairBatch.from_lists([p for p, _ in pairs], [t for _, t in pairs])
+    try:
+        batch_aligner.set_exec_shape(gw, False)
+        res = [batch_aligner.align(b, penalties=pen, metric=metric) for _ in range(2)]
+    finally:
+        batch_aligner.set_exec_shape(1, False)
+    for r in res:
+        assert (r.status == 0).all()
+    for i in range(n):
+        _, score, ops, _ = binding.oracle_align(b.pattern(i), b.text(i), pen, metric=metric)
+        for r in res:
+            assert pkg.runs_to_ops(r.runs_of(i)) == ops and r.scores[i] == (score if ops else 0), i
