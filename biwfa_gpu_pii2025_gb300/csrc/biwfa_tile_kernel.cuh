@@ -330,18 +330,21 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
 
     if (state == kPop) {
       // wavefront_bialign_alignment's recursion on an explicit stack (half_0 before half_1)
-      if (C.sp == 0 || C.status != ST_OK) {
+      // sp is read once and written behind a barrier: a lane that still compares must not see the
+      // root's -1 already replaced by 0, the empty stack.
+      const int sp = C.sp;
+      if (sp == 0 || C.status != ST_OK) {
         state = kFinish;
       } else {
-        if (C.sp > 0) {
-          const int sp = C.sp - 1;
-          const int4* e = reinterpret_cast<const int4*>(S.arena.stack + sp * 8);
+        if (sp > 0) {
+          const int4* e = reinterpret_cast<const int4*>(S.arena.stack + (sp - 1) * 8);
           const int4 a = e[0], b = e[1];
           __syncwarp();
-          C.sp = sp;
+          C.sp = sp - 1;
           C.pb = a.x; C.pe = a.y; C.tb = a.z; C.te = a.w;
           C.cb = b.x; C.ce = b.y; C.rem = b.z;
         } else {
+          __syncwarp();
           C.sp = 0;
         }
         __syncwarp();

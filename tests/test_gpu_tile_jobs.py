@@ -42,3 +42,22 @@ def test_several_owners_share_helpers(batch_aligner, n, gw, seed, metric, pen):
         _, score, ops, _ = binding.oracle_align(b.pattern(i), b.text(i), pen, metric=metric)
         for r in res:
             assert pkg.runs_to_ops(r.runs_of(i)) == ops and r.scores[i] == (score if ops else 0), i
+
+
+@pytest.mark.parametrize("n,lo,hi", [(20000, 1, 101), (3000, 101, 160)])
+def test_every_root_is_aligned(batch_aligner, n, lo, hi):
+    """The recursion's root is no stack entry: each pair, whether its root is a leaf (both sides up to
+    100 bases) or a search, ends with the oracle's CIGAR and none with an empty one."""
+    rng = np.random.default_rng(n)
+    pairs = []
+    for _ in range(n):
+        p = rng.choice(list(b"ACGT"), int(rng.integers(lo, hi))).astype(np.uint8)
+        t = p.copy()
+        t[rng.integers(0, t.size)] = ord("C")
+        pairs.append((bytes(p), bytes(np.append(t, t[:int(rng.integers(0, 4))]))))
+    b = pkg.PairBatch.from_lists([p for p, _ in pairs], [t for _, t in pairs])
+    res = batch_aligner.align(b)
+    assert (res.status == 0).all() and (res.run_len > 0).all()
+    for i in range(n):
+        _, score, ops, _ = binding.oracle_align(b.pattern(i), b.text(i))
+        assert pkg.runs_to_ops(res.runs_of(i)) == ops and res.scores[i] == score, i
