@@ -679,8 +679,8 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks) biwfa_tile_kerne
       const int tiles = my.ts.tiles, narrow = my.ts.narrow;
       TileArgs a;
       a.pitch = my.cfg.pitch;
-      a.old_rows = my.cfg.rdata + (b == 0 ? 2 : b - 1) * 12 * a.pitch;
-      a.new_rows = my.cfg.rdata + b * 12 * a.pitch;
+      a.old_rows = my.cfg.rdata + wfg_tile_row((b == 0 ? 2 : b - 1) * 12, a.pitch);
+      a.new_rows = my.cfg.rdata + wfg_tile_row(b * 12, a.pitch);
       a.mask = (uint32_t)my.cfg.W - 1u;
       a.old_lo = my.ts.lo; a.old_hi = my.ts.hi;
       a.first = tl == 0; a.last = tl == L - 1;

@@ -287,7 +287,7 @@ __device__ __noinline__ int tile_start(Dir& d, const SeqView& sv, int cb, int ce
   if (lane < 6) {
     const int row = lane < 4 ? (8 + lane) * 3 : 11 * 3 + lane - 3;
     const int mine = lane < 3 ? -1 : lane - 3;  // the component of row 0
-    *reinterpret_cast<int4*>(d.cfg.rdata + row * d.cfg.pitch) =
+    *reinterpret_cast<int4*>(d.cfg.rdata + wfg_tile_row(row, d.cfg.pitch)) =
         make_int4(mine == comp_index(cb) ? off0 : kTNull, kTNull, kTNull, kTNull);
   }
   __syncwarp();
@@ -310,8 +310,8 @@ __device__ __noinline__ void tile_gaps(const Dir& d, int t0, const Pen& p, int l
   const int lo = row_lo<false>(d.cb, t0 + 4, p) & ~3, hi = row_hi<false>(d.cb, t0 + 4, p);
   const int old_lo = row_lo<false>(d.cb, t0, p) & ~3, old_hi = (row_hi<false>(d.cb, t0, p) + 4) & ~3;
   const int b = (t0 >> 2) % 3, pitch = d.cfg.pitch;
-  const int32_t* old_rows = d.cfg.rdata + (b == 0 ? 2 : b - 1) * 12 * pitch;
-  int32_t* new_rows = d.cfg.rdata + b * 12 * pitch;
+  const int32_t* old_rows = d.cfg.rdata + wfg_tile_row((b == 0 ? 2 : b - 1) * 12, pitch);
+  int32_t* new_rows = d.cfg.rdata + wfg_tile_row(b * 12, pitch);
   #pragma unroll 1
   for (int base = lo - 4; base < hi; base += 120) {  // a halo of four diagonals per side
     const int k = base + lane * 4;
@@ -532,13 +532,13 @@ __device__ __noinline__ void tile_overlap(const Dir& d0, const Dir& d1, int s0, 
                                                plen + tlen);
   const uint32_t mask = (uint32_t)d0.cfg.W - 1u;
   const int pitch = d0.cfg.pitch;
-  const int32_t* r0 = d0.cfg.rdata + row_buffer(t0) * 3 * pitch;
+  const int32_t* r0 = d0.cfg.rdata + wfg_tile_row(row_buffer(t0) * 3, pitch);
   while (todo) {
     const int s = s1 - (__ffs((int)todo) - 1);
     todo &= todo - 1;
     if (s0 + s - p.go >= bp.score) continue;
     const int t1 = row_of(s, p);
-    const int32_t* r1 = d1.cfg.rdata + row_buffer(t1) * 3 * pitch;
+    const int32_t* r1 = d1.cfg.rdata + wfg_tile_row(row_buffer(t1) * 3, pitch);
     const int end = min(row_hi<LIN>(cb0, t0, p), A - row_lo<LIN>(cb1, t1, p));
     int first[3] = {INT_MAX, INT_MAX, INT_MAX};  // lowest diagonal where M, I, D meet
     #pragma unroll 1

@@ -103,6 +103,12 @@ struct KernelParams {
 #define WFG_TILE_BUFS 12
 #define WFG_TILE_PAD 64
 #define WFG_TILE_MARGIN 160
+// Ints from the start of a direction's tile rings to row `row` (buffer * 3 + component). 64 bits: the
+// longest accepted pairs (plen + tlen just below 2^26, at unit penalties) have rings of 2^27 diagonals,
+// and the last of 36 rows starts beyond 2^31 ints from 2^26 diagonals on. Within a block's 12 rows
+// 32 bits do.
+WFG_HD constexpr inline int64_t wfg_tile_row(int row, int pitch) { return (int64_t)row * pitch; }
+static_assert(12 * (int64_t)((1 << 27) + WFG_TILE_PAD) <= INT32_MAX, "a block's rows are indexed with 32 bits");
 
 // Physical ring buffers a direction needs: scores that can hold a wavefront are multiples of
 // g = gcd(x, o+e, e), so any window of `scope` consecutive scores holds at most ceil(scope/g)
