@@ -30,13 +30,18 @@
 // removes nulls, and the rows here equal WFA2-lib's with its nulls (any negative offset is null).
 // From the row after it the one-step functions (dir_step) continue from the stored rows.
 
-constexpr int kTNull = -(1 << 28);  // null offset of a row; the few units it drifts never make it positive
+// Null offset of a row. A row treats nulls as cells: one that it passes on grows by 1 and by the
+// matches in the window at the sequences' starts (up to 16), so by at most 17 per row. A search's rows
+// number at most half of the largest accepted score (2^26) plus the score scope, so no null becomes
+// positive; and twice a null, less a diagonal, still fits 32 bits (WFG_TILE_NULL).
+constexpr int kTNull = WFG_TILE_NULL;
 constexpr int kTileHalo = 4;
 constexpr int kTX = 2, kTO = 4;     // rows back to the mismatch and the gap-opening source
 constexpr int kTileMinRing = 256;   // narrowest ring that is worth tiles
 
-// Row of score s (rounded down) and whether s has one. The spacing is at most 8 and scores stay
-// below 2^27, so the product with tm = floor(2^32 / tg) + 1 divides exactly.
+// Row of score s (rounded down) and whether s has one. With tm = floor(2^32 / tg) + 1 the product is
+// exact while s * tg < 2^32: scores stay below 2^27, and the spacing is at most 31 (gap-linear 31/31,
+// the largest within the score scope of 32).
 __device__ __forceinline__ int row_of(int s, const Pen& p) { return p.tg == 1 ? s : (int)__umulhi((uint32_t)s, p.tm); }
 __device__ __forceinline__ bool holds_row(int s, const Pen& p) { return s == row_of(s, p) * p.tg; }
 

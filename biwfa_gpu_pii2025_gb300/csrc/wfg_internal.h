@@ -103,6 +103,12 @@ struct KernelParams {
 #define WFG_TILE_BUFS 12
 #define WFG_TILE_PAD 64
 #define WFG_TILE_MARGIN 160
+// Null offset of the tile kernel's rows (biwfa_tiles.cuh), between two bounds: below minus 17 for each
+// row of a search (2^25 + scope), and twice it less a diagonal (2^27) within 32 bits.
+#define WFG_TILE_NULL (-(5 << 27))
+static_assert(WFG_TILE_NULL + 17 * ((int64_t)(1 << 25) + 2 * WFG_MAX_SCOPE) < 0, "a null stays negative");
+static_assert(2 * (int64_t)WFG_TILE_NULL - (1 << 27) - 8 >= INT32_MIN, "twice a null fits 32 bits");
+
 // Ints from the start of a direction's tile rings to row `row` (buffer * 3 + component). 64 bits: the
 // longest accepted pairs (plen + tlen just below 2^26, at unit penalties) have rings of 2^27 diagonals,
 // and the last of 36 rows starts beyond 2^31 ints from 2^26 diagonals on. Within a block's 12 rows

@@ -61,3 +61,15 @@ def test_every_root_is_aligned(batch_aligner, n, lo, hi):
     for i in range(n):
         _, score, ops, _ = binding.oracle_align(b.pattern(i), b.text(i))
         assert pkg.runs_to_ops(res.runs_of(i)) == ops and res.scores[i] == score, i
+
+
+@pytest.mark.parametrize("pen,seed", [((0, 31, 31, 0), 41), ((0, 28, 28, 0), 42), ((0, 7, 28, 0), 43), ((0, 31, 31, 0), 44)])
+def test_widest_score_spacings(batch_aligner, pen, seed):
+    """Gap-linear scores that hold a row lie up to 31 apart, the most that the score scope allows."""
+    pairs = _pairs(np.random.default_rng(seed), 60)
+    b = pkg.PairBatch.from_lists([p for p, _ in pairs], [t for _, t in pairs])
+    res = batch_aligner.align(b, penalties=pen, metric=binding.METRIC_LINEAR)
+    assert (res.status == 0).all()
+    for i in range(b.n):
+        _, score, ops, _ = binding.oracle_align(b.pattern(i), b.text(i), pen, metric=binding.METRIC_LINEAR)
+        assert pkg.runs_to_ops(res.runs_of(i)) == ops and res.scores[i] == (score if ops else 0), i

@@ -36,3 +36,13 @@ def test_ring_rows_are_reached_through_the_64_bit_offset():
         for line in (CSRC / name).read_text().splitlines():
             if re.search(r"rdata \+", line):
                 assert "wfg_tile_row" in line, (name, line)
+
+
+def test_nulls_stay_negative_over_the_longest_search():
+    """A null grows by at most 17 a row (one and a window of 16 matches); a search has at most half of the
+    largest accepted score (2^26) in rows, plus the score scope, and adds two nulls and a diagonal."""
+    null = -5 * 2 ** 27
+    text = (CSRC / "wfg_internal.h").read_text()
+    assert "#define WFG_TILE_NULL (-(5 << 27))" in text
+    assert "constexpr int kTNull = WFG_TILE_NULL;" in (CSRC / "biwfa_tiles.cuh").read_text()
+    assert null + 17 * (2 ** 25 + 64) < 0 and 2 * null - 2 ** 27 >= -2 ** 31
