@@ -30,7 +30,11 @@ namespace {
 #endif
 constexpr int kTileWarps = WFG_TILE_WARPS;    // warps per thread block
 constexpr int kTileBlocks = WFG_TILE_BLOCKS;  // thread blocks per SM
-constexpr int kSpinLimit = 1 << 24;
+// Limits of the waits for other warps, in polls. A poll costs 20 ns at least. A tile ends by itself; the
+// longest follow four diagonals over both whole sequences, at worst half a window (4 bases of 8 bits) per
+// base and 1 us of memory latency per window, so an owner polls 128 times per base of its pair beyond
+// the constant before it gives a helper up. A helper without work leaves after about 10 s.
+constexpr int kSpinLimit = 1 << 24, kPollsPerBase = 128;
 // Warps of a block that own pairs, by the launch's warps per pair; the others help.
 __host__ __device__ constexpr int biwfa_owners(int group_warps) {
   return group_warps <= 1 ? kTileWarps : group_warps == 4 ? 2 : 1;
@@ -242,8 +246,21 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
   if (state == kHelp || state == kOwnJob) {
     if (state == kOwnJob) {  // no tile is left to take: wait for the helpers'
       const int tiles = S.job.tiles;
-      int spins = 0;
-      while (warp_read(S.job.done, lane) < tiles && spins < kSpinLimit) { ++spins; __nanosleep(20); }
+      const long long limit = P.wait_polls > 0 ? P.wait_polls
+                                               : kSpinLimit + (long long)kPollsPerBase * (C.q.plen + C.q.tlen);
+      long long polls = 0;
+      bool ended;
+      while (!(ended = warp_read(S.job.done, lane) >= tiles) && polls < limit) { ++polls; __nanosleep(20); }
+      if (!ended) {
+        // A helper holds a tile of this warp's rings and job, now or later: nothing may use them again in
+        // this launch. The run has failed; the warp takes no more pairs.
+        if (lane == 0) {
+          atomicAdd(P.lost, 1ull);
+          P.scores[C.pi] = 0; P.status[C.pi] = WFG_ST_DEVICE_ERROR; P.run_off[C.pi] = 0; P.run_len[C.pi] = 0;
+          atomicSub(&B.active, 1);
+        }
+        return false;
+      }
       __threadfence_block();
       __syncwarp();
       if (lane < 10) C.part[lane] = *(volatile int*)&S.job.part[lane];
@@ -259,7 +276,6 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
       tile_done(S.dir[C.d], C.t0, C.part[4]);
       if (both) tile_done(R, C.t0, C.part[9]);
       __syncwarp();
-      if (spins >= kSpinLimit) { st = WFG_ST_UNATTAINABLE; state = kBpDone; }  // a helper was lost
       if (state == kSearch) {
         // as behind the pass in the kernel: on to the next block unless a row may hold an event
         int nf = C.fmax, nr = C.rmax;
@@ -602,6 +618,7 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
         }
         __nanosleep(200);
       }
+      if (lane == 0) atomicSub(&B.idle, 1);
       return false;
     }
   }

@@ -63,6 +63,7 @@ constexpr int kSmemRingW = 1024;              // widest ring of the shared-memor
 constexpr int64_t kSmemRingBytes = 200 << 10;  // dynamic shared memory budget for both rings
 constexpr int kCountersPerPass = 4;  // [queue head, retry count, -, -]
 constexpr int kOutHeadIndex = kNumPasses * kCountersPerPass;
+constexpr int kLostIndex = kOutHeadIndex + 1;  // waits of the tile kernel that ran out
 constexpr int kNumCounters = kOutHeadIndex + 4;
 
 // Kernel launchers (biwfa_kernel.cu, mlp_kernel.cu).
@@ -128,6 +129,7 @@ struct wfg_context {
   bool ran = false;
   int last_score_only = 0;
   int limit_ring_w = 0, limit_leaf_words = 0;
+  int limit_wait_polls = 0;  // wfg_test_limit_waits
   // learned scheduling
   wfg::DevBuf<uint16_t> d_feats;   // num_pairs x 32 bf16
   wfg::DevBuf<float> d_pred;       // predicted scores

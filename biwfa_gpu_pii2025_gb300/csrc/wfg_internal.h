@@ -31,6 +31,7 @@ enum {
   WFG_ST_OOM = -200,              // WFA2's WF_STATUS_OOM
   WFG_ST_UNATTAINABLE = -300,
   WFG_ST_SCRATCH_OVERFLOW = -210, // the pair needs a larger per-warp arena (retried by the host)
+  WFG_ST_DEVICE_ERROR = -500,     // WF_STATUS_DEVICE_ERROR
   WFG_ST_OUTPUT_OVERFLOW = -220,  // the dense output span could not be reserved
 };
 
@@ -89,6 +90,10 @@ struct KernelParams {
   int ring_nphys;
   // rows in tiles (biwfa_tiles.cuh): the spacing of the scores that hold a row, 0 for one score at a time
   int tile_g;
+  // the tile kernel's waits for another warp: counter of those that ran out (the run has failed then),
+  // and their limit in polls (0: from the pair's length)
+  unsigned long long* lost;
+  int wait_polls;
 };
 
 // Score scope caps (max(x, o+e[, o2+e2]) + 1 after the match transform): the ring descriptors

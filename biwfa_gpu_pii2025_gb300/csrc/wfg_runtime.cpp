@@ -379,6 +379,8 @@ KernelParams launch_params(const wfg_context* c, const wfg_config_t* cfg, const 
   kp.ring_in_smem = l.smem;
   kp.ring_nphys = l.nphys;
   kp.tile_g = l.smem ? 0 : p.tile_g;
+  kp.lost = c->d_counters.ptr + kLostIndex;
+  kp.wait_polls = c->limit_wait_polls;
   kp.retry_out = (ps + 1 < kNumPasses) ? c->d_retry.ptr + (size_t)ps * n : nullptr;
   kp.retry_count = c->d_counters.ptr + ps * kCountersPerPass + 1;
   return kp;
@@ -489,9 +491,25 @@ int validate_config(wfg_context* c, const wfg_config_t* cfg, IntPen* p) {
   return WF_STATUS_ALG_COMPLETED;
 }
 
+// Whether the last run ended as it should (its counters are in pinned memory). A warp whose wait for
+// another one ran out takes no more pairs, so the results are not complete then.
+int run_status(wfg_context* c) {
+  if (!c->ran || c->h_counters.ptr[kLostIndex] == 0) return WF_STATUS_ALG_COMPLETED;
+  c->err = "a warp waited in vain for another warp's part of a pair; the results are not complete";
+  return WF_STATUS_DEVICE_ERROR;
+}
+
 }  // namespace
 
 extern "C" {
+
+// Not part of the API: how often the tile kernel polls before a wait has run out (0: from the pair's
+// length), so that a test can make one run out.
+int wfg_test_limit_waits(wfg_context_t* c, int polls) {
+  if (!c || polls < 0) return WF_STATUS_UNSUPPORTED;
+  c->limit_wait_polls = polls;
+  return WF_STATUS_ALG_COMPLETED;
+}
 
 int wfg_run(wfg_context_t* c, const wfg_config_t* cfg, wfg_sched_t sched) {
   if (!c || !cfg) return WF_STATUS_UNSUPPORTED;
@@ -791,7 +809,7 @@ int wfg_set_learned_policy(wfg_context_t* c, float wide_threshold, int wide_warp
 int wfg_synchronize(wfg_context_t* c) {
   if (!c) return WF_STATUS_UNSUPPORTED;
   WFG_CHECK(c, cudaStreamSynchronize(c->stream));
-  return WF_STATUS_ALG_COMPLETED;
+  return run_status(c);
 }
 
 int wfg_get_stats(wfg_context_t* c, wfg_stats_t* out) {
@@ -819,6 +837,8 @@ int wfg_fetch(wfg_context_t* c, int* scores, int* statuses, int64_t* run_off, in
   if (!c || !c->ran) return WF_STATUS_UNSUPPORTED;
   cudaSetDevice(c->device);
   WFG_CHECK(c, cudaStreamSynchronize(c->stream));  // counters are in pinned memory now
+  const int rst = run_status(c);
+  if (rst != WF_STATUS_ALG_COMPLETED) return rst;
   const int n = c->n;
   const int64_t nruns = c->last_score_only ? 0 : (int64_t)c->h_counters.ptr[kOutHeadIndex];
   int64_t d2h = 0;

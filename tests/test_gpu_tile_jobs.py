@@ -1,6 +1,8 @@
 """Tiles that a thread block's idle warps take (csrc/biwfa_tile_kernel.cuh) against the oracle, bit for
 bit: several owners per block with jobs open at once, pairs of very different width beside each other,
 one owner with all other warps helping."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -73,3 +75,27 @@ def test_widest_score_spacings(batch_aligner, pen, seed):
     for i in range(b.n):
         _, score, ops, _ = binding.oracle_align(b.pattern(i), b.text(i), pen, metric=binding.METRIC_LINEAR)
         assert pkg.runs_to_ops(res.runs_of(i)) == ops and res.scores[i] == (score if ops else 0), i
+
+
+def test_a_wait_that_runs_out_fails_the_run_and_leaves_the_context_usable(batch_aligner):
+    """With one poll before a wait for a helper's tile has run out, the run ends with a device error and
+    not with an alignment status; the next run, with the usual limit, is right."""
+    rng = np.random.default_rng(51)
+    pairs = [tuple(bytes(rng.choice(list(b"ACGT"), 3000).astype(np.uint8)) for _ in range(2)) for _ in range(4)]
+    b = pkg.PairBatch.from_lists([p for p, _ in pairs], [t for _, t in pairs])
+    limit = batch_aligner.lib.wfg_test_limit_waits
+    limit.argtypes = [C.c_void_p, C.c_int]
+    batch_aligner.upload(b)
+    try:
+        assert limit(batch_aligner.ctx, 1) == 0
+        batch_aligner.run()
+        with pytest.raises(RuntimeError, match="waited in vain"):
+            batch_aligner.fetch()
+        with pytest.raises(RuntimeError, match="waited in vain"):
+            batch_aligner.synchronize()
+    finally:
+        assert limit(batch_aligner.ctx, 0) == 0
+    res = batch_aligner.align(b)
+    for i in range(b.n):
+        _, score, ops, _ = binding.oracle_align(b.pattern(i), b.text(i))
+        assert res.status[i] == 0 and res.scores[i] == score and pkg.runs_to_ops(res.runs_of(i)) == ops, i
