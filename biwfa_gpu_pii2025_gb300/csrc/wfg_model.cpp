@@ -24,11 +24,18 @@ struct wfg_model {
   PinBuf<int> h_rows;
   PinBuf<float> h_loss;
   cudaEvent_t rows_copied[2] = {};
-  // captured epoch
+  // captured epoch, and what its nodes hold: sizes, the learning rate, and every buffer that a later
+  // call may replace by a larger one (wfg_model_gradient, or a larger batch)
   cudaGraphExec_t epoch_exec = nullptr;
-  int graph_rows = -1, graph_batch = -1;
-  float graph_lr = -1.f;
-  const void* graph_feats = nullptr;
+  struct EpochKey {
+    int rows, batch, num_sms;
+    float lr;
+    const void *feats, *targets, *row_order;
+    bool operator==(const EpochKey& k) const {
+      return rows == k.rows && batch == k.batch && num_sms == k.num_sms && lr == k.lr && feats == k.feats &&
+             targets == k.targets && row_order == k.row_order;
+    }
+  } epoch_key{};
 };
 
 namespace {
@@ -185,8 +192,8 @@ int wfg_model_train(wfg_model_t* m, wfg_context_t* c, const int* target_scores, 
   WFG_CHECK(c, launch_mlp_targets(n, m->d_rows.ptr, m->d_targets.ptr, c->stream));
   const float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
   // Capture one epoch (all minibatches) once; replays read the shuffled row order from d_rows.
-  if (!m->epoch_exec || m->graph_rows != n || m->graph_batch != batch_rows || m->graph_lr != lr ||
-      m->graph_feats != c->d_feats.ptr) {
+  const wfg_model::EpochKey key{n, batch_rows, c->num_sms, lr, c->d_feats.ptr, m->d_targets.ptr, m->d_rows.ptr};
+  if (!m->epoch_exec || !(m->epoch_key == key)) {
     if (m->epoch_exec) { cudaGraphExecDestroy(m->epoch_exec); m->epoch_exec = nullptr; }
     cudaGraph_t graph;
     WFG_CHECK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
@@ -208,7 +215,7 @@ int wfg_model_train(wfg_model_t* m, wfg_context_t* c, const int* target_scores, 
     const cudaError_t inst = cudaGraphInstantiate(&m->epoch_exec, graph, 0);
     cudaGraphDestroy(graph);
     if (inst != cudaSuccess) return wfg_fail(c, inst, "cudaGraphInstantiate");
-    m->graph_rows = n; m->graph_batch = batch_rows; m->graph_lr = lr; m->graph_feats = c->d_feats.ptr;
+    m->epoch_key = key;
   }
   // The epochs run one after another on the stream; the host draws the next epoch's row order
   // meanwhile and waits once, at the end.
