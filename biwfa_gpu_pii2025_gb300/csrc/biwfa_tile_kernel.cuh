@@ -522,11 +522,11 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
       }
       if (lane == 0) L.cfg.ldata[0] = off0;
       L.sv = sv; L.cb = C.cb; L.ce = C.ce; L.num_null = 0; L.status = ST_OK; L.end_k = sv.tlen - sv.plen;
-      C.leaf_end = leaf_at<LIN>(0);
+      C.leaf_end = leaf_at<LIN>(0, pen);
       __syncwarp();
       state = kLeafSteps;
       s = 0; done = false;
-      if (4 * pen.tg <= L.cfg.lmax && leaf_at<LIN>(1) <= L.lcap && tile_request<LIN>(0, false, 0, kLeaf, gib, lane)) {
+      if (4 * pen.tg <= L.cfg.lmax && leaf_at<LIN>(1, pen) <= L.lcap && tile_request<LIN>(0, false, 0, kLeaf, gib, lane)) {
         C.out = out; C.bp = bp;
         __syncwarp();
         return true;
@@ -540,7 +540,7 @@ __device__ __noinline__ bool tile_control(int gib, int lane, int owners) {
       s = last * pen.tg;
       if (touch < 4 && row_exists<LIN>(C.cb, last, ci, pen) && row_lo<LIN>(C.cb, last, pen) <= ak &&
           ak <= row_hi<LIN>(C.cb, last, pen))
-        done = L.cfg.ldata[leaf_cell<LIN>(C.cb, last, ci, ak)] >= L.sv.tlen;
+        done = L.cfg.ldata[leaf_cell<LIN>(C.cb, last, ci, ak, pen)] >= L.sv.tlen;
       state = kLeafSteps;
     }
 
@@ -704,8 +704,8 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks) biwfa_tile_kerne
       a.lane = lane;
       a.gaps = my.ts.gaps;
       if (LIN) { a.lx = S.pen.lx; a.lo = S.pen.lo; }
-      a.leaf = leaf ? S.dir[2].cfg.ldata + leaf_at<LIN>(t0 >> 2) : nullptr;
-      a.leaf_lo = leaf_lo<LIN>(my.cb, t0 >> 2); a.leaf_n = leaf ? leaf_n<LIN>(t0 >> 2) : 0;
+      a.leaf = leaf ? S.dir[2].cfg.ldata + leaf_at<LIN>(t0 >> 2, S.pen) : nullptr;
+      a.leaf_lo = leaf_lo<LIN>(my.cb, t0 >> 2, S.pen); a.leaf_n = leaf ? leaf_n<LIN>(t0 >> 2, S.pen) : 0;
       int ak = INT_MIN, tch = 4;
       const int step = C.step;
       int i = C.tile;
@@ -763,10 +763,10 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks) biwfa_tile_kerne
         C.state = kSearchEvent;
       }
     } else if (state == kLeaf) {
-      const int end = leaf_at<LIN>((t0 >> 2) + 1);
+      const int end = leaf_at<LIN>((t0 >> 2) + 1, S.pen);
       C.leaf_end = end;
       if (touch[0] == 4 && t0 <= C.guard && (t0 + 8) * S.pen.tg <= S.dir[2].cfg.lmax &&
-          leaf_at<LIN>((t0 >> 2) + 2) <= S.dir[2].lcap && tile_request<LIN>(0, false, t0 + 4, kLeaf, gib, lane)) {
+          leaf_at<LIN>((t0 >> 2) + 2, S.pen) <= S.dir[2].lcap && tile_request<LIN>(0, false, t0 + 4, kLeaf, gib, lane)) {
         control = false;
       } else {
         C.state = kLeafEvent;

@@ -401,20 +401,24 @@ __device__ __noinline__ int tile_advance(Dir& d, const Pen& p, int s, const Grp<
   return dir_step<1, 0, false>(d, p, s, g, max_ak_out);
 }
 
-// The leaf store of a leaf whose rows come in tiles: row 0's one cell at 0, then block b's four rows
-// (M, I, D each, or M alone) of leaf_n(b) diagonals from leaf_lo(cb, b) at leaf_at(b), all multiples
-// of 4 that cover row_lo .. row_hi. So a row's place follows from its number, without a descriptor.
+// The leaf store of a leaf whose rows come in tiles (layout and sizes: wfg_tile_leaf_at): block b's rows
+// of leaf_n(b) diagonals from leaf_lo(cb, b) at leaf_at(b) cover row_lo .. row_hi. So a row's place
+// follows from its number, without a descriptor.
 template <bool LIN>
-__device__ __forceinline__ int leaf_n(int b) { return 8 * b + (LIN ? 12 : 8); }
+__device__ __forceinline__ int leaf_q(int b, const Pen& p) { return LIN ? row_hi<true>(CM, b, p) : b; }  // LIN: b / lo
 template <bool LIN>
-__device__ __forceinline__ int leaf_lo(int cb, int b) { return !LIN && cb == CI ? -4 * b : -4 * b - 4; }
+__device__ __forceinline__ int leaf_n(int b, const Pen& p) { return wfg_tile_leaf_n(LIN, leaf_q<LIN>(b, p)); }
 template <bool LIN>
-__device__ __forceinline__ int leaf_at(int b) { return LIN ? 4 + 16 * b * (b + 2) : 4 + 48 * b * (b + 1); }
+__device__ __forceinline__ int leaf_lo(int cb, int b, const Pen& p) {
+  return !LIN && cb == CI ? -4 * b : -4 * leaf_q<LIN>(b, p) - 4;
+}
+template <bool LIN>
+__device__ __forceinline__ int leaf_at(int b, const Pen& p) { return wfg_tile_leaf_at(LIN, b, leaf_q<LIN>(b, p), p.lo); }
 // Row t's component ci on diagonal k (t >= 1).
 template <bool LIN>
-__device__ __forceinline__ int leaf_cell(int cb, int t, int ci, int k) {
+__device__ __forceinline__ int leaf_cell(int cb, int t, int ci, int k, const Pen& p) {
   const int b = (t - 1) >> 2, j = (t - 1) & 3;
-  return leaf_at<LIN>(b) + (LIN ? j : j * 3 + ci) * leaf_n<LIN>(b) + k - leaf_lo<LIN>(cb, b);
+  return leaf_at<LIN>(b, p) + (LIN ? j : j * 3 + ci) * leaf_n<LIN>(b, p) + k - leaf_lo<LIN>(cb, b, p);
 }
 
 // Leaf descriptors of the scores from .. s, for the one-step functions.
@@ -429,7 +433,7 @@ __device__ __noinline__ void leaf_describe(Dir& d, int s, int from, const Pen& p
       if (holds_row(q, p) && row_exists<LIN>(d.cb, t, ci, p))
         ds = t == 0 ? make_int4(0, 0, 0, 0)
                     : make_int4(row_lo<LIN>(d.cb, t, p), row_hi<LIN>(d.cb, t, p),
-                                leaf_cell<LIN>(d.cb, t, ci, leaf_lo<LIN>(d.cb, b)), leaf_lo<LIN>(d.cb, b));
+                                leaf_cell<LIN>(d.cb, t, ci, leaf_lo<LIN>(d.cb, b, p), p), leaf_lo<LIN>(d.cb, b, p));
       d.cfg.ldesc[q * 3 + ci] = ds;
     }
   }
@@ -471,7 +475,7 @@ __device__ __noinline__ int tile_backtrace(const Dir& B, const Pen& p, int s, in
             o = ref_raw<1>(B.cfg, sc, my_ci).get(kk);
           } else {
             const int t = row_of(sc, p);
-            const int at = t == 0 ? (my_ci == comp_index(cb) ? 0 : -1) : leaf_cell<LIN>(cb, t, my_ci, kk);
+            const int at = t == 0 ? (my_ci == comp_index(cb) ? 0 : -1) : leaf_cell<LIN>(cb, t, my_ci, kk, p);
             if (sc == t * p.tg && row_lo<LIN>(cb, t, p) <= kk && kk <= row_hi<LIN>(cb, t, p) && at >= 0) o = ldata[at];
           }
           if (o >= 0) mine = (o + my_add) * 16 + my_type;

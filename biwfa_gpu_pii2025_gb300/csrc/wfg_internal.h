@@ -121,6 +121,39 @@ static_assert(2 * (int64_t)WFG_TILE_NULL - (1 << 27) - 8 >= INT32_MIN, "twice a 
 WFG_HD constexpr inline int64_t wfg_tile_row(int row, int pitch) { return (int64_t)row * pitch; }
 static_assert(12 * (int64_t)((1 << 27) + WFG_TILE_PAD) <= INT32_MAX, "a block's rows are indexed with 32 bits");
 
+// The leaf store of a leaf whose rows come in tiles: row 0's one cell at 0, then block b's four rows
+// (rows 4b + 1 .. 4b + 4; M, I and D each, or M alone), all of one size, from wfg_tile_leaf_at(b), all
+// multiples of 4. Gap-affine rows span at most t diagonals on either side, 8b + 8 in all with one side
+// shorter by the gap opening; one-component rows t / lo on each side (lo: rows back to the gap source),
+// so with q = b / lo they lie within 4q + 4 of the middle. q = b for gap-affine.
+WFG_HD constexpr inline int wfg_tile_leaf_n(bool linear, int q) { return linear ? 8 * q + 12 : 8 * q + 8; }
+WFG_HD constexpr inline int wfg_tile_leaf_at(bool linear, int b, int q, int lo) {
+  // one component: 4 rows x sum over i < b of (8 (i / lo) + 12)
+  return 4 + (linear ? 48 * b + 32 * (lo * (q * (q - 1) / 2) + (b - q * lo) * q) : 48 * b * (b + 1));
+}
+
+// Words of a leaf store that holds every row of a leaf up to score smax, in a batch whose longest pair
+// has plen + tlen = maxsum; g: the spacing of the scores with a row. One score at a time a step at score
+// s takes at most ncomp * min(maxsum + 8, 2 s / emin + 8). Rows in tiles are not clipped to the window, so
+// where they need more, up to the largest score of a leaf (reach), that counts, and a last block's rows
+// beyond it.
+WFG_HD constexpr inline int64_t wfg_leaf_words(int smax, int maxsum, int g, int emin, int ncomp, bool tiles, bool linear,
+                                               int lo, int64_t reach) {
+  int64_t w = 0, tile = 0;
+  int q = 0, next = 4 * lo;  // q = (t - 1) / (4 lo) of row t = s / g
+  for (int s = 0, t = 0; s <= smax; s += g, ++t) {
+    const int64_t step = 2LL * s / emin + 8, clip = maxsum + 8;
+    int64_t row = ncomp * (step < clip ? step : clip);
+    if (tiles && s <= reach) {
+      if (t > next) { ++q; next += 4 * lo; }
+      tile = (int64_t)(linear ? 1 : 3) * wfg_tile_leaf_n(linear, q);
+      if (tile > row) row = tile;
+    }
+    w += row;
+  }
+  return w + 4 * tile;
+}
+
 // Physical ring buffers a direction needs: scores that can hold a wavefront are multiples of
 // g = gcd(x, o+e, e), so any window of `scope` consecutive scores holds at most ceil(scope/g)
 // live wavefronts, and round-robin buffers of that count are never overwritten while needed.

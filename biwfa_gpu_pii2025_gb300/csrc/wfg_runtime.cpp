@@ -291,14 +291,14 @@ void size_launch(const wfg_context* c, const IntPen& p, int pass, int ring_w_hin
   s.run_cap = maxsum + 2;
   s.leaf_run_cap = maxsum + 2;
   s.stack_cap = 64;
-  // Leaf store bound: a leaf's wavefronts sit at scores that are multiples of g, and the step
-  // at score s allocates at most nc * min(window + 8, 2*s/emin + 8) offsets. Pass 0 holds a
-  // leaf that starts at the BiWFA fallback score (250) with room to spare, pass 1 four times
+  // Leaf store (wfg_leaf_words): a leaf's wavefronts sit at scores that are multiples of g. Pass 0
+  // holds a leaf that starts at the BiWFA fallback score (250) with room to spare, pass 1 four times
   // that, pass 2 the full bound (recovery leaves up to score 500, whole short pairs).
+  const bool linear = p.metric != WFG_METRIC_GAP_AFFINE && p.metric != WFG_METRIC_GAP_AFFINE_2P;
+  const int64_t gap = p.metric == WFG_METRIC_GAP_LINEAR ? p.o : p.e;  // as score_guard, over windows of maxsum
+  const int64_t reach = std::max<int64_t>((p.x + 1) / 2, gap) * maxsum + p.o + p.e + 4 * p.scope + 16;
   auto leaf_words_upto = [&](int smax) {
-    int64_t w = 0;
-    for (int sc = 0; sc <= smax; sc += p.g) w += (int64_t)p.nc * std::min<int64_t>(maxsum + 8, 2LL * sc / p.emin + 8);
-    return w;
+    return wfg_leaf_words(smax, maxsum, p.g, p.emin, p.nc, tiles, linear, tiles && linear ? p.o / p.g : 1, reach);
   };
   const int64_t leaf_full = std::min<int64_t>(leaf_words_upto(s.leaf_max_score), (int64_t)1 << 28);
   const int64_t leaf_typical = leaf_words_upto(250) * 5 / 4;
