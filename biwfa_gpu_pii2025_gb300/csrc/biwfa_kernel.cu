@@ -1567,8 +1567,8 @@ cudaError_t biwfa_occupancy_shape(int gw, int ring_in_smem, size_t dyn, int* blo
   return occupancy_shape<false, kMaxScope>(gw, ring_in_smem, dyn, blocks_per_sm);
 }
 
-// Groups (pairs in flight) per block of a shape. A block of the tile kernel holds a pair per warp,
-// or fewer pairs that its other warps help with.
+// Most groups (pairs in flight) per block of a shape. A block of the tile kernel holds up to a pair per
+// warp, or fewer pairs that its other warps help with.
 int biwfa_groups_per_block(int group_warps, int tile_g) {
   if (tile_g > 0) return biwfa_owners(group_warps);
   return group_warps <= 1 ? kG1Groups : 1;

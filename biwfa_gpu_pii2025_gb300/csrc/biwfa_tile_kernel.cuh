@@ -35,7 +35,8 @@ constexpr int kTileBlocks = WFG_TILE_BLOCKS;  // thread blocks per SM
 // base and 1 us of memory latency per window, so an owner polls 128 times per base of its pair beyond
 // the constant before it gives a helper up. A helper without work leaves after about 10 s.
 constexpr int kSpinLimit = 1 << 24, kPollsPerBase = 128;
-// Warps of a block that own pairs, by the launch's warps per pair; the others help.
+// Most warps of a block that own pairs, by the launch's warps per pair; the others help. A launch of
+// few pairs has fewer owners (KernelParams::tile_owners), each of which needs an arena.
 __host__ __device__ constexpr int biwfa_owners(int group_warps) {
   return group_warps <= 1 ? kTileWarps : group_warps == 4 ? 2 : 1;
 }
@@ -632,7 +633,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, kTileBlocks) biwfa_tile_kerne
   TileBlockSmem& B = tile_smem();
   if (Pin.num_pairs_ptr != nullptr && *Pin.num_pairs_ptr == 0ull) return;  // a retry pass without pairs
   const int gib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int owners = biwfa_owners(Pin.group_warps);
+  const int owners = Pin.tile_owners;
   TileGroup& S = B.grp[gib];
   TileCtl& C = S.ctl;
   if (threadIdx.x == 0) { B.P = Pin; B.active = owners; B.idle = kTileWarps - owners; }

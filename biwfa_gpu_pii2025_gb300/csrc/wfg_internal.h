@@ -90,6 +90,7 @@ struct KernelParams {
   int ring_nphys;
   // rows in tiles (biwfa_tiles.cuh): the spacing of the scores that hold a row, 0 for one score at a time
   int tile_g;
+  int tile_owners;  // and the warps of a block that own pairs
   // the tile kernel's waits for another warp: counter of those that ran out (the run has failed then),
   // and their limit in polls (0: from the pair's length)
   unsigned long long* lost;

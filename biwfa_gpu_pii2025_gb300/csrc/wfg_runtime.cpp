@@ -275,6 +275,7 @@ struct Launch {
   int nphys = 0;         // ring buffers per direction
   int ring_w = 0, leaf_words = 0, leaf_max_score = 0, run_cap = 0, leaf_run_cap = 0, stack_cap = 0;
   int64_t groups = 0;    // pairs in flight
+  int per_block = 1;     // and of those in a thread block
   bool batched = false;  // consecutive launches of `groups` pairs each instead of one persistent launch
   ArenaLayout L{};
   int64_t arena_off = 0; // byte offset of this launch's arenas
@@ -346,11 +347,18 @@ int64_t max_groups(const wfg_context* c, const IntPen& p, const Launch& l) {
   return (int64_t)bps * c->num_sms * biwfa_groups_per_block(l.gw, l.smem ? 0 : p.tile_g);
 }
 
+// Resident warps of a launch: a block of the tile kernel has its 16 whatever its pairs.
+int resident_warps(const IntPen& p, const Launch& l) {
+  return p.tile_g > 0 && !l.smem ? (int)(l.groups / l.per_block) * biwfa_groups_per_block(1, p.tile_g)
+                                 : (int)(l.groups * l.gw);
+}
+
 // Kernel parameters of one launch of pass ps (0: first pass; the retry passes read the
 // previous pass's overflow list); the work queue (order, count, head) is set by the caller.
 KernelParams launch_params(const wfg_context* c, const wfg_config_t* cfg, const IntPen& p, const Launch& l, int ps) {
   const int n = c->n;
   KernelParams kp{};
+  kp.tile_owners = l.per_block;
   kp.x = p.x; kp.o = p.o; kp.e = p.e; kp.scope = p.scope; kp.o2 = p.o2; kp.e2 = p.e2;
   kp.match_o = cfg->match; kp.x_o = cfg->mismatch; kp.o_o = cfg->gap_opening; kp.e_o = cfg->gap_extension;
   if (p.nc == 5) { kp.o2_o = cfg->gap_opening2; kp.e2_o = cfg->gap_extension2; }
@@ -386,6 +394,34 @@ KernelParams launch_params(const wfg_context* c, const wfg_config_t* cfg, const 
   return kp;
 }
 
+// The groups in flight of a launch of up to `count` pairs: at most `most` of them, within the device's
+// residency and the arena budget (false: the budget is what limits them). Every pair of a small batch
+// in tiles gets a thread block, whose other warps help with the pair's tiles; blocks hold several pairs
+// only where there are more pairs than blocks, so that no arena is reserved for a warp that can only
+// help: 64 pairs of 1 kbp take 64 arenas, not 64 blocks of 16 (1.56 GB).
+bool plan_groups(const wfg_context* c, const IntPen& p, int64_t count, int64_t most, int64_t arena_budget, Launch& l) {
+  const bool tiles = p.tile_g > 0 && !l.smem;
+  const int64_t resident = std::min(max_groups(c, p, l), most), fit = arena_budget / std::max<int64_t>(l.L.total, 1);
+  const int gpb = biwfa_groups_per_block(l.gw, l.smem ? 0 : p.tile_g);
+  count = std::max<int64_t>(count, 1);
+  if (tiles) {
+    int64_t blocks = std::min<int64_t>(std::max<int64_t>(resident / gpb, 1), count);
+    int64_t owners = std::min<int64_t>(gpb, (count + blocks - 1) / blocks);
+    const bool enough = blocks * owners <= fit;
+    if (!enough) {
+      owners = std::max<int64_t>(1, std::min(owners, fit / blocks));
+      blocks = std::max<int64_t>(1, std::min(blocks, fit / owners));
+    }
+    l.per_block = (int)owners;
+    l.groups = blocks * owners;
+    return enough;
+  }
+  const int64_t want = std::min(resident, std::max<int64_t>(gpb, count));
+  l.per_block = gpb;
+  l.groups = std::max<int64_t>(gpb, (std::min(want, fit) / gpb) * gpb);
+  return want <= fit;
+}
+
 // Shapes and arenas of the retry passes (1 .. kNumPasses-1), which realign the pairs that
 // overflowed the previous pass; returns the arena bytes the largest of them needs.
 int64_t plan_retry_passes(const wfg_context* c, const IntPen& p, int64_t arena_budget, Launch* retry,
@@ -395,12 +431,8 @@ int64_t plan_retry_passes(const wfg_context* c, const IntPen& p, int64_t arena_b
     Launch& l = retry[ps];
     l.gw = c->tune.retry_warps;  // pairs that overflowed the first pass are wide
     size_launch(c, p, ps, 0, l);
-    const int gpb = biwfa_groups_per_block(l.gw, l.smem ? 0 : p.tile_g);
-    int64_t gmax = std::min<int64_t>(max_groups(c, p, l), std::max<int64_t>(gpb, (int64_t)c->n));
-    if (l.gw == 1) gmax = std::min<int64_t>(gmax, ps == 1 ? (int64_t)c->num_sms * 4 : (int64_t)c->num_sms * 2);
-    const int64_t fit = arena_budget / std::max<int64_t>(l.L.total, 1);
-    if (short_of_memory && fit < gmax) *short_of_memory = true;
-    l.groups = std::max<int64_t>(gpb, (std::min(gmax, fit) / gpb) * gpb);
+    const int64_t most = l.gw == 1 ? (int64_t)c->num_sms * (ps == 1 ? 4 : 2) : INT64_MAX;
+    if (!plan_groups(c, p, c->n, most, arena_budget, l) && short_of_memory) *short_of_memory = true;
     need = std::max(need, l.groups * l.L.total);
   }
   return need;
@@ -413,13 +445,7 @@ void plan_first_pass(const wfg_context* c, const IntPen& p, int hint, int64_t ar
   if (l.gw < 1) l.gw = 1;
   if (l.gw != 1 && l.gw != 4 && l.gw != 8) l.gw = 8;
   size_launch(c, p, 0, hint, l);
-  // Every pair of a small batch gets a block (its other warps help with the pair's tiles).
-  const int gpb = biwfa_groups_per_block(l.gw, l.smem ? 0 : p.tile_g);
-  const int64_t gmax = std::min<int64_t>(max_groups(c, p, l), std::max<int64_t>(1, l.count) * gpb);
-  const int64_t fit = arena_budget / std::max<int64_t>(l.L.total, 1);
-  if (short_of_memory && fit < gmax) *short_of_memory = true;
-  l.groups = std::max<int64_t>(1, std::min(gmax, fit));
-  l.groups = std::max<int64_t>(gpb, (l.groups / gpb) * gpb);
+  if (!plan_groups(c, p, l.count, INT64_MAX, arena_budget, l) && short_of_memory) *short_of_memory = true;
 }
 
 // The arena budget of a run: half of the device memory that is free or already held by the
@@ -694,14 +720,13 @@ int wfg_run(wfg_context_t* c, const wfg_config_t* cfg, wfg_sched_t sched) {
       if (l.count <= 0) continue;
       if (l.batched) {
         // one launch per resident set of pairs, each waiting for its slowest pair
-        const int gpb = biwfa_groups_per_block(l.gw, l.smem ? 0 : p.tile_g);
         for (int64_t b0 = 0; b0 < l.count; b0 += l.groups, ++batch_index) {
           KernelParams kp = params(l, 0);
           kp.num_pairs = (int)std::min<int64_t>(l.groups, l.count - b0);
           kp.num_pairs_ptr = nullptr;
           kp.order = c->d_order.ptr + l.order_off + b0;
           kp.queue_head = c->d_batch_heads.ptr + batch_index;
-          const int blocks = (int)((kp.num_pairs + gpb - 1) / gpb);
+          const int blocks = (int)((kp.num_pairs + l.per_block - 1) / l.per_block);
           if ((e = launch_biwfa(kp, blocks, c->stream)) != cudaSuccess) return e;
           ++launches;
         }
@@ -713,7 +738,7 @@ int wfg_run(wfg_context_t* c, const wfg_config_t* cfg, wfg_sched_t sched) {
       kp.order = c->d_order.ptr + l.order_off;
       kp.queue_head = c->d_counters.ptr + (li == 0 ? 0 : 2);
       const cudaStream_t st = (fork && li > 0) ? c->aux_stream : c->stream;
-      if ((e = launch_biwfa(kp, (int)(l.groups / biwfa_groups_per_block(l.gw, l.smem ? 0 : p.tile_g)), st)) != cudaSuccess) return e;
+      if ((e = launch_biwfa(kp, (int)(l.groups / l.per_block), st)) != cudaSuccess) return e;
       ++launches;
     }
     if (fork) {
@@ -729,7 +754,7 @@ int wfg_run(wfg_context_t* c, const wfg_config_t* cfg, wfg_sched_t sched) {
       kp.num_pairs_ptr = c->d_counters.ptr + (ps - 1) * kCountersPerPass + 1;
       kp.order = c->d_retry.ptr + (size_t)(ps - 1) * n;
       kp.queue_head = c->d_counters.ptr + ps * kCountersPerPass + 0;
-      if ((e = launch_biwfa(kp, (int)(l.groups / biwfa_groups_per_block(l.gw, l.smem ? 0 : p.tile_g)), c->stream)) != cudaSuccess)
+      if ((e = launch_biwfa(kp, (int)(l.groups / l.per_block), c->stream)) != cudaSuccess)
         return e;
       ++launches;
     }
@@ -765,7 +790,7 @@ int wfg_run(wfg_context_t* c, const wfg_config_t* cfg, wfg_sched_t sched) {
     WFG_CHECK(c, enqueue(false));
   }
   c->stats.launches = launches + predict_launches;
-  c->stats.num_warps = (int)(first[0].groups * first[0].gw);
+  c->stats.num_warps = resident_warps(p, first[0]);
   c->stats.ring_w = first[0].ring_w;
   c->stats.arena_bytes = first[0].L.total;
   c->ran = true;
@@ -976,7 +1001,7 @@ int align_host_pipelined(wfg_context* c, const wfg_config_t* cfg, wfg_sched_t sc
   WFG_CHECK(c, cudaStreamWaitEvent(as, c->ev[5], 0));  // the aux and alternate streams follow this run's start
   WFG_CHECK(c, cudaStreamWaitEvent(c->alt_stream, c->ev[5], 0));
   int launches = 0;
-  int64_t first_warps = 0;
+  int first_warps = 0;
   int first_ring = 0;
   int64_t first_arena = 0;
   for (int k = 0; k < K; ++k) {
@@ -1023,9 +1048,9 @@ int align_host_pipelined(wfg_context* c, const wfg_config_t* cfg, wfg_sched_t sc
     kp.num_pairs_ptr = nullptr;
     kp.order = c->d_order.ptr + a;
     kp.queue_head = c->d_batch_heads.ptr + k;
-    WFG_CHECK(c, launch_biwfa(kp, (int)(l.groups / biwfa_groups_per_block(l.gw, l.smem ? 0 : p.tile_g)), ks));
+    WFG_CHECK(c, launch_biwfa(kp, (int)(l.groups / l.per_block), ks));
     ++launches;
-    if (k == 0) { first_warps = l.groups * l.gw; first_ring = l.ring_w; first_arena = l.L.total; }
+    if (k == 0) { first_warps = resident_warps(p, l); first_ring = l.ring_w; first_arena = l.L.total; }
   }
   WFG_CHECK(c, cudaEventRecord(c->ev[4], c->alt_stream));
   WFG_CHECK(c, cudaStreamWaitEvent(ms, c->ev[4], 0));
@@ -1037,7 +1062,7 @@ int align_host_pipelined(wfg_context* c, const wfg_config_t* cfg, wfg_sched_t sc
     kp.num_pairs_ptr = c->d_counters.ptr + (ps - 1) * kCountersPerPass + 1;
     kp.order = c->d_retry.ptr + (size_t)(ps - 1) * n;
     kp.queue_head = c->d_counters.ptr + ps * kCountersPerPass + 0;
-    WFG_CHECK(c, launch_biwfa(kp, (int)(l.groups / biwfa_groups_per_block(l.gw, l.smem ? 0 : p.tile_g)), ms));
+    WFG_CHECK(c, launch_biwfa(kp, (int)(l.groups / l.per_block), ms));
     ++launches;
   }
   WFG_CHECK(c, cudaEventRecord(c->ev[3], ms));
@@ -1045,7 +1070,7 @@ int align_host_pipelined(wfg_context* c, const wfg_config_t* cfg, wfg_sched_t sc
                                cudaMemcpyDeviceToHost, ms));
   c->stats.used_graph = 0;
   c->stats.launches = launches;
-  c->stats.num_warps = (int)first_warps;
+  c->stats.num_warps = first_warps;
   c->stats.ring_w = first_ring;
   c->stats.arena_bytes = first_arena;
   c->stats.pipeline_chunks = K;
