@@ -276,6 +276,7 @@ struct Launch {
   int ring_w = 0, leaf_words = 0, leaf_max_score = 0, run_cap = 0, leaf_run_cap = 0, stack_cap = 0;
   int64_t groups = 0;    // pairs in flight
   int per_block = 1;     // and of those in a thread block
+  int most = INT_MAX;    // most of them that the plan may ask for
   bool batched = false;  // consecutive launches of `groups` pairs each instead of one persistent launch
   ArenaLayout L{};
   int64_t arena_off = 0; // byte offset of this launch's arenas
@@ -394,18 +395,18 @@ KernelParams launch_params(const wfg_context* c, const wfg_config_t* cfg, const 
   return kp;
 }
 
-// The groups in flight of a launch of up to `count` pairs: at most `most` of them, within the device's
+// The groups in flight of a launch of up to `count` pairs: at most l.most of them, within the device's
 // residency and the arena budget (false: the budget is what limits them). Every pair of a small batch
 // in tiles gets a thread block, whose other warps help with the pair's tiles; blocks hold several pairs
 // only where there are more pairs than blocks, so that no arena is reserved for a warp that can only
 // help: 64 pairs of 1 kbp take 64 arenas, not 64 blocks of 16 (1.56 GB).
-bool plan_groups(const wfg_context* c, const IntPen& p, int64_t count, int64_t most, int64_t arena_budget, Launch& l) {
+bool plan_groups(const wfg_context* c, const IntPen& p, int64_t count, int64_t arena_budget, Launch& l) {
   const bool tiles = p.tile_g > 0 && !l.smem;
-  const int64_t resident = std::min(max_groups(c, p, l), most), fit = arena_budget / std::max<int64_t>(l.L.total, 1);
+  const int64_t resident = max_groups(c, p, l), fit = arena_budget / std::max<int64_t>(l.L.total, 1);
   const int gpb = biwfa_groups_per_block(l.gw, l.smem ? 0 : p.tile_g);
-  count = std::max<int64_t>(count, 1);
+  count = std::min<int64_t>(std::max<int64_t>(count, 1), l.most);
   if (tiles) {
-    int64_t blocks = std::min<int64_t>(std::max<int64_t>(resident / gpb, 1), count);
+    int64_t blocks = std::min<int64_t>(resident / gpb, count);
     int64_t owners = std::min<int64_t>(gpb, (count + blocks - 1) / blocks);
     const bool enough = blocks * owners <= fit;
     if (!enough) {
@@ -431,8 +432,8 @@ int64_t plan_retry_passes(const wfg_context* c, const IntPen& p, int64_t arena_b
     Launch& l = retry[ps];
     l.gw = c->tune.retry_warps;  // pairs that overflowed the first pass are wide
     size_launch(c, p, ps, 0, l);
-    const int64_t most = l.gw == 1 ? (int64_t)c->num_sms * (ps == 1 ? 4 : 2) : INT64_MAX;
-    if (!plan_groups(c, p, c->n, most, arena_budget, l) && short_of_memory) *short_of_memory = true;
+    if (l.gw == 1) l.most = c->num_sms * (ps == 1 ? 4 : 2);
+    if (!plan_groups(c, p, c->n, arena_budget, l) && short_of_memory) *short_of_memory = true;
     need = std::max(need, l.groups * l.L.total);
   }
   return need;
@@ -445,7 +446,7 @@ void plan_first_pass(const wfg_context* c, const IntPen& p, int hint, int64_t ar
   if (l.gw < 1) l.gw = 1;
   if (l.gw != 1 && l.gw != 4 && l.gw != 8) l.gw = 8;
   size_launch(c, p, 0, hint, l);
-  if (!plan_groups(c, p, l.count, INT64_MAX, arena_budget, l) && short_of_memory) *short_of_memory = true;
+  if (!plan_groups(c, p, l.count, arena_budget, l) && short_of_memory) *short_of_memory = true;
 }
 
 // The arena budget of a run: half of the device memory that is free or already held by the
@@ -631,7 +632,13 @@ int wfg_run(wfg_context_t* c, const wfg_config_t* cfg, wfg_sched_t sched) {
     // 10-20 kbp at 12 %, 37 of which outgrow it: 123 -> 73 ms; one 10 kbp pair that does not: 8.45 and 8.42.
     if (by_length && p.tile_g && n <= c->num_sms && c->max_sum + 8 + WFG_TILE_MARGIN > (int)kPlainRingCap) n_long = n;
     if (n_long > 0) {
-      Launch lw; lw.gw = c->tune.retry_warps; lw.count = n_long; lw.order_off = 0;
+      // In tiles a block holds one long pair, or up to four where long pairs outnumber blocks: narrow
+      // wavefronts (low-error pairs) have no tiles to help with, and wide ones share the helpers. One
+      // -> four a block: 2,000 pairs of 17 kbp at 0.1 % 6.6 -> 2.4 ms (one score at a time 5.6), at
+      // 1 % 35.8 -> 13.3, 608 at 5 % 74.9 -> 38.8, 1,000 of 50-100 kbp at 12 % 4.54 -> 3.98 s. More (up to
+      // 16) are faster still at low error, but take four times the arenas of full width.
+      Launch lw; lw.gw = p.tile_g ? 1 : c->tune.retry_warps; lw.count = n_long; lw.order_off = 0;
+      if (p.tile_g) lw.most = c->num_sms * 4;
       lw.ring_w = (int)next_pow2((uint64_t)c->max_sum + 8);  // capped at the full width
       first.push_back(lw);
     }

@@ -99,3 +99,22 @@ def test_a_wait_that_runs_out_fails_the_run_and_leaves_the_context_usable(batch_
     for i in range(b.n):
         _, score, ops, _ = binding.oracle_align(b.pattern(i), b.text(i))
         assert res.status[i] == 0 and res.scores[i] == score and pkg.runs_to_ops(res.runs_of(i)) == ops, i
+
+
+@pytest.mark.parametrize("n", [152, 153, 320, 620])
+def test_long_pairs_several_to_a_block(batch_aligner, n):
+    """Pairs that start in rings of full width, as many as thread blocks, one more, two and up to four a
+    block: low-error ones and some with wide wavefronts beside them."""
+    rng = np.random.default_rng(n)
+    pairs = []
+    for i in range(n):
+        p = rng.choice(list(b"ACGT"), int(rng.integers(16500, 17000))).astype(np.uint8)
+        t = np.delete(p, rng.integers(0, p.size, 400 if i % 40 == 0 else 12))
+        t[rng.integers(0, t.size, 8)] = ord("G")
+        pairs.append((bytes(p), bytes(t)))
+    b = pkg.PairBatch.from_lists([p for p, _ in pairs], [t for _, t in pairs])
+    res = batch_aligner.align(b)
+    assert batch_aligner.stats().retried_pairs == 0 and (res.status == 0).all()
+    for i in range(n):
+        _, score, ops, _ = binding.oracle_align(b.pattern(i), b.text(i))
+        assert res.scores[i] == score and pkg.runs_to_ops(res.runs_of(i)) == ops, i
