@@ -108,7 +108,7 @@ def test_long_pairs_several_to_a_block(batch_aligner, n):
     rng = np.random.default_rng(n)
     pairs = []
     for i in range(n):
-        p = rng.choice(list(b"ACGT"), int(rng.integers(16500, 17000))).astype(np.uint8)
+        p = rng.choice(list(b"ACGT"), int(rng.integers(16900, 17300))).astype(np.uint8)
         t = np.delete(p, rng.integers(0, p.size, 400 if i % 40 == 0 else 12))
         t[rng.integers(0, t.size, 8)] = ord("G")
         pairs.append((bytes(p), bytes(t)))
