@@ -465,6 +465,49 @@ int64_t arena_budget_of(const wfg_context* c) {
   return budget;
 }
 
+// Whether rows stay out of tiles because the batch's pairs are short. A short pair has a few narrow
+// rows: a tile's lanes are mostly idle, and what the two kernels do between rows counts, for which the
+// one-score kernel has 32 warps an SM and the tile kernel 16. In a small batch the tile kernel's helpers
+// outweigh that. What a batch gains also depends on its error rate, which is not known here: tiles win
+// where a pair has more than a few edits. So the lines lie where single scores were not slower at any
+// rate measured, 0.5-10 %, with room for the bases that the text has more (time in tiles / time one
+// score at a time, GB300):
+//   gap-affine   20,000 pairs of 60 bp 1.01-1.08, 160,000 of 80 bp 1.04-1.22, of 40 bp 1.20-1.26; but
+//                20,000 of 75 bp at 10 % 0.94, 100,000 of 100 bp at 5 % 0.87, of 150 bp at 2 % 0.94 (at
+//                0.5 % 1.22). Scores only: 20,000 of 50 bp 1.01-1.31; 100,000 of 75 bp 1.18-1.44 up to
+//                5 %, though 0.75 at 10 %.
+//   gap-linear   10,000 pairs of up to 90 bp 1.05-1.17, 100,000 1.14-1.31; 20,000 of 110 bp at 5 % 0.79.
+//                Scores only: 0.9 at 10 % from 40 bp on, so in tiles.
+//   edit, indel  20,000 pairs of up to 500 bp 1.02-1.57; 3,000 of 500 bp 0.96-1.09, 20,000 of 1 kbp at
+//                10 % 0.89-0.98. Scores only: 100,000 of up to 500 bp 0.97-1.61; 20,000 0.89-1.35.
+// A few longer pairs do not move the batch as long as the longest, on one warp, takes no longer than
+// the rest: its time grows with the square of its length, the rest's with their number (edit, 200,000
+// of 100 bp and 1,000 of 1 kbp at 10 % 1.22; gap-linear, 200,000 of 70 bp and 1,000 of 300 bp 1.27;
+// gap-affine, 200,000 of 40 bp and 20 of 300 bp 1.07, but with one of 1 kbp 0.61).
+bool short_batch(const wfg_context* c, const wfg_config_t* cfg) {
+  const int n = c->n;
+  const int64_t longest = c->max_sum;
+  const bool scores = cfg->score_only != 0;
+  int line, min_pairs, few;  // plen + tlen of a short pair; batch size; longer ones: at most n / few
+  int64_t tail;              // and (plen + tlen)^2 <= tail * n
+  if (cfg->metric == WFG_METRIC_GAP_AFFINE) {
+    if (n >= 16384 && longest <= (scores ? 112 : 136)) return true;
+    line = scores ? 170 : 184; min_pairs = 65536; few = 1024; tail = 2;
+  } else if (cfg->metric == WFG_METRIC_GAP_LINEAR) {
+    if (scores) return false;
+    line = 204; min_pairs = 8192; few = 128; tail = 10;
+  } else {
+    if (longest <= 256) return true;
+    line = 1000; min_pairs = scores ? 65536 : 16384; few = 128; tail = 40;
+  }
+  if (n < min_pairs) return false;
+  if (longest <= line) return true;
+  if (longest * longest > tail * n) return false;
+  int over = 0;
+  for (int i = 0; i < n && over <= n / few; ++i) over += c->h_plen[(size_t)i] + c->h_tlen[(size_t)i] > line;
+  return over <= n / few;
+}
+
 // The distance and penalties of a run, checked against the resident batch; *p receives the
 // internal penalties. Configuration errors are statuses with a message, never exits.
 int validate_config(wfg_context* c, const wfg_config_t* cfg, IntPen* p) {
@@ -496,20 +539,16 @@ int validate_config(wfg_context* c, const wfg_config_t* cfg, IntPen* p) {
   }
   // Rows in tiles: gap-affine penalties with x = 2e, o + e = 4e (the defaults 4/6/2 among them)
   // within the usual kernels' score scope, the ratio that the tiles' row recurrence is written for;
-  // other ratios and distances take one score at a time. A step limit that a score can reach counts
-  // single scores. 10,000 pairs of 1 kbp: 7.7 ms one score at a time, 3.2 ms in tiles.
-  if (cfg->metric == WFG_METRIC_GAP_AFFINE && p->x == 2 * p->e && p->o == 3 * p->e && p->scope <= WFG_MAX_SCOPE &&
-      (cfg->max_alignment_steps <= 0 || cfg->max_alignment_steps >= (1 << 28)))
-    p->tile_g = p->e;
-  // And the one-component distances whose mismatch and gap lie at most four rows back: 20,000 uneven
-  // pairs of edit distance 18.7 ms end to end one score at a time, 9.1 ms in tiles; 5,000 of 5 kbp at
-  // 3-8 %: edit 12.4 and 7.2 ms, indel 17.4 and 10.0, gap-linear 4/2 24.9 and 11.0. Batches whose
-  // longest pair has 128 bp a side keep single scores for edit and indel (20,000 pairs of 100 bp: 0.51
-  // and 0.56 ms; of 200 bp 1.18 and 1.11).
-  const bool edits = cfg->metric == WFG_METRIC_EDIT || cfg->metric == WFG_METRIC_INDEL;
-  if (((edits && c->max_sum > kEditTilesMinSum) ||
-       (cfg->metric == WFG_METRIC_GAP_LINEAR && p->x <= 4 * p->g && p->o <= 4 * p->g && p->scope <= WFG_MAX_SCOPE)) &&
-      (cfg->max_alignment_steps <= 0 || cfg->max_alignment_steps >= (1 << 28)))
+  // other ratios and distances take one score at a time. 10,000 pairs of 1 kbp: 7.7 ms one score at a
+  // time, 3.2 ms in tiles. And the one-component distances whose mismatch and gap lie at most four rows
+  // back: 20,000 uneven pairs of edit distance 18.7 ms end to end one score at a time, 9.1 ms in tiles;
+  // 5,000 of 5 kbp at 3-8 %: edit 12.4 and 7.2 ms, indel 17.4 and 10.0, gap-linear 4/2 24.9 and 11.0.
+  // A step limit that a score can reach counts single scores.
+  const bool affine = cfg->metric == WFG_METRIC_GAP_AFFINE && p->x == 2 * p->e && p->o == 3 * p->e;
+  const bool one_component = cfg->metric == WFG_METRIC_EDIT || cfg->metric == WFG_METRIC_INDEL ||
+                             (cfg->metric == WFG_METRIC_GAP_LINEAR && p->x <= 4 * p->g && p->o <= 4 * p->g);
+  if ((affine || one_component) && p->scope <= WFG_MAX_SCOPE &&
+      (cfg->max_alignment_steps <= 0 || cfg->max_alignment_steps >= (1 << 28)) && !short_batch(c, cfg))
     p->tile_g = p->g;
   if ((int64_t)(c->max_sum + 16) * (int64_t)std::max(p->x, std::max(p->o + p->e, p->o2 + p->e2)) >= ((int64_t)1 << 26)) {
     c->err = "pair too long for 27-bit scores";
