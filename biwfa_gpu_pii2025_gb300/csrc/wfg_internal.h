@@ -130,7 +130,7 @@ static_assert(12 * (int64_t)((1 << 27) + WFG_TILE_PAD) <= INT32_MAX, "a block's 
 WFG_HD constexpr inline int wfg_tile_leaf_n(bool linear, int q) { return linear ? 8 * q + 12 : 8 * q + 8; }
 WFG_HD constexpr inline int wfg_tile_leaf_at(bool linear, int b, int q, int lo) {
   // one component: 4 rows x sum over i < b of (8 (i / lo) + 12)
-  return 4 + (linear ? 48 * b + 32 * (lo * (q * (q - 1) / 2) + (b - q * lo) * q) : 48 * b * (b + 1));
+  return 4 + (linear ? 48 * b + 16 * q * (2 * b - lo * (q + 1)) : 48 * b * (b + 1));
 }
 
 // Words of a leaf store that holds every row of a leaf up to score smax, in a batch whose longest pair
