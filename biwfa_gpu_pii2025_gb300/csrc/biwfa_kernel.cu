@@ -45,7 +45,8 @@ constexpr int kMaxScope2p = WFG_MAX_SCOPE_2P;  // the cap of the large-scope and
 #endif
 // Single-warp shape: kG1Groups pairs (warps) per block; resident warps per SM fix the register
 // cap. The three-component kernels keep 32 warps per SM (64 registers), the two-piece one 28
-// (72 registers). Measured (same GB300, identical results) against 28 warps for all: gap-affine
+// (72 registers). Measured (same GB300, identical results; every distance ran here then, before the
+// default penalties and the one-component distances had rows in tiles) against 28 warps for all: gap-affine
 // mixture 1.3 % faster, uneven pairs 1.6 %, edit mixture 5.4 % faster, 150 bp pairs 2.6 %
 // slower, two-piece mixture 7.9 % slower (its step spills at 64 registers); 36 warps (56
 // registers) 4 % and 40 warps (48 registers) 15 % slower on the gap-affine mixture. One warp
@@ -60,7 +61,7 @@ constexpr int g1_min_blocks() { return (TWO ? WFG_G1_WARPS5 : WFG_G1_WARPS3) / k
 #endif
 constexpr int kStepUnroll = WFG_STEP_UNROLL;        // diagonals per thread per step iteration (rings)
 // The same for the leaf store (narrower steps). One diagonal per thread there, measured against
-// two at 32 warps per SM (same GB300, identical results): gap-affine mixture 3.2 % faster,
+// two at 32 warps per SM (same GB300, identical results, every distance in this kernel): gap-affine mixture 3.2 % faster,
 // 1 kbp pairs 6.7 %, 150 bp pairs 4.3 %, uneven pairs 2.4 %, two-piece equal, edit 2.8 %
 // slower; three diagonals 3.5 % slower on the mixture. In the ring steps two per thread stay
 // best (one 4.3 %, three 8.7 % slower). The multi-warp shapes keep two in the leaf steps (the

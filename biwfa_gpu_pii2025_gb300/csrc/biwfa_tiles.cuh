@@ -74,10 +74,6 @@ __device__ __forceinline__ bool row_exists(int cb, int t, int ci, const Pen& p) 
 }
 __device__ __forceinline__ int row_buffer(int t) { return (t + kTileBufs - 1) % kTileBufs; }
 
-template <int C> struct TileVec;
-template <> struct TileVec<1> { typedef int type; };
-template <> struct TileVec<2> { typedef int2 type; };
-template <> struct TileVec<4> { typedef int4 type; };
 template <int C>
 __device__ __forceinline__ void tile_load(const int32_t* p, int (&v)[C]) {
   if (C == 1) { v[0] = *p; }

@@ -4,9 +4,9 @@
 // One wfg_context owns a CUDA stream and grow-only device buffers. wfg_run enqueues,
 // without any host synchronisation:
 //   1. pack_pairs_kernel            ASCII -> 2-bit (or 8-bit) words, forward and reversed
-//   2. biwfa_persistent_kernel x3   main pass + two retry passes with larger arenas; each
-//                                   pass reads the previous pass's overflow count from HBM,
-//                                   so an empty retry pass costs one launch and exits.
+//   2. biwfa_tile_kernel or         main pass (one or two launches) + two retry passes with larger
+//      biwfa_persistent_kernel      arenas; each pass reads the previous pass's overflow count from
+//                                   HBM, so an empty retry pass costs one launch and exits.
 // Results stay in HBM until wfg_fetch.
 #include <cuda_runtime.h>
 
@@ -617,7 +617,7 @@ int wfg_run(wfg_context_t* c, const wfg_config_t* cfg, wfg_sched_t sched) {
     const bool use_wide = c->tune.wide_warps > 1 && c->tune.wide_threshold < 3.0e38f;  // FLT_MAX: no wide launch
     int64_t wide_cap = 0;
     if (use_wide) {
-      Launch lw; lw.gw = c->tune.wide_warps; lw.smem = c->tune.wide_smem; lw.ring_w = kSmemRingW;
+      Launch lw; lw.gw = c->tune.wide_warps; lw.smem = p.tile_g == 0 ? c->tune.wide_smem : 0; lw.ring_w = kSmemRingW;
       wide_cap = max_groups(c, p, lw);
     }
     WFG_CHECK(c, c->d_bin_work.reserve((size_t)sched_bin_words()));
@@ -753,8 +753,9 @@ int wfg_run(wfg_context_t* c, const wfg_config_t* cfg, wfg_sched_t sched) {
       return e;
     if ((e = launch_pack(n, c->d_seq.ptr, c->d_pairs.ptr, c->d_words.ptr, c->num_sms, c->stream)) != cudaSuccess) return e;
     if ((e = mark(c->ev[1])) != cudaSuccess) return e;
-    // pass 0: the first launch on the context's stream, a second one on the aux stream,
-    // forked before the first so that the two run concurrently, joined before the retry passes
+    // pass 0: the first launch on the context's stream, a second one on the aux stream, forked
+    // before the first so that the two run concurrently (in tiles on different SMs: a block fills
+    // one), joined before the retry passes
     int64_t batch_index = 0;
     const bool fork = first.size() > 1 && first[1].count > 0 && first[0].count > 0;
     if (fork) {
@@ -950,13 +951,13 @@ constexpr int kPipelineHeadDiv = 8;        // the head chunk: the first 1/8 of t
 // each chunk's last byte, chunk by chunk. As soon as chunk k's bytes are in, the aux stream
 // packs it and (learned schedule) computes its features, predictions and binned order; chunk
 // k's first pass then runs on the main stream (even k) or the alternate stream (odd k), in its
-// own arena region, so that it takes over the SMs as chunk k-1's persistent warps retire. The
-// head's alignment outlasts the copy of everything else, and the rest then runs in one
-// launch, heaviest first: with many equal chunks, each chunk's heaviest pairs (about 0.3 s for
-// one warp) started only when the chunk did, and the last chunk's ones ended after the rest
-// (measured: 8 equal chunks cost 190 ms of device time, as much as the copy they hid). The
-// retry passes run once, over the overflows of every chunk. Scheduling only: every pair's
-// result is the one wfg_run gives.
+// own arena region, so that it takes over the SMs as chunk k-1's blocks retire (SM by SM in tiles,
+// where a block fills one; warp by warp in the one-score kernel). The head's alignment outlasts the
+// copy of everything else, and the rest then runs in one launch, heaviest first: with many equal
+// chunks, each chunk's heaviest pairs (about 0.3 s for one warp, one score at a time) started only
+// when the chunk did, and the last chunk's ones ended after the rest (measured then: 8 equal chunks
+// cost 190 ms of device time, as much as the copy they hid). The retry passes run once, over the
+// overflows of every chunk. Scheduling only: every pair's result is the one wfg_run gives.
 int align_host_pipelined(wfg_context* c, const wfg_config_t* cfg, wfg_sched_t sched, int n, const char* seq,
                          int64_t seq_len, const int64_t* p_off, const int* plen, const int64_t* t_off, const int* tlen,
                          int K) {

@@ -282,8 +282,8 @@ typedef enum {
   WFG_SCHED_LEARNED = 1,
   WFG_SCHED_GIVEN = 2,    /* the caller's order (wfg_set_order), one persistent launch */
   /* pairs sorted by length (descending), one persistent launch; pairs with plen + tlen above
-   * 32,768 take a multi-warp launch (the retry passes' shape) with rings as wide as the
-   * batch's longest pair, concurrent with the single-warp launch of the rest */
+   * 32,768 take a launch of their own, with several warps to a pair and rings as wide as the
+   * batch's longest pair, concurrent with the launch of the rest */
   WFG_SCHED_SORTED = 3,
 } wfg_sched_t;
 
@@ -296,7 +296,7 @@ typedef struct {
   int retried_pairs;      /* pairs rerun with a larger arena after a scratch overflow */
   int num_warps;          /* resident warps of the main launch */
   int ring_w;             /* ring width (diagonals) of the main launch */
-  int64_t arena_bytes;    /* per-warp arena of the main launch */
+  int64_t arena_bytes;    /* arena of one pair in flight of the main launch */
   int64_t total_runs;     /* CIGAR runs produced */
   int64_t h2d_bytes, d2h_bytes; /* bytes copied by the last upload / fetch */
   int used_graph;         /* 1 when the last wfg_run's device work ran as one CUDA graph */
