@@ -396,7 +396,7 @@ def run_ours(args):
                       "autotuned warps-per-pair and shared-memory rings)")
     elif args.sched == "sorted" and not args.plain_only:
         sched = _capi.SCHED_SORTED
-        sched_name = ("length-sorted persistent (pairs above 32,768 bp total on 8-warp groups with full-width "
+        sched_name = ("length-sorted persistent (pairs above 32,768 bp total in a launch with full-width "
                       "rings, concurrently)")
     else:
         sched = _capi.SCHED_PLAIN
